@@ -2,6 +2,7 @@
 // tables :180-257) together with the grid / wavenumber setup the driver performs
 // (src/specter.fpp:683-800, kes module src/pseudo/pseudospec_mod.fpp:84-91).
 #include "batch.h"
+#include "tcdft.h"
 #include "plan.h"
 
 #include <cmath>
@@ -357,6 +358,7 @@ void *Plan::scratch_field(int i) {
 unsigned long long plan_bytes(const Plan &P) {
     unsigned long long b = 0;
     for (void *m : P.scratch) b += m ? P.field_bytes() : 0;
+    b += tc_bytes(P);
     b += (P.kx.size() + P.ky.size() + P.kz.size() + P.z.size() + P.dir.size() + P.fx.size() + P.fy.size() + P.fz.size()) * 12ull;
     auto tab = [](const FFTTable &t, size_t es) { return t.mem ? (unsigned long long)(4 * (size_t)t.d.L + 2 * (size_t)t.d.n) * es : 0ull; };
     const size_t es = P.elt();
@@ -419,6 +421,7 @@ void plan_destroy(Plan *p) {
     p->prof_flush();
     for (cudaEvent_t e : p->evpool) cudaEventDestroy(e);
     for (void *m : p->scratch) cudaFree(m);
+    tc_free(*p);
     free_fft_table(p->tx); free_fft_table(p->ty); free_fft_table(p->tz);
     free_fft4_table(p->tx4); free_fft4_table(p->ty4); free_fft4_table(p->tz4);
     if (p->dgeo) cudaFree(p->dgeo);

@@ -11,6 +11,7 @@
 namespace sg {
 
 struct Batch;  // batch.h
+struct TcState;  // tcdft.cu
 
 // Plans are FP64 or FP32; FF (float-float) is the precision of internal tables and kernels of
 // the precision form on FP64 plans.
@@ -90,6 +91,7 @@ struct Plan {
     void *dxtw = nullptr;
     FFTTable tx, ty, tz;      // lengths H = nx/2, ny, nz
     FFT4Table tx4, ty4, tz4;  // four-step tables of the same lengths (FP32 plans)
+    TcState *tc = nullptr;    // FP64 plans: digit-product transforms (tcdft.h), built on first use
     cudaStream_t stream = nullptr;
     // host transfers of several fields: copies on their own stream, double-buffered staging
     // (scratch slots kStageSlot, kStageSlot + 1) and events ordering copies with conversions

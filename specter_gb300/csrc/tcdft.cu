@@ -1,0 +1,912 @@
+// FP64 column transforms as exact integer-digit products on the tensor cores.
+//
+// FP64 arithmetic runs at 1/70 of the FP32 rate on this chip (503 GFMA/s), the tensor cores at
+// 1970 TFLOP/s in bf16.  A transform of length n = 2m splits by parity of the frequency (inputs
+// x[k] +- x[k+m]) and folds k <-> m-k, which leaves four real matrix products of about n/4 x n/4 per
+// column: cosines and sines of the even and of the odd frequencies, the same for real and imaginary
+// parts.  Inputs become 62-bit integers against their column's largest value, folded exactly, and
+// split into seven signed 9-bit digits (|d| <= 256, exact in bf16); the matrices are held as seven
+// digits too.  Products of digit i of the data and digit j of the matrix, i + j <= 6, accumulate in
+// FP32 in tensor memory, one accumulator per level i + j (levels 5 and 6 share one).  A level's sums
+// are integers below 2^24 (checked for every matrix when its table is built: levels 0 to 2 for any
+// data), so they are exact whatever the order; what is dropped is below 2^-60 of the column's
+// largest value.  The levels are put together as a 64-bit integer and rounded once to FP64.
+//
+// Error against long double, relative L2 (n = 58 .. 538): 5e-17 .. 1.7e-16, a double-precision FFT
+// 1.4e-16 .. 5e-16.
+#include <cmath>
+#include <complex>
+#include <cstring>
+#include <map>
+#include <string>
+#include <vector>
+
+#include <cuda_bf16.h>
+
+#include "fast.h"
+#include "ops.h"
+#include "tcdft.h"
+
+namespace sg {
+
+namespace {
+
+constexpr int kDig = 7;             // digits of data and matrix
+constexpr int kLev = 6;             // accumulators (levels 0..4, 5 + 6)
+constexpr int kLanes = 128;         // rows of an MMA: 64 columns, real and imaginary parts
+constexpr int kMaxNc = 80;          // outputs per block: kLev * 80 = 480 of 512 tensor-memory columns
+constexpr int kMaxLen = 550;        // every even length up to here holds the exactness bound of level 2
+constexpr int kAStage = kDig * kLanes * 16 * 2;  // bytes of one 16-deep step of data digits
+constexpr int kEpi = 512;           // epilogue threads
+constexpr int kDigThreads = 256;
+constexpr int kLoadWarp = kEpi / 32, kMmaWarp = kLoadWarp + 1;
+constexpr int kGemmThreads = kEpi + 64;
+constexpr int kNaN = 0x40000000;    // column exponent of a column that holds a non-finite value
+
+struct Dims {
+    int n, m, K, ks, nq[2], nchunk, nc, sh;
+};
+Dims dims(int n) {
+    Dims d;
+    d.n = n;
+    d.m = n / 2;
+    d.K = d.m / 2 + 1;
+    d.ks = (d.K + 15) / 16;
+    d.nq[0] = d.m / 2 + 1;
+    d.nq[1] = (d.m + 1) / 2;
+    const int np = (d.nq[0] + 15) / 16 * 16;
+    d.nchunk = (np + kMaxNc - 1) / kMaxNc;
+    d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
+    // results are below n * 2^14 level-0 units: as many fraction bits as fit 63 bits
+    int lg = 14;
+    while ((1ll << (lg + 1)) <= (long long)n << 14) lg++;
+    d.sh = 62 - lg;
+    if (d.sh > 44) d.sh = 44;
+    return d;
+}
+
+}  // namespace
+
+struct TcSet {
+    unsigned char *mat = nullptr;
+    size_t bytes = 0;
+    int expo = 0;
+    double post = 1.0;
+};
+
+struct TcState {
+    std::map<std::pair<int, double>, TcSet> sets;
+    unsigned char *ws = nullptr;  // digits
+    size_t ws_bytes = 0;
+    int *expo = nullptr;          // column exponents of the digits in ws
+    size_t expo_count = 0;
+    double2 *ext = nullptr;       // continuation rows of kMaxF fields
+    int *err = nullptr, *err_dev = nullptr;  // host-mapped: set by a kernel that gave up a wait
+};
+
+namespace {
+
+// ------------------------------------------------------------------ device helpers
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Waits for the phase, at most about two seconds; false when it gave up or the block is aborting.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, volatile int *abort_flag) {
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+        for (int i = 0; i < 64; i++)
+            if (mbar_try(bar, parity)) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > 4000000000ll) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// shared-memory operand descriptor, K-major without swizzle: 8-row x 16-byte core matrices, lbo
+// bytes apart along K and sbo bytes apart along the rows
+__device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned lbo, unsigned sbo) {
+    return (unsigned long long)((addr & 0x3FFFF) >> 4) | ((unsigned long long)(lbo >> 4) << 16) |
+           ((unsigned long long)(sbo >> 4) << 32) | (1ull << 46);
+}
+__device__ __forceinline__ void mma_bf16(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc,
+                                         unsigned acc) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(unsigned bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(float (&v)[4], unsigned addr) {
+    unsigned r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ size_t col_offset(const TcShape &s, unsigned c) {
+    const unsigned q = c / s.w;
+    return (size_t)q * s.s + (c - q * s.w);
+}
+
+// t * 2^q as a double, rounded to nearest (|t| < 2^63); the result's exponent is a normal number's.
+// The implicit bit carries into the exponent field, as does rounding up to the next power of two.
+__device__ __forceinline__ double plain_double(long long t, int q) {
+    const unsigned long long u = t < 0 ? -(unsigned long long)t : (unsigned long long)t;
+    const int lz = __clzll((long long)u);
+    const unsigned long long M = u << lz;
+    const unsigned long long mant = (M >> 11) + ((M >> 10) & 1);
+    unsigned long long b = ((unsigned long long)(unsigned)(1085 + q - lz) << 52) + mant;
+    b |= (unsigned long long)t & 0x8000000000000000ull;
+    return u ? __longlong_as_double((long long)b) : 0.0;
+}
+__device__ __forceinline__ double scaled_double(long long t, int q) {
+    if (q > -1023 && q < 960) return plain_double(t, q);
+    return scalbn(plain_double(t, 0), q);
+}
+
+// ------------------------------------------------------------------ digits
+struct DigArgs {
+    TcShape s;
+    TcJob job[kTcMaxJobs];
+    int m, K, ks;
+    unsigned tile0, ntile;  // tiles [tile0, tile0 + ntile) of every job
+    unsigned char *ws;
+    int *expo;              // [job][ntile * 64]
+};
+
+// Columns are split into digits of the four folded lists: memory traffic (8 bytes read and 14 written a
+// value) and the integer conversions beside it.
+//
+// A value (times k for the derivative) as an integer in units of 2^-60 of 2^(emax - 1022).
+template <bool DERIV>
+__device__ __forceinline__ long long fixed_point(double x, int k, int emax) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const unsigned hi = (unsigned)(b >> 32);
+    int e = (hi >> 20) & 0x7ff;
+    unsigned long long M = b & 0xfffffffffffffull;
+    if (e) M |= 1ull << 52;
+    else e = 1;
+    bool neg = (int)hi < 0;
+    int sh;
+    if (DERIV) {
+        if (k < 0) { k = -k; neg = !neg; }
+        M *= (unsigned)k;
+        sh = emax - e - 7;
+        if (sh < 0) { M <<= -sh; sh = 0; }
+    } else {
+        M <<= 7;
+        sh = emax - e;
+    }
+    M = sh < 64 ? M >> sh : 0;
+    return neg ? -(long long)M : (long long)M;
+}
+
+__device__ __forceinline__ void put_digits(unsigned char *dst, const long long (&v)[8]) {
+    unsigned long long w[8];
+    unsigned long long bias = 0;
+#pragma unroll
+    for (int i = 1; i < kDig; i++) bias += 256ull << (54 - 9 * i);
+#pragma unroll
+    for (int t = 0; t < 8; t++) w[t] = (unsigned long long)v[t] + bias;
+#pragma unroll
+    for (int i = 0; i < kDig; i++) {
+        unsigned r[4];
+#pragma unroll
+        for (int t = 0; t < 8; t += 2) {
+            float f[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                // 2^23 + u, scaled by 2^-9i through the exponent field, minus the same of the bias:
+                // d * 2^-9i exactly
+                unsigned u;
+                if (i == 0) u = (unsigned)((long long)w[t + h] >> 54) + 256u;
+                else u = (unsigned)(w[t + h] >> (54 - 9 * i)) & 511u;
+                const float off = (8388608.f + 256.f) / (float)(1ull << (9 * i));
+                f[h] = __uint_as_float(0x4B000000u - ((unsigned)(9 * i) << 23) | u) - off;
+            }
+            const __nv_bfloat162 p = __floats2bfloat162_rn(f[0], f[1]);
+            r[t / 2] = *reinterpret_cast<const unsigned *>(&p);
+        }
+        *reinterpret_cast<uint4 *>(dst + (size_t)i * kLanes * 32) = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
+// One block: LW lanes (LW / 2 columns) of a tile, all rows staged in shared memory once, so that the
+// largest value and the digits cost one read.  A thread owns one lane and eight consecutive k of the
+// lists, so that it writes whole 16-byte rows of core matrices; LW = 16 keeps three blocks on an SM
+// at n = 538 (69 KB), LW = 32 at up to half of that.
+template <bool DERIV, int LW>
+__device__ __forceinline__ void digits_body(const DigArgs &a, const TcJob &J, int job, const double *tile_s, int *s_e,
+                                            unsigned lt, int lane0) {
+    const int n = a.s.n, m = a.m;
+    const int l = threadIdx.x % LW, part = l & 1, lane = lane0 + l;
+    const double *x = tile_s + l;
+    // column exponents: every value (times k) is below 2^(e - 1022)
+    int emax = 0;
+    for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW) {
+        const double v = x[row * LW];
+        const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
+        int e = hi >> 20;
+        if (e == 0x7ff) e = kNaN;
+        else if (hi || __double2loint(v)) {
+            const unsigned top = ((hi & 0xfffffu) | (e ? 0x100000u : 0u)) + 1u;
+            e = max(e, 1);
+            if (DERIV) {
+                const int k = row < m ? row : n - row;
+                e = k ? max(e + 31 - __clz((int)(top * (unsigned)k)) - 20, 1) : 0;
+            }
+        }
+        emax = max(emax, e);
+    }
+    atomicMax(&s_e[l >> 1], emax);
+    __syncthreads();
+    emax = s_e[l >> 1];
+    if (emax == 0) emax = 1023;  // a column of zeros: any exponent
+    if (blockIdx.y == 0 && threadIdx.x < LW && part == 0)
+        a.expo[((size_t)job * a.ntile + lt) * 64 + (lane >> 1)] = emax;
+    if (emax >= kNaN) emax = 0x7ff;  // a non-finite column's digits are not used
+    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage;
+    // effective part: multiplying by i moves real data to imaginary lanes and imaginary data, negated,
+    // to real lanes; so does the sine list
+    const int epart = DERIV ? part ^ 1 : part;
+    const int row0 = DERIV ? lane ^ 1 : lane;
+    const bool flip = DERIV && part == 1;
+    const size_t st = (size_t)a.ks * kAStage;
+    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks; g += gridDim.y * (kDigThreads / LW)) {
+        unsigned char *d = tb + (size_t)(g >> 1) * kAStage + (size_t)(g & 1) * kLanes * 16;
+#pragma unroll 1
+        for (int par = 0; par < 2; par++) {  // even frequencies: x[k] + x[k+m]; odd: x[k] - x[k+m]
+            long long c[8], w[8];
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+                const int k = 8 * g + t;
+                c[t] = w[t] = 0;
+                if (k >= a.K) continue;
+                const bool self = k == 0 || 2 * k == m;
+                // row r as a wavenumber: r for r < m, r - n above
+                long long x0 = fixed_point<DERIV>(x[k * LW], k, emax);
+                long long x1 = fixed_point<DERIV>(x[(k + m) * LW], k - m, emax);
+                long long x2 = 0, x3 = 0;
+                if (!self) {
+                    x2 = fixed_point<DERIV>(x[(m - k) * LW], m - k, emax);
+                    x3 = fixed_point<DERIV>(x[(n - k) * LW], -k, emax);
+                }
+                if (par) { x1 = -x1; x3 = -x3; }
+                long long E = x0 + x1, E2 = x2 + x3;
+                if (flip) { E = -E; E2 = -E2; }
+                // even: cos gets E + E', sin E - E'; odd: cos O - O', sin O + O'
+                if (par) E2 = -E2;
+                c[t] = E + E2;
+                w[t] = E - E2;
+                if (par ? k == 0 : self) w[t] = 0;
+                if (par && 2 * k == m) c[t] = 0;
+                if (epart == 1) w[t] = -w[t];
+            }
+            put_digits(d + 2 * par * st + row0 * 16, c);
+            put_digits(d + (2 * par + 1) * st + (row0 ^ 1) * 16, w);
+        }
+    }
+}
+
+template <int LW>
+__global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_e[LW / 2];
+    const TcShape &s = a.s;
+    const int job = blockIdx.z;
+    const TcJob &J = a.job[job];
+    constexpr int kParts = kLanes / LW, kCols = LW / 2;
+    const unsigned lt = blockIdx.x / kParts;
+    const int lane0 = (blockIdx.x % kParts) * LW;
+    const int n0 = J.ext ? s.n - s.next : s.n;  // rows below n0 come from the field
+    if (threadIdx.x < kCols) s_e[threadIdx.x] = 0;
+    {
+        const int cc = threadIdx.x % kCols;
+        const unsigned c = (a.tile0 + lt) * 64 + lane0 / 2 + cc;
+        const bool live = c < s.ncol;
+        const size_t off = live ? col_offset(s, c) : 0;
+        const double2 *in = J.in + off, *ext = J.ext ? J.ext + off : nullptr;
+        double2 *dst = (double2 *)smem + cc;
+        for (int row = threadIdx.x / kCols; row < s.n; row += kDigThreads / kCols) {
+            if (live) cp_async<16>(dst + row * kCols, row < n0 ? in + (size_t)row * s.rs : ext + (size_t)(row - n0) * s.es);
+            else dst[row * kCols] = make_double2(0.0, 0.0);
+        }
+        async_commit();
+        async_wait();
+    }
+    __syncthreads();
+    if (J.deriv) digits_body<true, LW>(a, J, job, (const double *)smem, s_e, lt, lane0);
+    else digits_body<false, LW>(a, J, job, (const double *)smem, s_e, lt, lane0);
+}
+
+// ------------------------------------------------------------------ products
+struct GemmArgs {
+    TcShape s;
+    TcJob job[kTcMaxJobs];
+    int m, ks, nq[2], nchunk, nc, sh, nstage;
+    unsigned tile0, ntile, units;
+    const unsigned char *ws;
+    const int *expo;
+    int *err;
+};
+
+// A unit of work: one tile of 64 columns, one parity of the frequency, one chunk of nc outputs.  The
+// data digits are the M = 128 rows (64 columns x real, imaginary), the matrix digits the N = nc columns
+// of the MMAs; a pipeline of bulk copies feeds 28 MMAs a 16-deep step.  One block per SM walks over
+// units: the cosine product moves from tensor memory to shared memory as integers, the sine product to
+// registers, and while the next unit's MMAs run, their sum and difference (the frequencies f and n - f)
+// become doubles.  The MMAs (operand reads from shared memory: (128 + nc) * 32 bytes each) and the
+// integer work of the epilogue bound it.
+struct Unit {
+    int job, par, chunk;
+    unsigned lt;
+};
+__device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
+    Unit w;
+    w.par = u % 2;
+    u /= 2;
+    w.chunk = u % a.nchunk;
+    u /= a.nchunk;
+    w.lt = u % a.ntile;
+    w.job = u / a.ntile;
+    return w;
+}
+
+// the general form of an output: any exponent, a non-finite column, a further factor, an addend
+__device__ __noinline__ double output_general(long long t, int q, int e, double post, const double *add) {
+    double v = scaled_double(t, q);
+    if (e >= kNaN) v = __longlong_as_double(0x7ff8000000000000ll);
+    if (post != 1.0) v *= post;
+    if (add) v += *add;
+    return v;
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ unsigned long long bars[2 * 8 + 2];
+    __shared__ unsigned s_tmem;
+    __shared__ int s_abort;
+    const TcShape &s = a.s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nc = a.nc;
+    const unsigned b_bytes = kDig * nc * 32, stage_bytes = kAStage + b_bytes;
+    const unsigned full = smem_u32(bars), empty = full + 8 * 8, accfull = full + 16 * 8, accempty = accfull + 8;
+    unsigned tcols = 32;
+    while (tcols < (unsigned)(kLev * nc)) tcols *= 2;
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int i = 0; i < a.nstage; i++) {
+            mbar_init(full + 8 * i, 1);
+            mbar_init(empty + 8 * i, 1);
+        }
+        mbar_init(accfull, 1);
+        mbar_init(accempty, kEpi);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(tcols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const unsigned tmem = s_tmem;
+    volatile int *ab = &s_abort;
+    const int nit = 2 * a.ks;  // steps of a unit: cosine list, then sine list
+    if (warp == kLoadWarp) {
+        if (lane == 0) {
+            int it = 0;  // steps issued so far, over all units
+            bool ok = true;
+            for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+                const Unit w = unit_of(a, u);
+                const unsigned char *A = a.ws + (((size_t)w.job * a.ntile + w.lt) * 4 + 2 * w.par) * a.ks * kAStage;
+                const unsigned char *B = a.job[w.job].mat + ((size_t)w.par * 2 * a.nchunk + w.chunk) * a.ks * b_bytes;
+                for (int i = 0; i < nit; i++, it++) {
+                    const int st = it % a.nstage, round = it / a.nstage;
+                    if (round && !mbar_wait(empty + 8 * st, (round - 1) & 1, ab)) { ok = false; break; }
+                    const int list = i >= a.ks;
+                    const unsigned dst = smem_u32(smem) + st * stage_bytes;
+                    mbar_expect(full + 8 * st, stage_bytes);
+                    bulk_load(dst, A + (size_t)i * kAStage, kAStage, full + 8 * st);
+                    bulk_load(dst + kAStage, B + ((size_t)list * a.nchunk * a.ks + (i - list * a.ks)) * b_bytes, b_bytes,
+                              full + 8 * st);
+                }
+            }
+            if (!ok)  // giving up: this block's own copies land before it ends
+                for (int i = max(0, it - a.nstage); i < it; i++) {
+                    const long long t0 = clock64();
+                    while (!mbar_try(full + 8 * (i % a.nstage), (i / a.nstage) & 1) && clock64() - t0 < 2000000000ll) {}
+                }
+        }
+    } else if (warp == kMmaWarp) {
+        if (lane == 0) {
+            // D FP32, A and B bf16, both K-major, N = nc, M = 128
+            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nc >> 3) << 17) | (8u << 24);
+            int it = 0, lists = 0;
+            bool ok = true;
+            for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x)
+                for (int i = 0; i < nit; i++, it++) {
+                    const int st = it % a.nstage, round = it / a.nstage;
+                    const bool first = i == 0 || i == a.ks;
+                    if (first && lists) {  // the previous list's sums have left tensor memory
+                        ok = mbar_wait(accempty, (lists - 1) & 1, ab);
+                        if (!ok) break;
+                        fence_after();
+                    }
+                    ok = mbar_wait(full + 8 * st, round & 1, ab);
+                    if (!ok) break;
+                    fence_after();
+                    const unsigned sa = smem_u32(smem) + st * stage_bytes, sb = sa + kAStage;
+// neighbours in this order add to different accumulators
+#pragma unroll
+                    for (int d = 0; d < kDig; d++)
+#pragma unroll
+                        for (int j = 0; j < kDig - d; j++) {
+                            const int acc = d + j < kLev ? d + j : kLev - 1;
+                            const bool fresh = first && d == 0 && j < kLev;
+                            mma_bf16(tmem + acc * nc, smem_desc(sa + d * (kLanes * 32), kLanes * 16, 128),
+                                     smem_desc(sb + j * (nc * 32), nc * 16, 128), idesc, fresh ? 0u : 1u);
+                        }
+                    mma_commit(empty + 8 * st);
+                    if (i == a.ks - 1 || i == nit - 1) {
+                        mma_commit(accfull);
+                        lists++;
+                    }
+                }
+        }
+    } else {
+        // 16 warps: quarter q of the lanes, every fourth group of 4 outputs
+        const int quad = warp & 3, g0 = warp >> 2, ngr = nc / 16;
+        const int r = quad * 32 + lane;
+        const unsigned taddr = tmem + ((unsigned)(quad * 32) << 16);
+        long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;  // [nc][128]
+        const int sh = a.sh;
+        const float fsh = (float)(1ull << sh);
+        // the levels of 4 outputs as integers in units of 2^-sh
+        auto gather = [&](int col, long long (&u)[4]) {
+            float l[kLev][4];
+#pragma unroll
+            for (int v = 0; v < kLev; v++) tmem_ld4(l[v], taddr + v * nc + col);
+            tmem_wait_ld();
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const int i0 = __float2int_rn(l[0][t]), i1 = __float2int_rn(l[1][t] * 512.f),
+                          i2 = __float2int_rn(l[2][t] * 262144.f), i3 = __float2int_rn(l[3][t] * 134217728.f),
+                          i4 = __float2int_rn(l[4][t] * 68719476736.f), i5 = __float2int_rn(l[5][t] * fsh);
+                const long long A = (long long)i0 * 262144 + ((long long)i1 * 512 + i2);
+                u[t] = (A << (sh - 18)) + ((long long)i3 * (1 << (sh - 27)) + ((long long)i4 * (1 << (sh - 36)) + i5));
+            }
+        };
+        int lists = 0;
+        bool ok = true;
+        for (unsigned u = blockIdx.x; u < a.units; u += gridDim.x) {
+            const Unit w = unit_of(a, u);
+            const TcJob &J = a.job[w.job];
+            ok = __all_sync(~0u, ok && mbar_wait(accfull, lists & 1, ab));
+            if (!ok) break;
+            lists++;
+            fence_after();
+#pragma unroll 1
+            for (int gi = 0; gi < ngr; gi++) {
+                const int col = (g0 + 4 * gi) * 4;
+                long long P[4];
+                gather(col, P);
+#pragma unroll
+                for (int t = 0; t < 4; t++) Ps[(col + t) * kLanes] = P[t];
+            }
+            fence_before();
+            mbar_arrive(accempty);
+            ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
+            if (!ok) break;
+            lists++;
+            fence_after();
+            long long Q[5][4];
+#pragma unroll
+            for (int gi = 0; gi < 5; gi++)
+                if (gi < ngr) gather((g0 + 4 * gi) * 4, Q[gi]);
+            fence_before();
+            mbar_arrive(accempty);
+            const unsigned c = (a.tile0 + w.lt) * 64 + (r >> 1);
+            const bool live = c < s.ncol;
+            const size_t off = live ? 2 * col_offset(s, c) + (r & 1) : 0;
+            const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * 64 + (r >> 1)];
+            const int q = e - 1022 - 14 - sh + J.expo;
+            double *out = (double *)J.out + off;
+            const double *add = J.add ? (const double *)J.add + off : nullptr;
+            // every result's exponent 1086 + q - lz, 0 <= lz < 64, is a normal number's
+            const bool plain = e < kNaN && q > -1023 && q < 960 && J.post == 1.0 && !add;
+            auto put = [&](int row, long long t) {
+                if (row >= s.nrows || !live) return;
+                const size_t o = 2 * (size_t)row * s.rs;
+                out[o] = plain ? plain_double(t, q) : output_general(t, q, e, J.post, add ? add + o : nullptr);
+            };
+#pragma unroll
+            for (int gi = 0; gi < 5; gi++)
+                if (gi < ngr) {
+                    const int col = (g0 + 4 * gi) * 4;
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        const int j = w.chunk * nc + col + t;
+                        if (j < a.nq[w.par]) {
+                            const int f = 2 * j + w.par;
+                            const long long p = Ps[(col + t) * kLanes], d = s.sign > 0 ? Q[gi][t] : -Q[gi][t];
+                            put(f, p + d);
+                            if (f && 2 * f != s.n) put(s.n - f, p - d);
+                        }
+                    }
+                }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_abort) {
+        *(volatile int *)a.err = 1;
+        __threadfence_system();
+    }
+    if (warp == kMmaWarp) {
+        if (s_abort) {  // issued MMAs end before their tensor memory is given back
+            const long long t0 = clock64();
+            while (clock64() - t0 < 2000000ll) {}
+        }
+        __syncwarp();
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols));
+    }
+}
+
+// FC-Gram continuation rows (src/fftp/fftp.fpp:755-773) of every column, FP64: a thread per real
+// lane; bound by the FP64 pipe (2 C d multiply-adds a lane).
+struct ContArgs {
+    const double *in[kMaxF];
+    double *ext[kMaxF];
+};
+__global__ void __launch_bounds__(128) k_continuation(Geo g, ContArgs a) {
+    const int C = g.cz, d = g.oz;
+    const size_t ps = 2 * (size_t)g.ny * g.ldx;
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= ps) return;
+    const double *in = a.in[blockIdx.y] + q;
+    double *ext = a.ext[blockIdx.y] + q;
+    double t[kMaxOz], b[kMaxOz];
+#pragma unroll
+    for (int j = 0; j < kMaxOz; j++)
+        if (j < d) {
+            t[j] = in[(size_t)(g.nzp - d + j) * ps];
+            b[j] = in[(size_t)(d - 1 - j) * ps];
+        }
+    for (int i = 0; i < C; i++) {
+        double x = __ldg(g.dir + i) * t[0] + __ldg(g.dir + (C - 1 - i)) * b[0];
+#pragma unroll
+        for (int j = 1; j < kMaxOz; j++)
+            if (j < d) x = x + __ldg(g.dir + i + C * j) * t[j] + __ldg(g.dir + (C - 1 - i) + C * j) * b[j];
+        ext[(size_t)i * ps] = x;
+    }
+}
+
+// ------------------------------------------------------------------ tables
+// digits [angle][7] of factor * cos, factor * sin at 2 pi t / n -> the matrices of one set
+__global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, int K, int ks, int nq0, int nq1, int nchunk,
+                           int nc) {
+    const long long total = 4ll * nchunk * ks * 16 * nc;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
+        const int kk = (int)(q % 16), col = (int)(q / 16 % nc);
+        long long t = q / 16 / nc;
+        const int step = (int)(t % ks);
+        t /= ks;
+        const int chunk = (int)(t % nchunk), list = (int)(t / nchunk % 2), par = (int)(t / nchunk / 2);
+        const int k = 16 * step + kk, j = chunk * nc + col;
+        const bool on = k < K && j < (par ? nq1 : nq0);
+        const int ang = on ? (int)((long long)(2 * j + par) * k % n) : 0;
+        __nv_bfloat16 *dst = mat + (((long long)(par * 2 + list) * nchunk + chunk) * ks + step) * (kDig * 16 * nc) +
+                             (kk / 8) * (nc * 8) + col * 8 + kk % 8;
+        for (int i = 0; i < kDig; i++)
+            dst[(long long)i * nc * 16] = on ? dig[((long long)list * n + ang) * kDig + i] : __float2bfloat16(0.f);
+    }
+}
+
+// cos and sin of 2 pi t / n for every t from one octant, in long double
+void circle(int n, std::vector<long double> &c, std::vector<long double> &s) {
+    const long double pi = 3.14159265358979323846264338327950288L;
+    c.assign(n, 0.0L);
+    s.assign(n, 0.0L);
+    std::map<int, std::pair<long double, long double>> cache;  // by 8 t / n folded into the first octant
+    for (int t = 0; t < n; t++) {
+        // angle = 2 pi t / n = (pi / 4) (8 t / n): octant o and remainder u = 8 t - o n, in units of pi / (4 n)
+        const int o = 8 * t / n, u = 8 * t - o * n;
+        const int v = o & 1 ? n - u : u;
+        auto it = cache.find(v);
+        if (it == cache.end()) {
+            const long double x = pi * (long double)v / (4.0L * (long double)n);
+            it = cache.insert({v, {cosl(x), sinl(x)}}).first;
+        }
+        long double a = it->second.first, b = it->second.second;
+        switch (o) {
+            case 0: break;
+            case 1: std::swap(a, b); break;
+            case 2: { const long double w = a; a = -b; b = w; break; }
+            case 3: a = -a; break;
+            case 4: a = -a; b = -b; break;
+            case 5: { const long double w = a; a = -b; b = -w; break; }
+            case 6: { const long double w = a; a = b; b = -w; break; }
+            default: b = -b; break;
+        }
+        c[t] = a;
+        s[t] = b;
+    }
+}
+
+void matrix_digits(long double v, int d[kDig]) {
+    const long long V = llrintl(v * 4611686018427387904.0L);  // 2^62
+    unsigned long long bias = 0;
+    for (int i = 1; i < kDig; i++) bias += 256ull << (54 - 9 * i);
+    const unsigned long long w = (unsigned long long)V + bias;
+    d[0] = (int)((long long)w >> 54);
+    for (int i = 1; i < kDig; i++) d[i] = (int)((w >> (54 - 9 * i)) & 511) - 256;
+}
+
+// Levels 0, 1 and 2 of a column's sums stay below 2^24 for any data digits (|d| <= 256).
+bool exact_levels(const Dims &D, const std::vector<int> &dc, const std::vector<int> &ds) {
+    for (int par = 0; par < 2; par++)
+        for (int j = 0; j < D.nq[par]; j++) {
+            long long sc = 0, ss = 0;
+            for (int k = 0; k < D.K; k++) {
+                const size_t t = (size_t)((long long)(2 * j + par) * k % D.n) * kDig;
+                for (int i = 0; i < 3; i++) {
+                    sc += std::abs(dc[t + i]);
+                    ss += std::abs(ds[t + i]);
+                }
+            }
+            if (256 * std::max(sc, ss) > (1ll << 24)) return false;
+        }
+    return true;
+}
+
+TcState *state(Plan &P) {
+    if (!P.tc) P.tc = new TcState();
+    return P.tc;
+}
+
+}  // namespace
+
+bool tc_length_ok(int n) { return n >= 32 && n <= kMaxLen && n % 2 == 0; }
+
+void tc_job_set(TcJob &j, const TcSet *s) {
+    j.mat = s->mat;
+    j.expo = s->expo;
+    j.post = s->post;
+}
+
+const TcSet *tc_set(Plan &P, int n, double factor, int *status) {
+    *status = OK;
+    TcState *S = state(P);
+    auto it = S->sets.find({n, factor});
+    if (it != S->sets.end()) return &it->second;
+    const Dims D = dims(n);
+    std::vector<long double> c, s;
+    circle(n, c, s);
+    TcSet set;
+    std::vector<int> dc((size_t)n * kDig), ds((size_t)n * kDig);
+    // factor = scale * 2^expo with scale in (1/2, 1]; a smaller scale where the digits of this one miss
+    // the exactness bound, and the plain matrices with a multiplication after them where all do
+    bool ok = false;
+    int ex = 0;
+    double fr = frexp(factor, &ex);
+    if (fr == 0.5) { fr = 1.0; ex -= 1; }
+    for (int t = 0; t < 5 && !ok; t++) {
+        const long double sc = t < 4 ? (long double)fr / (long double)(1 << t) : 1.0L;
+        for (int k = 0; k < n; k++) {
+            matrix_digits(c[k] * sc, &dc[(size_t)k * kDig]);
+            matrix_digits(s[k] * sc, &ds[(size_t)k * kDig]);
+        }
+        set.expo = t < 4 ? ex + t : 0;
+        set.post = t < 4 ? 1.0 : factor;
+        ok = exact_levels(D, dc, ds);
+    }
+    if (!ok) { set_error("digit tables: exactness bound"); *status = ERR_SHAPE; return nullptr; }
+    std::vector<__nv_bfloat16> h(2 * (size_t)n * kDig);
+    for (int l = 0; l < 2; l++)
+        for (size_t q = 0; q < (size_t)n * kDig; q++) {
+            const int i = (int)(q % kDig);
+            h[(size_t)l * n * kDig + q] = __float2bfloat16(ldexpf((float)(l ? ds[q] : dc[q]), -9 * i));
+        }
+    set.bytes = 4ull * D.nchunk * D.ks * kDig * 32 * D.nc;
+    __nv_bfloat16 *dig = nullptr;
+    if (cudaMalloc(&set.mat, set.bytes) != cudaSuccess || cudaMalloc(&dig, h.size() * 2) != cudaSuccess) {
+        cudaGetLastError();
+        if (set.mat) cudaFree(set.mat);
+        set_error("out of device memory (digit tables)");
+        *status = ERR_OOM;
+        return nullptr;
+    }
+    cudaMemcpyAsync(dig, h.data(), h.size() * 2, cudaMemcpyHostToDevice, P.stream);
+    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, dig, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc);
+    const cudaError_t e = cudaStreamSynchronize(P.stream);  // the host digits go out of scope
+    cudaFree(dig);
+    if (e != cudaSuccess || (*status = check_launch("digit tables"))) {
+        cudaFree(set.mat);
+        if (!*status) *status = ERR_CUDA;
+        return nullptr;
+    }
+    return &(S->sets[{n, factor}] = set);
+}
+
+// The digit workspace of a plan has one size for its lifetime (captured graphs hold its address):
+// what its largest axis needs for all columns of eight transforms, at most 2 GiB; longer launches run
+// in ranges of tiles.
+static int workspace(Plan &P) {
+    TcState *S = state(P);
+    if (S->ws) return OK;
+    size_t want = 0, tiles = 0;
+    const int len[2] = {P.nz, P.ny};
+    const size_t cols[2] = {(size_t)P.ny * P.ldx, (size_t)P.nz * P.ldx};
+    for (int i = 0; i < 2; i++) {
+        if (!tc_length_ok(len[i])) continue;
+        const Dims D = dims(len[i]);
+        const size_t nt = (cols[i] + 63) / 64 * kTcMaxJobs;
+        const size_t per = 4ull * D.ks * kAStage;
+        size_t b = nt * per;
+        if (b > (2ull << 30)) b = std::max<size_t>((2ull << 30) / per * per, (size_t)kTcMaxJobs * per);
+        if (b > want) want = b;
+        if (b / per > tiles) tiles = b / per;
+    }
+    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * 64 * sizeof(int)) != cudaSuccess ||
+        cudaHostAlloc(&S->err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&S->err_dev, S->err, 0) != cudaSuccess) {
+        cudaGetLastError();
+        if (S->ws) cudaFree(S->ws);
+        if (S->expo) cudaFree(S->expo);
+        if (S->err) cudaFreeHost(S->err);
+        S->ws = nullptr;
+        S->expo = nullptr;
+        S->err = nullptr;
+        set_error("out of device memory (digit workspace)");
+        return ERR_OOM;
+    }
+    *S->err = 0;
+    S->ws_bytes = want;
+    S->expo_count = tiles * 64;
+    return OK;
+}
+
+int tc_status(const Plan &P) {
+    if (!P.tc || !P.tc->err || !*(volatile int *)P.tc->err) return OK;
+    set_error("a transform kernel gave up a wait");
+    return ERR_CUDA;
+}
+
+int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes) {
+    if (int st = workspace(P)) return st;
+    if (int st = tc_status(P)) return st;
+    TcState *S = P.tc;
+    const Dims D = dims(s.n);
+    const size_t per = 4ull * D.ks * kAStage;
+    const unsigned tiles = (s.ncol + 63) / 64;
+    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / 64);
+    // all jobs at once when they fit, else job by job in ranges of tiles
+    const int jstep = (size_t)tiles * njobs <= cap ? njobs : 1;
+    const unsigned tstep = jstep == njobs ? tiles : (unsigned)std::min<size_t>(tiles, cap);
+    const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)D.nc * kLanes * 8;
+    const int nstage = std::min(8, (int)((226 * 1024 - psize) / stage));
+    const size_t smem = (size_t)nstage * stage + psize;
+    cudaFuncSetAttribute(k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int lw = s.n <= 300 ? 32 : 16;
+    const size_t dsm = (size_t)s.n * lw * 8;
+    auto kd = lw == 32 ? k_digits<32> : k_digits<16>;
+    cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
+    for (int j0 = 0; j0 < njobs; j0 += jstep)
+        for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
+            const unsigned nt = std::min(tstep, tiles - t0);
+            DigArgs d{};
+            GemmArgs g{};
+            d.s = g.s = s;
+            for (int j = 0; j < jstep; j++) d.job[j] = g.job[j] = jobs[j0 + j];
+            d.m = g.m = D.m;
+            d.K = D.K;
+            d.ks = g.ks = D.ks;
+            d.tile0 = g.tile0 = t0;
+            d.ntile = g.ntile = nt;
+            d.ws = S->ws;
+            g.ws = S->ws;
+            d.expo = S->expo;
+            g.expo = S->expo;
+            g.nq[0] = D.nq[0];
+            g.nq[1] = D.nq[1];
+            g.nchunk = D.nchunk;
+            g.nc = D.nc;
+            g.sh = D.sh;
+            g.nstage = nstage;
+            g.err = S->err_dev;
+            g.units = nt * 2 * D.nchunk * jstep;
+            // small launches: split a tile's lists over blocks (each reads the columns itself)
+            const int blocks = (int)nt * (kLanes / lw) * jstep, rounds = (2 * D.ks * lw + kDigThreads - 1) / kDigThreads;
+            int split = 1;
+            while (split < rounds && blocks * split < 304) split++;
+            const double share = (double)nt * jstep / ((double)tiles * njobs);
+            {
+                Launch L(P, "digits", share * bytes * 0.5 + (double)nt * jstep * per);
+                kd<<<dim3(nt * (kLanes / lw), split, jstep), kDigThreads, dsm, P.stream>>>(d);
+            }
+            {
+                Launch L(P, name, share * bytes);
+                k_gemm<<<std::min(g.units, 152u), kGemmThreads, smem, P.stream>>>(g);
+            }
+        }
+    return check_launch(name);
+}
+
+int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf) {
+    TcState *S = state(P);
+    const size_t rows = (size_t)P.cz * P.ny * P.ldx;
+    if (!S->ext && cudaMalloc(&S->ext, kMaxF * rows * sizeof(double2)) != cudaSuccess) {
+        cudaGetLastError();
+        S->ext = nullptr;
+        set_error("out of device memory (continuation rows)");
+        return ERR_OOM;
+    }
+    ContArgs a{};
+    for (int f = 0; f < nf; f++) {
+        a.in[f] = (const double *)in[f];
+        a.ext[f] = (double *)(S->ext + f * rows);
+        ext[f] = S->ext + f * rows;
+    }
+    const size_t per = 2 * (size_t)P.ny * P.ldx;
+    {
+        Launch L(P, "continuation", nf * 8.0 * per * (2 * P.oz + P.cz));
+        k_continuation<<<dim3((unsigned)((per + 127) / 128), nf), 128, 0, P.stream>>>(P.geo, a);
+    }
+    return check_launch("continuation");
+}
+
+void tc_free(Plan &P) {
+    if (!P.tc) return;
+    for (auto &e : P.tc->sets) cudaFree(e.second.mat);
+    if (P.tc->ws) cudaFree(P.tc->ws);
+    if (P.tc->expo) cudaFree(P.tc->expo);
+    if (P.tc->ext) cudaFree(P.tc->ext);
+    if (P.tc->err) cudaFreeHost(P.tc->err);
+    delete P.tc;
+    P.tc = nullptr;
+}
+
+unsigned long long tc_bytes(const Plan &P) {
+    if (!P.tc) return 0;
+    unsigned long long b = P.tc->ws_bytes + P.tc->expo_count * sizeof(int);
+    if (P.tc->ext) b += (unsigned long long)kMaxF * P.cz * P.ny * P.ldx * sizeof(double2);
+    for (const auto &e : P.tc->sets) b += e.second.bytes;
+    return b;
+}
+
+}  // namespace sg

@@ -1,0 +1,46 @@
+// FP64 discrete Fourier transforms as exact integer-digit products on the tensor cores (tcdft.cu).
+#pragma once
+
+#include "plan.h"
+
+namespace sg {
+
+constexpr int kTcMaxJobs = 8;  // column transforms per launch
+
+// One column transform of a launch: out = factor * DFT^sign(in) over rows (row stride rs, in
+// complex elements), factor taken from the table set; deriv = 1 first multiplies row k by i * k
+// (k in [-n/2, n/2)), the table set's factor holding the wavenumber unit.
+struct TcJob {
+    const double2 *in;
+    double2 *out;
+    const double2 *add;   // added to the result when not null (same layout as out)
+    const double2 *ext;   // rows [n - next, n) of the input come from here when not null
+    const unsigned char *mat;  // matrix digits of the table set
+    int deriv, expo;      // expo: power of two of the set's factor
+    double post;          // further factor applied to the result (1: none)
+};
+
+// Columns: column c of a launch is at element (c / w) * s + c % w of a field, c in [0, ncol).
+struct TcShape {
+    int n, sign, nrows;         // nrows: rows of the result that are written
+    int next;                   // rows taken from ext
+    unsigned ncol, w, s, rs;    // rs: row stride of in and out
+    unsigned es;                // row stride of ext (its columns are laid out as the field's)
+};
+
+// true when length n has digit-product transforms (FP64 plans)
+bool tc_length_ok(int n);
+// the table set of length n scaled by `factor`; built on first use
+struct TcSet;
+const TcSet *tc_set(Plan &P, int n, double factor, int *status);
+void tc_job_set(TcJob &j, const TcSet *s);
+int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes);
+// continuation rows of FC-Gram columns of nf <= kMaxF fields, in a buffer of the plan:
+// ext[f][(i * ny + ky) * ldx + kx], i < cz
+int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf);
+void tc_free(Plan &P);
+unsigned long long tc_bytes(const Plan &P);
+// non-zero when a kernel of the plan gave up a wait (checked after synchronising)
+int tc_status(const Plan &P);
+
+}  // namespace sg
