@@ -69,77 +69,6 @@ static int two_outputs(void *const out0[], void *const out1[], int nf) {
     return 0;
 }
 
-// FP64 passes over the digit-product transforms (tcdft.cu).  They serve every even length of 32 to
-// 550: at all of them they are faster than the FP64 Stockham engine, which the FP64 pipe bounds.
-// kNoFast: a form that they do not take (another length, a scale on part of the rows).
-static int tc_add(Plan &P, TcJob *jobs, int *nj, int n, double factor, const void *in, void *out, const void *add,
-                  int deriv, const double2 *ext) {
-    int st = OK;
-    const TcSet *set = tc_set(P, n, factor, &st);
-    if (!set) return st;
-    TcJob &j = jobs[(*nj)++];
-    j = TcJob{};
-    j.in = (const double2 *)in;
-    j.out = (double2 *)out;
-    j.add = (const double2 *)add;
-    j.ext = ext;
-    j.deriv = deriv;
-    tc_job_set(j, set);
-    return OK;
-}
-
-static TcShape tc_z_shape(const Plan &P, int sign, int nrows) {
-    TcShape s{};
-    s.n = P.nz;
-    s.sign = sign;
-    s.nrows = nrows;
-    s.ncol = s.w = s.s = s.rs = s.es = (unsigned)P.ny * P.ldx;
-    return s;
-}
-
-static int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes) {
-    if (!tc_length_ok(P.nz) || (a.scale_rows > 0 && a.scale_rows < a.nrows)) return kNoFast;
-    const double sc = a.scale_rows > 0 ? a.scale : 1.0;
-    TcJob jobs[kTcMaxJobs];
-    int nj = 0;
-    // derivatives first: out0 may alias in
-    for (int f = 0; f < nf; f++)
-        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, P.Dkz * sc, a.in[f], a.out1[f], nullptr, 1, nullptr));
-    for (int f = 0; f < nf; f++)
-        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, sc, a.in[f], a.out0[f], a.add[f], 0, nullptr));
-    return tc_run(P, tc_z_shape(P, +1, a.nrows), jobs, nj, "z_inverse", bytes);
-}
-
-static int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
-    if (!tc_length_ok(P.nz) || a.in_scale != 1.0) return kNoFast;
-    const double2 *ext[kMaxF];
-    SG_TRY(tc_continuation(P, a.in, ext, nf));
-    TcJob jobs[kTcMaxJobs];
-    int nj = 0;
-    for (int f = 0; f < nf; f++) SG_TRY(tc_add(P, jobs, &nj, P.nz, 1.0, a.in[f], a.out[f], nullptr, 0, ext[f]));
-    TcShape s = tc_z_shape(P, -1, P.nz);
-    s.next = P.cz;
-    return tc_run(P, s, jobs, nj, "z_forward", bytes);
-}
-
-static int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes) {
-    if (!tc_length_ok(P.ny)) return kNoFast;
-    TcJob jobs[kTcMaxJobs];
-    int nj = 0;
-    for (int f = 0; f < nf; f++)
-        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, P.Dky * a.scale, a.in[f], a.out1[f], nullptr, 1, nullptr));
-    for (int f = 0; f < nf; f++)
-        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, a.scale, a.in[f], a.out0[f], nullptr, 0, nullptr));
-    TcShape s{};
-    s.n = P.ny;
-    s.sign = a.sign;
-    s.nrows = P.ny;
-    s.w = s.rs = P.ldx;
-    s.s = (unsigned)P.ny * P.ldx;
-    s.ncol = (unsigned)nplanes * P.ldx;
-    return tc_run(P, s, jobs, nj, a.sign < 0 ? "y_forward" : "y_inverse", bytes);
-}
-
 template <typename T>
 static int launch_z_inverse(Plan &P, const ZInvArgs &a0, int nf) {
     const size_t es = sizeof(C2<T>);
@@ -235,7 +164,9 @@ static int launch_x_nl(Plan &P, const XNLArgs &a) {
     // rows read: 3 velocity rows (+ theta), d/dy and d/dz rows of each component; written: NL rows
     const double nin = 3 + (a.c1 == 4 ? 1 : 0) + 2 * nc;
     const double bytes = cplx_rows(P, a.nrows) * (nin + nc);
-    const int fst = fast_x_nl(P, a, bytes);
+    int fst = kNoFast;
+    if constexpr (!is_f64<T>) fst = fast_x_nl(P, a, bytes);
+    else fst = tc_x_nonlinear(P, a, bytes);
     if (fst != kNoFast) return fst;
     set_smem(k_x_nonlinear<T, GenericFFT<T>>, sm);
     Launch L(P, "x_nonlinear", bytes);

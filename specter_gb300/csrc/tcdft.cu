@@ -41,7 +41,10 @@ constexpr int kEpi = 512;           // epilogue threads
 constexpr int kDigThreads = 256;
 constexpr int kLoadWarp = kEpi / 32, kMmaWarp = kLoadWarp + 1;
 constexpr int kGemmThreads = kEpi + 64;
-constexpr int kNaN = 0x40000000;    // column exponent of a column that holds a non-finite value
+constexpr int kNaN = 0x40000000;    // exponent of a column that holds a non-finite value
+
+// what a launch transforms: complex columns; real rows to half spectra; half spectra to real rows
+enum { kCol = 0, kR2C = 1, kC2R = 2 };
 
 struct Dims {
     int n, m, K, ks, nq[2], nchunk, nc, sh;
@@ -57,11 +60,10 @@ Dims dims(int n) {
     const int np = (d.nq[0] + 15) / 16 * 16;
     d.nchunk = (np + kMaxNc - 1) / kMaxNc;
     d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
-    // results are below n * 2^14 level-0 units: as many fraction bits as fit 63 bits
-    int lg = 14;
-    while ((1ll << (lg + 1)) <= (long long)n << 14) lg++;
-    d.sh = 62 - lg;
-    if (d.sh > 44) d.sh = 44;
+    // results are below (n + 2) * sqrt(2) * 2^14 level-0 units (each input is below 2^14 of them, twice
+    // that in a half spectrum): as many fraction bits as fit 63 bits
+    d.sh = 44;
+    while ((n + 2) * 1.41421357 * 16384.0 * (double)(1ll << d.sh) >= 9.2233720368547e18) d.sh--;
     return d;
 }
 
@@ -75,11 +77,13 @@ struct TcSet {
 };
 
 struct TcState {
-    std::map<std::pair<int, double>, TcSet> sets;
+    std::map<std::pair<int, double>, TcSet> sets;  // by length (negative: half spectrum to real) and factor
     unsigned char *ws = nullptr;  // digits
     size_t ws_bytes = 0;
     int *expo = nullptr;          // column exponents of the digits in ws
     size_t expo_count = 0;
+    double *phys = nullptr;       // physical rows of the nonlinear term's x pass, one range of tiles
+    size_t phys_tiles = 0;        // tiles of it per field
     double2 *ext = nullptr;       // continuation rows of kMaxF fields
     int *err = nullptr, *err_dev = nullptr;  // host-mapped: set by a kernel that gave up a wait
 };
@@ -184,7 +188,7 @@ struct DigArgs {
     int m, K, ks;
     unsigned tile0, ntile;  // tiles [tile0, tile0 + ntile) of every job
     unsigned char *ws;
-    int *expo;              // [job][ntile * 64]
+    int *expo;              // [job][ntile][128 lanes]
 };
 
 // Columns are split into digits of the four folded lists: memory traffic (8 bytes read and 14 written a
@@ -244,45 +248,43 @@ __device__ __forceinline__ void put_digits(unsigned char *dst, const long long (
     }
 }
 
-// One block: LW lanes (LW / 2 columns) of a tile, all rows staged in shared memory once, so that the
-// largest value and the digits cost one read.  A thread owns one lane and eight consecutive k of the
-// lists, so that it writes whole 16-byte rows of core matrices; LW = 16 keeps three blocks on an SM
-// at n = 538 (69 KB), LW = 32 at up to half of that.
-template <bool DERIV, int LW>
-__device__ __forceinline__ void digits_body(const DigArgs &a, const TcJob &J, int job, const double *tile_s, int *s_e,
-                                            unsigned lt, int lane0) {
+// the exponent field e of a bound: |x| (times k) < 2^(e - 1022); 0 for zero
+template <bool DERIV>
+__device__ __forceinline__ int value_exponent(double v, int k) {
+    const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
+    int e = hi >> 20;
+    if (e == 0x7ff) return kNaN;
+    if (!hi && !__double2loint(v)) return 0;
+    const unsigned top = ((hi & 0xfffffu) | (e ? 0x100000u : 0u)) + 1u;
+    e = max(e, 1);
+    if (DERIV) e = k ? max(e + 31 - __clz((int)(top * (unsigned)abs(k))) - 20, 1) : 0;
+    return e;
+}
+
+// Digits of LW lanes staged in shared memory (x[row * LW + l]), so that the largest value and the
+// digits cost one read of the field.  A thread owns one lane and eight consecutive k of the lists, so
+// that it writes whole 16-byte rows of core matrices.  REAL: lanes are real rows; else lanes are the
+// real and imaginary parts of columns.
+template <bool DERIV, bool REAL, int LW>
+__device__ __forceinline__ void digits_body(const DigArgs &a, int job, const double *tile_s, int *s_e, unsigned lt,
+                                            int lane0) {
     const int n = a.s.n, m = a.m;
-    const int l = threadIdx.x % LW, part = l & 1, lane = lane0 + l;
+    const int l = threadIdx.x % LW, part = REAL ? 0 : l & 1, lane = lane0 + l;
     const double *x = tile_s + l;
-    // column exponents: every value (times k) is below 2^(e - 1022)
     int emax = 0;
-    for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW) {
-        const double v = x[row * LW];
-        const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
-        int e = hi >> 20;
-        if (e == 0x7ff) e = kNaN;
-        else if (hi || __double2loint(v)) {
-            const unsigned top = ((hi & 0xfffffu) | (e ? 0x100000u : 0u)) + 1u;
-            e = max(e, 1);
-            if (DERIV) {
-                const int k = row < m ? row : n - row;
-                e = k ? max(e + 31 - __clz((int)(top * (unsigned)k)) - 20, 1) : 0;
-            }
-        }
-        emax = max(emax, e);
-    }
-    atomicMax(&s_e[l >> 1], emax);
+    for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW)
+        emax = max(emax, value_exponent<DERIV>(x[row * LW], row < m ? row : row - n));
+    atomicMax(&s_e[REAL ? l : l & ~1], emax);
     __syncthreads();
-    emax = s_e[l >> 1];
+    emax = s_e[REAL ? l : l & ~1];
     if (emax == 0) emax = 1023;  // a column of zeros: any exponent
-    if (blockIdx.y == 0 && threadIdx.x < LW && part == 0)
-        a.expo[((size_t)job * a.ntile + lt) * 64 + (lane >> 1)] = emax;
+    if (blockIdx.y == 0 && threadIdx.x < LW) a.expo[((size_t)job * a.ntile + lt) * kLanes + lane] = emax;
     if (emax >= kNaN) emax = 0x7ff;  // a non-finite column's digits are not used
     unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage;
     // effective part: multiplying by i moves real data to imaginary lanes and imaginary data, negated,
-    // to real lanes; so does the sine list
+    // to real lanes; so does the sine list of a complex transform
     const int epart = DERIV ? part ^ 1 : part;
-    const int row0 = DERIV ? lane ^ 1 : lane;
+    const int row0 = DERIV ? lane ^ 1 : lane, row1 = REAL ? lane : row0 ^ 1;
     const bool flip = DERIV && part == 1;
     const size_t st = (size_t)a.ks * kAStage;
     for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks; g += gridDim.y * (kDigThreads / LW)) {
@@ -316,15 +318,16 @@ __device__ __forceinline__ void digits_body(const DigArgs &a, const TcJob &J, in
                 if (epart == 1) w[t] = -w[t];
             }
             put_digits(d + 2 * par * st + row0 * 16, c);
-            put_digits(d + (2 * par + 1) * st + (row0 ^ 1) * 16, w);
+            put_digits(d + (2 * par + 1) * st + row1 * 16, w);
         }
     }
 }
 
+// Columns: LW = 16 keeps three blocks on an SM at n = 538 (69 KB), LW = 32 at up to half of that.
 template <int LW>
 __global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_e[LW / 2];
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ int s_e[LW];
     const TcShape &s = a.s;
     const int job = blockIdx.z;
     const TcJob &J = a.job[job];
@@ -332,7 +335,7 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
     const unsigned lt = blockIdx.x / kParts;
     const int lane0 = (blockIdx.x % kParts) * LW;
     const int n0 = J.ext ? s.n - s.next : s.n;  // rows below n0 come from the field
-    if (threadIdx.x < kCols) s_e[threadIdx.x] = 0;
+    if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
     {
         const int cc = threadIdx.x % kCols;
         const unsigned c = (a.tile0 + lt) * 64 + lane0 / 2 + cc;
@@ -348,15 +351,122 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
         async_wait();
     }
     __syncthreads();
-    if (J.deriv) digits_body<true, LW>(a, J, job, (const double *)smem, s_e, lt, lane0);
-    else digits_body<false, LW>(a, J, job, (const double *)smem, s_e, lt, lane0);
+    if (J.deriv) digits_body<true, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
+    else digits_body<false, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
+}
+
+// Real rows.  PROD: the rows are sums of products of physical rows in tiles [k][128 lanes] (the
+// nonlinear term: sum over i of phys[i] * phys[J.deriv + i], times scale); else they come from a
+// field's rows.
+template <int LW, bool PROD>
+__global__ void __launch_bounds__(kDigThreads, 3) k_digits_real(DigArgs a, const double *phys, size_t fstride, double scale) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ int s_e[LW];
+    const TcShape &s = a.s;
+    const int job = blockIdx.z;
+    const TcJob &J = a.job[job];
+    constexpr int kParts = kLanes / LW;
+    const unsigned lt = blockIdx.x / kParts;
+    const int lane0 = (blockIdx.x % kParts) * LW;
+    if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
+    double *dst = (double *)smem;
+    if (PROD) {
+        const int l = threadIdx.x % LW;
+        const double *u = phys + (size_t)lt * s.n * kLanes + lane0 + l, *d = u + J.deriv * fstride;
+#pragma unroll 2
+        for (int k = threadIdx.x / LW; k < s.n; k += kDigThreads / LW) {
+            const size_t o = (size_t)k * kLanes;
+            const double u0 = u[o], u1 = u[o + fstride], u2 = u[o + 2 * fstride];
+            const double d0 = d[o], d1 = d[o + fstride], d2 = d[o + 2 * fstride];
+            dst[k * LW + l] = (u0 * d0 + u1 * d1 + u2 * d2) * scale;
+        }
+    } else {
+        const unsigned r0 = (a.tile0 + lt) * kLanes + lane0;
+        for (int i = threadIdx.x; i < s.n * LW; i += kDigThreads) {
+            const int l = i / s.n, k = i - l * s.n;
+            dst[k * LW + l] = r0 + l < s.ncol ? __ldg((const double *)J.in + (size_t)(r0 + l) * s.n + k) : 0.0;
+        }
+    }
+    __syncthreads();
+    digits_body<false, true, LW>(a, job, dst, s_e, lt, lane0);
+}
+
+// Half spectra (rows of n/2 + 1 complex values, row stride s.rs): the lists are the real and imaginary
+// parts of the even and of the odd frequencies, doubled but for frequencies 0 and n/2, whose imaginary
+// parts do not count.
+template <bool DERIV, int LW>
+__device__ __forceinline__ void half_digits(const DigArgs &a, int job, const double2 *tile_s, int *s_e, unsigned lt,
+                                            int lane0) {
+    const int m = a.m, l = threadIdx.x % LW, lane = lane0 + l;
+    const double2 *x = tile_s + l;
+    int emax = 0;
+    for (int f = threadIdx.x / LW; f <= m; f += kDigThreads / LW) {
+        const double2 v = x[f * (LW + 1)];
+        emax = max(emax, max(value_exponent<DERIV>(v.x, f), value_exponent<DERIV>(v.y, f)));
+    }
+    atomicMax(&s_e[l], emax);
+    __syncthreads();
+    emax = s_e[l];
+    if (emax == 0) emax = 1023;
+    if (blockIdx.y == 0 && threadIdx.x < LW) a.expo[((size_t)job * a.ntile + lt) * kLanes + lane] = emax;
+    if (emax >= kNaN) emax = 0x7ff;
+    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage + lane * 16;
+    const size_t st = (size_t)a.ks * kAStage;
+    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks; g += gridDim.y * (kDigThreads / LW)) {
+        unsigned char *d = tb + (size_t)(g >> 1) * kAStage + (size_t)(g & 1) * kLanes * 16;
+#pragma unroll 1
+        for (int par = 0; par < 2; par++) {
+            long long c[8], w[8];
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+                const int f = 2 * (8 * g + t) + par;
+                c[t] = w[t] = 0;
+                if (f > m) continue;
+                const double2 v = x[f * (LW + 1)];
+                const bool end = f == 0 || f == m;
+                // frequency n/2 is the wavenumber -n/2; i k (re, im) = (-k im, k re)
+                const int k = f == m ? -m : f;
+                long long re = fixed_point<DERIV>(DERIV ? v.y : v.x, DERIV ? -k : k, emax);
+                long long im = fixed_point<DERIV>(DERIV ? v.x : v.y, k, emax);
+                c[t] = end ? re : 2 * re;
+                w[t] = end ? 0 : 2 * im;
+            }
+            put_digits(d + 2 * par * st, c);
+            put_digits(d + (2 * par + 1) * st, w);
+        }
+    }
+}
+
+template <int LW>
+__global__ void __launch_bounds__(kDigThreads, 3) k_digits_half(DigArgs a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ int s_e[LW];
+    const TcShape &s = a.s;
+    const int job = blockIdx.z, H = a.m + 1;
+    const TcJob &J = a.job[job];
+    constexpr int kParts = kLanes / LW;
+    const unsigned lt = blockIdx.x / kParts;
+    const int lane0 = (blockIdx.x % kParts) * LW;
+    const unsigned r0 = (a.tile0 + lt) * kLanes + lane0;
+    if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
+    double2 *dst = (double2 *)smem;  // [frequency][LW + 1]: the odd stride keeps the row writes off one bank
+    for (int i = threadIdx.x; i < H * LW; i += kDigThreads) {
+        const int l = i / H, f = i - l * H;
+        if (r0 + l < s.ncol) cp_async<16>(dst + f * (LW + 1) + l, J.in + (size_t)(r0 + l) * s.rs + f);
+        else dst[f * (LW + 1) + l] = make_double2(0.0, 0.0);
+    }
+    async_commit();
+    async_wait();
+    __syncthreads();
+    if (J.deriv) half_digits<true, LW>(a, job, dst, s_e, lt, lane0);
+    else half_digits<false, LW>(a, job, dst, s_e, lt, lane0);
 }
 
 // ------------------------------------------------------------------ products
 struct GemmArgs {
     TcShape s;
     TcJob job[kTcMaxJobs];
-    int m, ks, nq[2], nchunk, nc, sh, nstage;
+    int m, ks, nq[2], nchunk, nc, sh, nstage;  // m = n / 2
     unsigned tile0, ntile, units;
     const unsigned char *ws;
     const int *expo;
@@ -368,16 +478,22 @@ struct GemmArgs {
 // of the MMAs; a pipeline of bulk copies feeds 28 MMAs a 16-deep step.  One block per SM walks over
 // units: the cosine product moves from tensor memory to shared memory as integers, the sine product to
 // registers, and while the next unit's MMAs run, their sum and difference (the frequencies f and n - f)
-// become doubles.  The MMAs (operand reads from shared memory: (128 + nc) * 32 bytes each) and the
+// become doubles.  Half spectra to real rows (kC2R): a unit holds both parities; with A the even and B
+// the odd frequencies' sum, x[k] = A + B and x[k + n/2] = A - B, and the integers A wait in the output
+// until the same thread has B.  The MMAs (operand reads from shared memory: (128 + nc) * 32 bytes each) and the
 // integer work of the epilogue bound it.
 struct Unit {
     int job, par, chunk;
     unsigned lt;
 };
+template <int MODE>
 __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
     Unit w;
-    w.par = u % 2;
-    u /= 2;
+    w.par = 0;
+    if (MODE != kC2R) {
+        w.par = u % 2;
+        u /= 2;
+    }
     w.chunk = u % a.nchunk;
     u /= a.nchunk;
     w.lt = u % a.ntile;
@@ -385,15 +501,13 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
     return w;
 }
 
-// the general form of an output: any exponent, a non-finite column, a further factor, an addend
-__device__ __noinline__ double output_general(long long t, int q, int e, double post, const double *add) {
-    double v = scaled_double(t, q);
-    if (e >= kNaN) v = __longlong_as_double(0x7ff8000000000000ll);
-    if (post != 1.0) v *= post;
-    if (add) v += *add;
-    return v;
+// the general form of an output: any exponent, a non-finite column, a further factor
+__device__ __noinline__ double output_general(long long t, int q, int e, double post) {
+    const double v = scaled_double(t, q);
+    return e >= kNaN ? __longlong_as_double(0x7ff8000000000000ll) : v * post;
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned long long bars[2 * 8 + 2];
@@ -426,19 +540,19 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
     fence_after();
     const unsigned tmem = s_tmem;
     volatile int *ab = &s_abort;
-    const int nit = 2 * a.ks;  // steps of a unit: cosine list, then sine list
+    const int nit = (MODE == kC2R ? 4 : 2) * a.ks;  // steps of a unit: cosine list, sine list (of each parity)
     if (warp == kLoadWarp) {
         if (lane == 0) {
             int it = 0;  // steps issued so far, over all units
             bool ok = true;
             for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-                const Unit w = unit_of(a, u);
+                const Unit w = unit_of<MODE>(a, u);
                 const unsigned char *A = a.ws + (((size_t)w.job * a.ntile + w.lt) * 4 + 2 * w.par) * a.ks * kAStage;
                 const unsigned char *B = a.job[w.job].mat + ((size_t)w.par * 2 * a.nchunk + w.chunk) * a.ks * b_bytes;
                 for (int i = 0; i < nit; i++, it++) {
                     const int st = it % a.nstage, round = it / a.nstage;
                     if (round && !mbar_wait(empty + 8 * st, (round - 1) & 1, ab)) { ok = false; break; }
-                    const int list = i >= a.ks;
+                    const int list = i / a.ks;
                     const unsigned dst = smem_u32(smem) + st * stage_bytes;
                     mbar_expect(full + 8 * st, stage_bytes);
                     bulk_load(dst, A + (size_t)i * kAStage, kAStage, full + 8 * st);
@@ -461,7 +575,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
             for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x)
                 for (int i = 0; i < nit; i++, it++) {
                     const int st = it % a.nstage, round = it / a.nstage;
-                    const bool first = i == 0 || i == a.ks;
+                    const bool first = i % a.ks == 0;
                     if (first && lists) {  // the previous list's sums have left tensor memory
                         ok = mbar_wait(accempty, (lists - 1) & 1, ab);
                         if (!ok) break;
@@ -482,7 +596,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
                                      smem_desc(sb + j * (nc * 32), nc * 16, 128), idesc, fresh ? 0u : 1u);
                         }
                     mma_commit(empty + 8 * st);
-                    if (i == a.ks - 1 || i == nit - 1) {
+                    if ((i + 1) % a.ks == 0) {
                         mma_commit(accfull);
                         lists++;
                     }
@@ -513,62 +627,101 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
         };
         int lists = 0;
         bool ok = true;
-        for (unsigned u = blockIdx.x; u < a.units; u += gridDim.x) {
-            const Unit w = unit_of(a, u);
+        for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+            const Unit w = unit_of<MODE>(a, u);
             const TcJob &J = a.job[w.job];
-            ok = __all_sync(~0u, ok && mbar_wait(accfull, lists & 1, ab));
-            if (!ok) break;
-            lists++;
-            fence_after();
-#pragma unroll 1
-            for (int gi = 0; gi < ngr; gi++) {
-                const int col = (g0 + 4 * gi) * 4;
-                long long P[4];
-                gather(col, P);
-#pragma unroll
-                for (int t = 0; t < 4; t++) Ps[(col + t) * kLanes] = P[t];
+            bool live;
+            size_t off;  // of this lane's column or row in the output
+            if (MODE == kCol) {
+                const unsigned c = (a.tile0 + w.lt) * 64 + (r >> 1);
+                live = c < s.ncol;
+                off = live ? 2 * col_offset(s, c) + (r & 1) : 0;
+            } else {
+                live = (a.tile0 + w.lt) * kLanes + r < s.ncol;
+                off = (size_t)w.lt * s.ts + (size_t)r * s.ls;
             }
-            fence_before();
-            mbar_arrive(accempty);
-            ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
-            if (!ok) break;
-            lists++;
-            fence_after();
-            long long Q[5][4];
-#pragma unroll
-            for (int gi = 0; gi < 5; gi++)
-                if (gi < ngr) gather((g0 + 4 * gi) * 4, Q[gi]);
-            fence_before();
-            mbar_arrive(accempty);
-            const unsigned c = (a.tile0 + w.lt) * 64 + (r >> 1);
-            const bool live = c < s.ncol;
-            const size_t off = live ? 2 * col_offset(s, c) + (r & 1) : 0;
-            const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * 64 + (r >> 1)];
+            const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * kLanes + r];
             const int q = e - 1022 - 14 - sh + J.expo;
             double *out = (double *)J.out + off;
-            const double *add = J.add ? (const double *)J.add + off : nullptr;
+            const double *add = MODE == kCol && J.add ? (const double *)J.add + off : nullptr;
             // every result's exponent 1086 + q - lz, 0 <= lz < 64, is a normal number's
-            const bool plain = e < kNaN && q > -1023 && q < 960 && J.post == 1.0 && !add;
-            auto put = [&](int row, long long t) {
-                if (row >= s.nrows || !live) return;
-                const size_t o = 2 * (size_t)row * s.rs;
-                out[o] = plain ? plain_double(t, q) : output_general(t, q, e, J.post, add ? add + o : nullptr);
-            };
-#pragma unroll
-            for (int gi = 0; gi < 5; gi++)
-                if (gi < ngr) {
+            const bool plain = e < kNaN && q > -1023 && q < 960 && J.post == 1.0;
+            auto value = [&](long long t) { return plain ? plain_double(t, q) : output_general(t, q, e, J.post); };
+            for (int par = w.par; par < (MODE == kC2R ? 2 : w.par + 1); par++) {
+                ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
+                if (!ok) break;
+                lists++;
+                fence_after();
+#pragma unroll 1
+                for (int gi = 0; gi < ngr; gi++) {
                     const int col = (g0 + 4 * gi) * 4;
+                    long long P[4];
+                    gather(col, P);
 #pragma unroll
-                    for (int t = 0; t < 4; t++) {
-                        const int j = w.chunk * nc + col + t;
-                        if (j < a.nq[w.par]) {
-                            const int f = 2 * j + w.par;
-                            const long long p = Ps[(col + t) * kLanes], d = s.sign > 0 ? Q[gi][t] : -Q[gi][t];
-                            put(f, p + d);
-                            if (f && 2 * f != s.n) put(s.n - f, p - d);
+                    for (int t = 0; t < 4; t++) Ps[(col + t) * kLanes] = P[t];
+                }
+                fence_before();
+                mbar_arrive(accempty);
+                ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
+                if (!ok) break;
+                lists++;
+                fence_after();
+                long long Q[5][4];
+#pragma unroll
+                for (int gi = 0; gi < 5; gi++)
+                    if (gi < ngr) gather((g0 + 4 * gi) * 4, Q[gi]);
+                fence_before();
+                mbar_arrive(accempty);
+                if (!live) continue;
+#pragma unroll
+                for (int gi = 0; gi < 5; gi++)
+                    if (gi < ngr) {
+                        const int col = (g0 + 4 * gi) * 4;
+#pragma unroll
+                        for (int t = 0; t < 4; t++) {
+                            const int j = w.chunk * nc + col + t;
+                            if (j >= a.nq[MODE == kC2R ? 0 : par]) continue;
+                            const long long p = Ps[(col + t) * kLanes], d = Q[gi][t];
+                            if (MODE == kCol) {
+                                const int f = 2 * j + par, f2 = s.n - f;
+                                const long long sd = s.sign > 0 ? d : -d;
+                                if (f < s.nrows) {
+                                    const size_t o = 2 * (size_t)f * s.rs;
+                                    double v = value(p + sd);
+                                    if (add) v += add[o];
+                                    out[o] = v;
+                                }
+                                if (f && f != f2 && f2 < s.nrows) {
+                                    const size_t o = 2 * (size_t)f2 * s.rs;
+                                    double v = value(p - sd);
+                                    if (add) v += add[o];
+                                    out[o] = v;
+                                }
+                            } else if (MODE == kR2C) {
+                                const int f = 2 * j + par;
+                                if (f <= a.m) *(double2 *)(out + 2 * f) = make_double2(value(p), value(-d));
+                            } else {
+                                // even: A[k] = p - d, A[n/2 - k] = p + d; odd: B[k] = p - d, B[n/2 - k] = -p - d
+                                double *o0 = out + (size_t)j * s.rs, *o1 = out + (size_t)(a.m - j) * s.rs;
+                                const bool two = j && 2 * j != a.m;
+                                if (par == 0) {
+                                    *(long long *)o0 = p - d;
+                                    if (two) *(long long *)o1 = p + d;
+                                } else {
+                                    const size_t h = (size_t)a.m * s.rs;
+                                    const long long A = *(const long long *)o0, B = p - d;
+                                    o0[0] = value(A + B);
+                                    o0[h] = value(A - B);
+                                    if (two) {
+                                        const long long A1 = *(const long long *)o1, B1 = -p - d;
+                                        o1[0] = value(A1 + B1);
+                                        o1[h] = value(A1 - B1);
+                                    }
+                                }
+                            }
                         }
                     }
-                }
+            }
         }
     }
     __syncthreads();
@@ -619,7 +772,7 @@ __global__ void __launch_bounds__(128) k_continuation(Geo g, ContArgs a) {
 // ------------------------------------------------------------------ tables
 // digits [angle][7] of factor * cos, factor * sin at 2 pi t / n -> the matrices of one set
 __global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, int K, int ks, int nq0, int nq1, int nchunk,
-                           int nc) {
+                           int nc, int half) {
     const long long total = 4ll * nchunk * ks * 16 * nc;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
         const int kk = (int)(q % 16), col = (int)(q / 16 % nc);
@@ -628,8 +781,10 @@ __global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, 
         t /= ks;
         const int chunk = (int)(t % nchunk), list = (int)(t / nchunk % 2), par = (int)(t / nchunk / 2);
         const int k = 16 * step + kk, j = chunk * nc + col;
-        const bool on = k < K && j < (par ? nq1 : nq0);
-        const int ang = on ? (int)((long long)(2 * j + par) * k % n) : 0;
+        // the K side runs over points and the N side over frequencies, the other way about for half spectra
+        const int pt = half ? j : k, fq = half ? k : j;
+        const bool on = pt < K && fq < (par ? nq1 : nq0);
+        const int ang = on ? (int)((long long)(2 * fq + par) * pt % n) : 0;
         __nv_bfloat16 *dst = mat + (((long long)(par * 2 + list) * nchunk + chunk) * ks + step) * (kDig * 16 * nc) +
                              (kk / 8) * (nc * 8) + col * 8 + kk % 8;
         for (int i = 0; i < kDig; i++)
@@ -677,20 +832,30 @@ void matrix_digits(long double v, int d[kDig]) {
     for (int i = 1; i < kDig; i++) d[i] = (int)((w >> (54 - 9 * i)) & 511) - 256;
 }
 
-// Levels 0, 1 and 2 of a column's sums stay below 2^24 for any data digits (|d| <= 256).
-bool exact_levels(const Dims &D, const std::vector<int> &dc, const std::vector<int> &ds) {
-    for (int par = 0; par < 2; par++)
-        for (int j = 0; j < D.nq[par]; j++) {
+// Levels 0, 1 and 2 of every output's sums stay below 2^24 for any data digits (|d| <= 256).
+bool exact_levels(const Dims &D, bool half, const std::vector<int> &dc, const std::vector<int> &ds) {
+    std::vector<int> ac(D.n, 0), as(D.n, 0);
+    for (int t = 0; t < D.n; t++)
+        for (int i = 0; i < 3; i++) {
+            ac[t] += std::abs(dc[(size_t)t * kDig + i]);
+            as[t] += std::abs(ds[(size_t)t * kDig + i]);
+        }
+    for (int par = 0; par < 2; par++) {
+        const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
+        for (int o = 0; o < no; o++) {
+            // angles (2 f + par) * point: advance by a fixed step from one input to the next
+            const int step = half ? 2 * o % D.n : (2 * o + par) % D.n;
+            int ang = half ? par * o % D.n : 0;
             long long sc = 0, ss = 0;
-            for (int k = 0; k < D.K; k++) {
-                const size_t t = (size_t)((long long)(2 * j + par) * k % D.n) * kDig;
-                for (int i = 0; i < 3; i++) {
-                    sc += std::abs(dc[t + i]);
-                    ss += std::abs(ds[t + i]);
-                }
+            for (int i = 0; i < ni; i++) {
+                sc += ac[ang];
+                ss += as[ang];
+                ang += step;
+                if (ang >= D.n) ang -= D.n;
             }
             if (256 * std::max(sc, ss) > (1ll << 24)) return false;
         }
+    }
     return true;
 }
 
@@ -709,10 +874,11 @@ void tc_job_set(TcJob &j, const TcSet *s) {
     j.post = s->post;
 }
 
-const TcSet *tc_set(Plan &P, int n, double factor, int *status) {
+const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     *status = OK;
     TcState *S = state(P);
-    auto it = S->sets.find({n, factor});
+    const std::pair<int, double> key(half ? -n : n, factor);
+    auto it = S->sets.find(key);
     if (it != S->sets.end()) return &it->second;
     const Dims D = dims(n);
     std::vector<long double> c, s;
@@ -733,7 +899,7 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status) {
         }
         set.expo = t < 4 ? ex + t : 0;
         set.post = t < 4 ? 1.0 : factor;
-        ok = exact_levels(D, dc, ds);
+        ok = exact_levels(D, half, dc, ds);
     }
     if (!ok) { set_error("digit tables: exactness bound"); *status = ERR_SHAPE; return nullptr; }
     std::vector<__nv_bfloat16> h(2 * (size_t)n * kDig);
@@ -752,7 +918,8 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status) {
         return nullptr;
     }
     cudaMemcpyAsync(dig, h.data(), h.size() * 2, cudaMemcpyHostToDevice, P.stream);
-    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, dig, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc);
+    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, dig, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc,
+                                            half ? 1 : 0);
     const cudaError_t e = cudaStreamSynchronize(P.stream);  // the host digits go out of scope
     cudaFree(dig);
     if (e != cudaSuccess || (*status = check_launch("digit tables"))) {
@@ -760,29 +927,27 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status) {
         if (!*status) *status = ERR_CUDA;
         return nullptr;
     }
-    return &(S->sets[{n, factor}] = set);
+    return &(S->sets[key] = set);
 }
 
 // The digit workspace of a plan has one size for its lifetime (captured graphs hold its address):
-// what its largest axis needs for all columns of eight transforms, at most 2 GiB; longer launches run
-// in ranges of tiles.
+// what its largest axis needs for all its columns, at most 2 GiB; longer launches run in ranges of tiles.
 static int workspace(Plan &P) {
     TcState *S = state(P);
     if (S->ws) return OK;
     size_t want = 0, tiles = 0;
-    const int len[2] = {P.nz, P.ny};
-    const size_t cols[2] = {(size_t)P.ny * P.ldx, (size_t)P.nz * P.ldx};
-    for (int i = 0; i < 2; i++) {
+    const int len[3] = {P.nz, P.ny, P.nx}, jobs[3] = {kTcMaxJobs, kTcMaxJobs, kTcMaxJobs};
+    const size_t cols[3] = {((size_t)P.ny * P.ldx + 63) / 64, ((size_t)P.nz * P.ldx + 63) / 64,
+                            ((size_t)P.nz * P.ny + kLanes - 1) / kLanes};
+    for (int i = 0; i < 3; i++) {
         if (!tc_length_ok(len[i])) continue;
-        const Dims D = dims(len[i]);
-        const size_t nt = (cols[i] + 63) / 64 * kTcMaxJobs;
-        const size_t per = 4ull * D.ks * kAStage;
-        size_t b = nt * per;
-        if (b > (2ull << 30)) b = std::max<size_t>((2ull << 30) / per * per, (size_t)kTcMaxJobs * per);
-        if (b > want) want = b;
-        if (b / per > tiles) tiles = b / per;
+        const size_t per = 4ull * dims(len[i]).ks * kAStage;
+        size_t t = cols[i] * jobs[i];
+        t = std::min(t, std::max<size_t>((2ull << 30) / per, kTcMaxJobs));
+        want = std::max(want, t * per);
+        tiles = std::max(tiles, t);
     }
-    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * 64 * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * kLanes * sizeof(int)) != cudaSuccess ||
         cudaHostAlloc(&S->err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&S->err_dev, S->err, 0) != cudaSuccess) {
         cudaGetLastError();
@@ -797,7 +962,7 @@ static int workspace(Plan &P) {
     }
     *S->err = 0;
     S->ws_bytes = want;
-    S->expo_count = tiles * 64;
+    S->expo_count = tiles * kLanes;
     return OK;
 }
 
@@ -807,6 +972,61 @@ int tc_status(const Plan &P) {
     return ERR_CUDA;
 }
 
+namespace {
+
+// One range of tiles of one set of jobs: arguments of the digit and of the product kernels.
+void fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int nj, unsigned t0, unsigned nt, DigArgs &d,
+               GemmArgs &g) {
+    TcState *S = P.tc;
+    d.s = g.s = s;
+    for (int j = 0; j < nj; j++) d.job[j] = g.job[j] = jobs[j];
+    d.m = g.m = D.m;
+    d.K = D.K;
+    d.ks = g.ks = D.ks;
+    d.tile0 = g.tile0 = t0;
+    d.ntile = g.ntile = nt;
+    d.ws = S->ws;
+    g.ws = S->ws;
+    d.expo = S->expo;
+    g.expo = S->expo;
+    g.nq[0] = D.nq[0];
+    g.nq[1] = D.nq[1];
+    g.nchunk = D.nchunk;
+    g.nc = D.nc;
+    g.sh = D.sh;
+    g.err = S->err_dev;
+}
+
+// lanes per digit block: three blocks on an SM
+int digit_lanes(int n) { return n <= 300 ? 32 : 16; }
+
+// Small launches split a tile's lists over blocks (each reads its columns itself) until there are two
+// blocks per SM.
+int digit_split(const Dims &D, int lw, size_t blocks) {
+    const int rounds = (2 * D.ks * lw + kDigThreads - 1) / kDigThreads;
+    int split = 1;
+    while (split < rounds && blocks * split < 304) split++;
+    return split;
+}
+
+template <int MODE>
+void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
+    const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)D.nc * kLanes * 8;
+    g.nstage = std::min(8, (int)((226 * 1024 - psize) / stage));
+    g.units = g.ntile * (MODE == kC2R ? 1 : 2) * D.nchunk * nj;
+    const size_t smem = (size_t)g.nstage * stage + psize;
+    cudaFuncSetAttribute(k_gemm<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_gemm<MODE><<<std::min(g.units, 152u), kGemmThreads, smem, P.stream>>>(g);
+}
+
+template <typename K>
+K with_smem(K k, size_t bytes) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return k;
+}
+
+}  // namespace
+
 int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes) {
     if (int st = workspace(P)) return st;
     if (int st = tc_status(P)) return st;
@@ -814,57 +1034,128 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
     const Dims D = dims(s.n);
     const size_t per = 4ull * D.ks * kAStage;
     const unsigned tiles = (s.ncol + 63) / 64;
-    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / 64);
+    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     // all jobs at once when they fit, else job by job in ranges of tiles
     const int jstep = (size_t)tiles * njobs <= cap ? njobs : 1;
     const unsigned tstep = jstep == njobs ? tiles : (unsigned)std::min<size_t>(tiles, cap);
-    const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)D.nc * kLanes * 8;
-    const int nstage = std::min(8, (int)((226 * 1024 - psize) / stage));
-    const size_t smem = (size_t)nstage * stage + psize;
-    cudaFuncSetAttribute(k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const int lw = s.n <= 300 ? 32 : 16;
+    const int lw = digit_lanes(s.n);
     const size_t dsm = (size_t)s.n * lw * 8;
-    auto kd = lw == 32 ? k_digits<32> : k_digits<16>;
-    cudaFuncSetAttribute(kd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm);
     for (int j0 = 0; j0 < njobs; j0 += jstep)
         for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
             const unsigned nt = std::min(tstep, tiles - t0);
             DigArgs d{};
             GemmArgs g{};
-            d.s = g.s = s;
-            for (int j = 0; j < jstep; j++) d.job[j] = g.job[j] = jobs[j0 + j];
-            d.m = g.m = D.m;
-            d.K = D.K;
-            d.ks = g.ks = D.ks;
-            d.tile0 = g.tile0 = t0;
-            d.ntile = g.ntile = nt;
-            d.ws = S->ws;
-            g.ws = S->ws;
-            d.expo = S->expo;
-            g.expo = S->expo;
-            g.nq[0] = D.nq[0];
-            g.nq[1] = D.nq[1];
-            g.nchunk = D.nchunk;
-            g.nc = D.nc;
-            g.sh = D.sh;
-            g.nstage = nstage;
-            g.err = S->err_dev;
-            g.units = nt * 2 * D.nchunk * jstep;
-            // small launches: split a tile's lists over blocks (each reads the columns itself)
-            const int blocks = (int)nt * (kLanes / lw) * jstep, rounds = (2 * D.ks * lw + kDigThreads - 1) / kDigThreads;
-            int split = 1;
-            while (split < rounds && blocks * split < 304) split++;
+            fill_args(P, D, s, jobs + j0, jstep, t0, nt, d, g);
+            const size_t blocks = (size_t)nt * (kLanes / lw);
+            const dim3 grid((unsigned)blocks, digit_split(D, lw, blocks * jstep), jstep);
             const double share = (double)nt * jstep / ((double)tiles * njobs);
             {
                 Launch L(P, "digits", share * bytes * 0.5 + (double)nt * jstep * per);
-                kd<<<dim3(nt * (kLanes / lw), split, jstep), kDigThreads, dsm, P.stream>>>(d);
+                with_smem(lw == 32 ? k_digits<32> : k_digits<16>, dsm)<<<grid, kDigThreads, dsm, P.stream>>>(d);
             }
             {
                 Launch L(P, name, share * bytes);
-                k_gemm<<<std::min(g.units, 152u), kGemmThreads, smem, P.stream>>>(g);
+                launch_gemm<kCol>(P, D, g, jstep);
             }
         }
     return check_launch(name);
+}
+
+// gradre / advect between the y passes (pseudospec_hd.f90:209-319, pseudospec_phd.f90:23-113): the
+// velocity and the derivatives of components [c0, c1) to physical rows, the products, and back, in
+// ranges of tiles whose physical rows ([field][tile][x][128 rows]) stay in a buffer of the plan.
+int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
+    if (!tc_length_ok(P.nx)) return kNoFast;
+    const void *const *u = x.u, *const *dy = x.dy, *const *dz = x.dz;
+    void *const *out = x.out;
+    const int c0 = x.c0, c1 = x.c1, nrows = x.nrows;
+    const double scale = x.tmp;
+    if (int st = workspace(P)) return st;
+    if (int st = tc_status(P)) return st;
+    TcState *S = P.tc;
+    int st = OK;
+    const int n = P.nx, nc = c1 - c0, nin = 3 + 3 * nc;
+    const TcSet *inv = tc_set(P, n, 1.0, &st, true), *dinv = inv ? tc_set(P, n, P.Dkx, &st, true) : nullptr;
+    const TcSet *fwd = dinv ? tc_set(P, n, 1.0, &st, false) : nullptr;
+    if (!fwd) return st;
+    const Dims D = dims(n);
+    const size_t per = 4ull * D.ks * kAStage, ptile = (size_t)n * kLanes;
+    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const unsigned rows = (unsigned)nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
+    const unsigned alltiles = ((unsigned)P.nzp * P.ny + kLanes - 1) / kLanes;
+    if (!S->phys) {  // sized for four components; its address is fixed like the digits'
+        const size_t t = std::min<size_t>(alltiles, std::max<size_t>(cap / kTcMaxJobs, 1));
+        if (cudaMalloc(&S->phys, t * 15 * ptile * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            S->phys = nullptr;
+            set_error("out of device memory (physical rows)");
+            return ERR_OOM;
+        }
+        S->phys_tiles = t;
+    }
+    const unsigned tstep = (unsigned)std::min<size_t>(S->phys_tiles, tiles);
+    const size_t fstride = S->phys_tiles * ptile;
+    const int lw = digit_lanes(n);
+    for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
+        const unsigned nt = std::min(tstep, tiles - t0);
+        const double share = (double)nt / tiles * bytes;
+        const size_t blocks = (size_t)nt * (kLanes / lw);
+        TcJob jobs[kTcMaxJobs];
+        // physical fields: u, v, w, then d/dx, d/dy, d/dz of each component
+        for (int j = 0; j < nin; j++) {
+            const int c = c0 + (j - 3) / 3, dir = (j - 3) % 3;
+            TcJob &J = jobs[j];
+            J = TcJob{};
+            J.in = (const double2 *)(j < 3 ? u[j] : dir == 0 ? u[c] : dir == 1 ? dy[c] : dz[c]);
+            J.out = (double2 *)(S->phys + j * fstride);
+            J.deriv = j >= 3 && dir == 0;
+            tc_job_set(J, J.deriv ? dinv : inv);
+        }
+        TcShape s{};
+        s.n = n;
+        s.ncol = rows;
+        s.rs = P.ldx;
+        DigArgs d{};
+        GemmArgs g{};
+        fill_args(P, D, s, jobs, nin, t0, nt, d, g);
+        {
+            const size_t sm = (size_t)(D.m + 1) * (lw + 1) * sizeof(double2);
+            Launch L(P, "digits", share * nin / (nin + nc) + (double)nt * nin * per);
+            with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm)
+                <<<dim3((unsigned)blocks, digit_split(D, lw, blocks * nin), nin), kDigThreads, sm, P.stream>>>(d);
+        }
+        g.s.rs = kLanes;
+        g.s.ls = 1;
+        g.s.ts = ptile;
+        {
+            Launch L(P, "x_inverse", (double)nt * nin * (per + ptile * 8.0));
+            launch_gemm<kC2R>(P, D, g, nin);
+        }
+        for (int c = 0; c < nc; c++) {
+            TcJob &J = jobs[c];
+            J = TcJob{};
+            J.out = (double2 *)out[c0 + c] + (size_t)t0 * kLanes * P.ldx;
+            J.deriv = 3 + 3 * c;
+            tc_job_set(J, fwd);
+        }
+        s.ls = 2 * P.ldx;
+        s.ts = (size_t)kLanes * s.ls;
+        DigArgs d2{};
+        GemmArgs g2{};
+        fill_args(P, D, s, jobs, nc, t0, nt, d2, g2);
+        {
+            const size_t sm = (size_t)n * lw * sizeof(double);
+            Launch L(P, "products", (double)nt * (nin * ptile * 8.0 + nc * per));
+            with_smem(lw == 32 ? k_digits_real<32, true> : k_digits_real<16, true>, sm)
+                <<<dim3((unsigned)blocks, digit_split(D, lw, blocks * nc), nc), kDigThreads, sm, P.stream>>>(
+                    d2, S->phys, fstride, scale);
+        }
+        {
+            Launch L(P, "x_forward", share * nc / (nin + nc) + (double)nt * nc * per);
+            launch_gemm<kR2C>(P, D, g2, nc);
+        }
+    }
+    return check_launch("x_nonlinear");
 }
 
 int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf) {
@@ -890,12 +1181,90 @@ int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int n
     return check_launch("continuation");
 }
 
+#define SG_TRY(x)                  \
+    do {                           \
+        int _st = (x);             \
+        if (_st != OK) return _st; \
+    } while (0)
+
+// FP64 passes over the digit-product transforms (tcdft.cu).  They serve every even length of 32 to
+// 550: at all of them they are faster than the FP64 Stockham engine, which the FP64 pipe bounds.
+// kNoFast: a form that they do not take (another length, a scale on part of the rows).
+static int tc_add(Plan &P, TcJob *jobs, int *nj, int n, double factor, const void *in, void *out, const void *add,
+                  int deriv, const double2 *ext) {
+    int st = OK;
+    const TcSet *set = tc_set(P, n, factor, &st);
+    if (!set) return st;
+    TcJob &j = jobs[(*nj)++];
+    j = TcJob{};
+    j.in = (const double2 *)in;
+    j.out = (double2 *)out;
+    j.add = (const double2 *)add;
+    j.ext = ext;
+    j.deriv = deriv;
+    tc_job_set(j, set);
+    return OK;
+}
+
+static TcShape tc_z_shape(const Plan &P, int sign, int nrows) {
+    TcShape s{};
+    s.n = P.nz;
+    s.sign = sign;
+    s.nrows = nrows;
+    s.ncol = s.w = s.s = s.rs = s.es = (unsigned)P.ny * P.ldx;
+    return s;
+}
+
+int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes) {
+    if (!tc_length_ok(P.nz) || (a.scale_rows > 0 && a.scale_rows < a.nrows)) return kNoFast;
+    const double sc = a.scale_rows > 0 ? a.scale : 1.0;
+    TcJob jobs[kTcMaxJobs];
+    int nj = 0;
+    // derivatives first: out0 may alias in
+    for (int f = 0; f < nf; f++)
+        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, P.Dkz * sc, a.in[f], a.out1[f], nullptr, 1, nullptr));
+    for (int f = 0; f < nf; f++)
+        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, sc, a.in[f], a.out0[f], a.add[f], 0, nullptr));
+    return tc_run(P, tc_z_shape(P, +1, a.nrows), jobs, nj, "z_inverse", bytes);
+}
+
+int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
+    if (!tc_length_ok(P.nz) || a.in_scale != 1.0) return kNoFast;
+    const double2 *ext[kMaxF];
+    SG_TRY(tc_continuation(P, a.in, ext, nf));
+    TcJob jobs[kTcMaxJobs];
+    int nj = 0;
+    for (int f = 0; f < nf; f++) SG_TRY(tc_add(P, jobs, &nj, P.nz, 1.0, a.in[f], a.out[f], nullptr, 0, ext[f]));
+    TcShape s = tc_z_shape(P, -1, P.nz);
+    s.next = P.cz;
+    return tc_run(P, s, jobs, nj, "z_forward", bytes);
+}
+
+int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes) {
+    if (!tc_length_ok(P.ny)) return kNoFast;
+    TcJob jobs[kTcMaxJobs];
+    int nj = 0;
+    for (int f = 0; f < nf; f++)
+        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, P.Dky * a.scale, a.in[f], a.out1[f], nullptr, 1, nullptr));
+    for (int f = 0; f < nf; f++)
+        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, a.scale, a.in[f], a.out0[f], nullptr, 0, nullptr));
+    TcShape s{};
+    s.n = P.ny;
+    s.sign = a.sign;
+    s.nrows = P.ny;
+    s.w = s.rs = P.ldx;
+    s.s = (unsigned)P.ny * P.ldx;
+    s.ncol = (unsigned)nplanes * P.ldx;
+    return tc_run(P, s, jobs, nj, a.sign < 0 ? "y_forward" : "y_inverse", bytes);
+}
+
 void tc_free(Plan &P) {
     if (!P.tc) return;
     for (auto &e : P.tc->sets) cudaFree(e.second.mat);
     if (P.tc->ws) cudaFree(P.tc->ws);
     if (P.tc->expo) cudaFree(P.tc->expo);
     if (P.tc->ext) cudaFree(P.tc->ext);
+    if (P.tc->phys) cudaFree(P.tc->phys);
     if (P.tc->err) cudaFreeHost(P.tc->err);
     delete P.tc;
     P.tc = nullptr;
@@ -904,6 +1273,7 @@ void tc_free(Plan &P) {
 unsigned long long tc_bytes(const Plan &P) {
     if (!P.tc) return 0;
     unsigned long long b = P.tc->ws_bytes + P.tc->expo_count * sizeof(int);
+    b += (unsigned long long)P.tc->phys_tiles * 15 * P.nx * kLanes * sizeof(double);
     if (P.tc->ext) b += (unsigned long long)kMaxF * P.cz * P.ny * P.ldx * sizeof(double2);
     for (const auto &e : P.tc->sets) b += e.second.bytes;
     return b;

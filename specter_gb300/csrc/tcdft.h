@@ -5,7 +5,12 @@
 
 namespace sg {
 
-constexpr int kTcMaxJobs = 8;  // column transforms per launch
+struct ZInvArgs;
+struct ZFwdArgs;
+struct YArgs;
+struct XNLArgs;
+
+constexpr int kTcMaxJobs = 16;  // transforms per launch
 
 // One column transform of a launch: out = factor * DFT^sign(in) over rows (row stride rs, in
 // complex elements), factor taken from the table set; deriv = 1 first multiplies row k by i * k
@@ -26,15 +31,24 @@ struct TcShape {
     int next;                   // rows taken from ext
     unsigned ncol, w, s, rs;    // rs: row stride of in and out
     unsigned es;                // row stride of ext (its columns are laid out as the field's)
+    // transforms of rows: ncol rows; row r of tile t (128 rows) starts at t * ts + r * ls of the output
+    unsigned ls;
+    size_t ts;
 };
 
 // true when length n has digit-product transforms (FP64 plans)
 bool tc_length_ok(int n);
-// the table set of length n scaled by `factor`; built on first use
+// the table set of length n scaled by `factor` (half: for half spectra to real rows); built on first use
 struct TcSet;
-const TcSet *tc_set(Plan &P, int n, double factor, int *status);
+const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half = false);
 void tc_job_set(TcJob &j, const TcSet *s);
+// complex columns
 int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes);
+// the passes of kernels.cuh over these transforms; kNoFast (fast.h) for a form that they do not take
+int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes);
+int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes);
+int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes);
+int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes);
 // continuation rows of FC-Gram columns of nf <= kMaxF fields, in a buffer of the plan:
 // ext[f][(i * ny + ky) * ldx + kx], i < cz
 int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf);

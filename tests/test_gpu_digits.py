@@ -7,6 +7,7 @@ L2 of a column), the digit products within 3e-16: 2e-15 between the two."""
 import numpy as np
 import pytest
 
+from conftest import make_pair, rel, smooth_spectral
 from specter_gb300 import api
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +79,20 @@ def test_non_finite_and_denormal_columns():
     big = np.fft.ifft(a[0, 1] * 2.0**-60) * 58
     fits = (np.abs(big.real) < 1e289) & (np.abs(big.imag) < 1e289)
     assert np.allclose(got[0, 1][fits] * 2.0**-60, big[fits], rtol=1e-12, atol=0)
+
+
+# the x pass of the nonlinear term and the whole plain FP64 stage: shortest and longest lengths, halves
+# that are odd, rows that end inside a tile of 128.  1e-11: the continuation amplifies rounding by 1e4
+# (tests/test_gpu_parity.py).
+@pytest.mark.parametrize("nx,ny,nzp", [(32, 4, 33), (34, 6, 29), (62, 10, 11), (100, 32, 13), (254, 4, 11), (512, 4, 11),
+                                       (550, 2, 11)])
+def test_nonlinear_term(nx, ny, nzp):
+    p, g = make_pair(nx, ny, nzp, 1.0)
+    rng = np.random.default_rng(nx)
+    v = [smooth_spectral(g, rng) for _ in range(4)]
+    f, out = [p.field(data=a) for a in v], [p.field() for _ in range(4)]
+    api.gradre(p, f[0], f[1], f[2], out[0], out[1], out[2])
+    api.advect(p, f[0], f[1], f[2], f[3], out[3])
+    want = list(g.gradre(*v[:3])) + [g.advect(*v[:3], v[3])]
+    for a, b in zip(out, want):
+        assert rel(a.download(), b) < 1e-11
