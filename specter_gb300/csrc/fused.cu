@@ -4,6 +4,7 @@
 #include "fused.h"
 #include "fast.h"
 #include "fused_launch.cuh"
+#include "stage_f64.h"
 
 namespace sg {
 
@@ -139,6 +140,11 @@ static int harmonic_spectra(Plan &P, void *E1, void *E2) {
     return st;
 }
 
+// Plain FP64 solvers run the stage of stage_f64.cu where the z length has digit-product transforms; the
+// column kernels on the FP64 Stockham engine serve the others (211 against 37 ms an RK2 step of
+// Rayleigh-Benard convection at 256^2 x 257).
+static bool plain_f64(const Plan &P, const StageParams &sp) { return P.prec == FP64 && !sp.nl_fp32 && f64_stage_ok(P); }
+
 int fused_create(Plan &P, const StageParams &sp, FusedState **out) {
     *out = nullptr;
     FusedState *fs = new FusedState();
@@ -149,9 +155,10 @@ int fused_create(Plan &P, const StageParams &sp, FusedState **out) {
         ok = ok && cudaMalloc(&fs->X1[i], P.field_bytes()) == cudaSuccess;
         if (sp.ord >= 3) ok = ok && cudaMalloc(&fs->X2[i], P.field_bytes()) == cudaSuccess;
     }
-    if (sp.solver == 1) ok = ok && cudaMalloc(&fs->side, 2 * (size_t)P.ny * P.nzp * P.elt()) == cudaSuccess;  // BOUSS only
+    const bool columns = !plain_f64(P, sp);  // buffers of the column kernels
+    if (sp.solver == 1 && columns) ok = ok && cudaMalloc(&fs->side, 2 * (size_t)P.ny * P.nzp * P.elt()) == cudaSuccess;  // BOUSS only
     for (int i = 0; i < 2; i++) ok = ok && cudaMalloc(&fs->E[i], P.field_bytes()) == cudaSuccess;
-    for (int i = 0; i < 3; i++) ok = ok && cudaMalloc(&fs->W[i], P.field_bytes()) == cudaSuccess;
+    for (int i = 0; i < 3 && columns; i++) ok = ok && cudaMalloc(&fs->W[i], P.field_bytes()) == cudaSuccess;
     if (ok && sp.nl_fp32) {
         if (P.prec != FP64) {
             fused_destroy(fs);
@@ -274,6 +281,8 @@ template <typename T>
 static int run_stage(Plan &P, FusedState *fs, int o, const void *const vin[4], const void *const cold[4],
                      void *const vout[4], void *pr) {
     const StageParams &sp = fs->sp;
+    if constexpr (is_f64<T>)
+        if (plain_f64(P, sp)) return f64_stage(P, sp, o, vin, cold, vout, pr, fs->E);
     const bool bouss = sp.solver >= 1, rot = sp.solver == 2;
     const void *nl[4] = {nullptr, nullptr, nullptr, nullptr};
     int st = OK;
