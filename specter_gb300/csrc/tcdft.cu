@@ -37,17 +37,17 @@ constexpr int kLanes = 128;         // rows of an MMA: 64 columns, real and imag
 constexpr int kMaxNc = 80;          // outputs per block: kLev * 80 = 480 of 512 tensor-memory columns
 constexpr int kMaxLen = 550;        // every even length up to here holds the exactness bound of level 2
 constexpr int kAStage = kDig * kLanes * 16 * 2;  // bytes of one 16-deep step of data digits
-constexpr int kEpi = 512;           // epilogue threads
 constexpr int kDigThreads = 256;
-constexpr int kLoadWarp = kEpi / 32, kMmaWarp = kLoadWarp + 1;
-constexpr int kGemmThreads = kEpi + 64;
+// Outputs as integers in units of 2^-kSh of the level-0 unit: results are below (n + 2) * sqrt(2) * 2^14
+// level-0 units (each input is below 2^14 of them, twice that in a half spectrum), 2^62.7 at n = 550.
+constexpr int kSh = 39;
 constexpr int kNaN = 0x40000000;    // exponent of a column that holds a non-finite value
 
 // what a launch transforms: complex columns; real rows to half spectra; half spectra to real rows
 enum { kCol = 0, kR2C = 1, kC2R = 2 };
 
 struct Dims {
-    int n, m, K, ks, nq[2], nchunk, nc, sh;
+    int n, m, K, ks, nq[2], nchunk, nc;
 };
 Dims dims(int n) {
     Dims d;
@@ -60,10 +60,6 @@ Dims dims(int n) {
     const int np = (d.nq[0] + 15) / 16 * 16;
     d.nchunk = (np + kMaxNc - 1) / kMaxNc;
     d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
-    // results are below (n + 2) * sqrt(2) * 2^14 level-0 units (each input is below 2^14 of them, twice
-    // that in a half spectrum): as many fraction bits as fit 63 bits
-    d.sh = 44;
-    while ((n + 2) * 1.41421357 * 16384.0 * (double)(1ll << d.sh) >= 9.2233720368547e18) d.sh--;
     return d;
 }
 
@@ -137,26 +133,42 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned addr, unsigned 
     return (unsigned long long)((addr & 0x3FFFF) >> 4) | ((unsigned long long)(lbo >> 4) << 16) |
            ((unsigned long long)(sbo >> 4) << 32) | (1ull << 46);
 }
+// Issued by the lane with lead != 0 of a converged warp: operands that are the same in all lanes stay in
+// uniform registers (39 clocks an instruction at most, against 60 from a branch that one lane takes).
 __device__ __forceinline__ void mma_bf16(unsigned d, unsigned long long a, unsigned long long b, unsigned idesc,
-                                         unsigned acc) {
+                                         unsigned acc, unsigned lead) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        "{\n.reg .pred p, e;\nsetp.ne.u32 p, %4, 0;\nsetp.ne.u32 e, %5, 0;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void mma_commit(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void mma_commit(unsigned bar, unsigned lead) {
+    asm volatile(
+        "{\n.reg .pred e;\nsetp.ne.u32 e, %1, 0;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
+        "r"(lead)
+        : "memory");
 }
-__device__ __forceinline__ void tmem_ld4(float (&v)[4], unsigned addr) {
-    unsigned r[4];
+__device__ __forceinline__ unsigned elect_one() {
+    unsigned r;
+    asm volatile("{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\nselp.u32 %0, 1, 0, e;\n}\n" : "=r"(r));
+    return r;
+}
+// four columns of every level, asynchronously; the values are there after tmem_wait
+__device__ __forceinline__ void tmem_ld4(unsigned (&r)[4], unsigned addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
-#pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// waits for this thread's loads; the operands keep their uses behind it
+__device__ __forceinline__ void tmem_wait(unsigned (&r)[kLev][4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[1][0]), "+r"(r[1][1]), "+r"(r[1][2]),
+                   "+r"(r[1][3]), "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]), "+r"(r[3][0]), "+r"(r[3][1]),
+                   "+r"(r[3][2]), "+r"(r[3][3]), "+r"(r[4][0]), "+r"(r[4][1]), "+r"(r[4][2]), "+r"(r[4][3]), "+r"(r[5][0]),
+                   "+r"(r[5][1]), "+r"(r[5][2]), "+r"(r[5][3])::"memory");
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -165,20 +177,69 @@ __device__ __forceinline__ size_t col_offset(const TcShape &s, unsigned c) {
     return (size_t)q * s.s + (c - q * s.w);
 }
 
-// t * 2^q as a double, rounded to nearest (|t| < 2^63); the result's exponent is a normal number's.
-// The implicit bit carries into the exponent field, as does rounding up to the next power of two.
-__device__ __forceinline__ double plain_double(long long t, int q) {
-    const unsigned long long u = t < 0 ? -(unsigned long long)t : (unsigned long long)t;
-    const int lz = __clzll((long long)u);
-    const unsigned long long M = u << lz;
-    const unsigned long long mant = (M >> 11) + ((M >> 10) & 1);
-    unsigned long long b = ((unsigned long long)(unsigned)(1085 + q - lz) << 52) + mant;
-    b |= (unsigned long long)t & 0x8000000000000000ull;
-    return u ? __longlong_as_double((long long)b) : 0.0;
+// The levels of four outputs as integers, sum over v of l[v] * 2^kSh.  A level times 2^9v (level 5 times
+// 2^kSh, rounded) is an integer that an addition of 1.5 * 2^23 leaves in the low mantissa bits while it
+// is below 2^22, as sums of signed digits nearly always are; level 0 goes up to 2^24 and hands what is
+// below its multiples of 4 down to level 1.  False where a level was too large.  (Conversion instructions
+// would run at 16 a clock: 4400 clocks a list against 2500.)
+__device__ __forceinline__ bool join_levels(const unsigned (&l)[kLev][4], long long (&u)[4]) {
+    constexpr unsigned kB4 = 0x4C400000u, kB = 0x4B400000u;  // 1.5 * 2^25, 1.5 * 2^23
+    constexpr unsigned long long kOff = ((unsigned long long)kB4 << (kSh + 2)) + ((unsigned long long)kB << (kSh - 9)) +
+                                        ((unsigned long long)kB << (kSh - 18)) + ((unsigned long long)kB << (kSh - 27)) +
+                                        ((unsigned long long)kB << (kSh - 36)) + kB;
+    unsigned bad = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        auto f = [&](int v) { return __uint_as_float(l[v][t]); };
+        const float m4 = __uint_as_float(kB4), m = __uint_as_float(kB);
+        const float r0 = f(0) + m4, rem = f(0) - (r0 - m4);
+        const unsigned b0 = __float_as_uint(r0), b1 = __float_as_uint(fmaf(f(1) + rem, 512.f, m)),
+                       b2 = __float_as_uint(fmaf(f(2), 262144.f, m)), b3 = __float_as_uint(fmaf(f(3), 134217728.f, m)),
+                       b4 = __float_as_uint(fmaf(f(4), 68719476736.f, m)),
+                       b5 = __float_as_uint(fmaf(f(5), (float)(1ull << kSh), m));
+        bad |= (b1 ^ kB) | (b2 ^ kB) | (b3 ^ kB) | (b4 ^ kB) | (b5 ^ kB);
+        unsigned long long y = (unsigned long long)b3 * (1u << (kSh - 27)) - kOff;
+        y = (unsigned long long)b4 * (1u << (kSh - 36)) + y;
+        y = (unsigned long long)b2 * (1u << (kSh - 18)) + y;
+        y = (unsigned long long)b1 * (1u << (kSh - 9)) + y;
+        y += b5;
+        u[t] = (long long)(y + ((unsigned long long)(b0 << (kSh + 2 - 32)) << 32));
+    }
+    return (bad & 0xFF800000u) == 0;
 }
+
+// The same for levels of any size, read again from tensor memory.
+struct Four {
+    long long u[4];
+};
+__device__ __noinline__ Four join_levels_wide(unsigned at, int nc) {
+    unsigned l[kLev][4];
+#pragma unroll
+    for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
+    tmem_wait(l);
+    Four r;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        auto level = [&](int v, float w) { return (long long)__float2int_rn(__uint_as_float(l[v][t]) * w); };
+        r.u[t] = (level(0, 1.f) << kSh) + (level(1, 512.f) << (kSh - 9)) + (level(2, 262144.f) << (kSh - 18)) +
+                 (level(3, 134217728.f) << (kSh - 27)) + (level(4, 68719476736.f) << (kSh - 36)) +
+                 level(5, (float)(1ull << kSh));
+    }
+    return r;
+}
+
+// t * 2^q as a double, rounded to nearest, for |t| < 2^63 and a result whose exponent is a normal
+// number's.  The leading bit goes to bit 62, the rounding addend cannot overflow, and the implicit bit
+// carries into the exponent field, as does rounding up to the next power of two.
 __device__ __forceinline__ double scaled_double(long long t, int q) {
-    if (q > -1023 && q < 960) return plain_double(t, q);
-    return scalbn(plain_double(t, 0), q);
+    const long long sg = t >> 63;
+    const unsigned long long u = (unsigned long long)((t ^ sg) - sg);
+    const unsigned uh = (unsigned)(u >> 32), ul = (unsigned)u;
+    const int lz = __clz((int)(uh ? uh : ul)) + (uh ? 0 : 32);
+    const unsigned long long mant = ((u << (lz - 1)) + 0x200) >> 10;
+    const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)(1085 + q - lz) << 20);
+    const double v = __hiloint2double((int)(hi | ((unsigned)(sg >> 32) & 0x80000000u)), (int)(unsigned)mant);
+    return u ? v : 0.0;
 }
 
 // ------------------------------------------------------------------ digits
@@ -466,11 +527,23 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits_half(DigArgs a) {
 struct GemmArgs {
     TcShape s;
     TcJob job[kTcMaxJobs];
-    int m, ks, nq[2], nchunk, nc, sh, nstage;  // m = n / 2
+    int m, ks, nq[2], nchunk, nc, nstage;  // m = n / 2
     unsigned tile0, ntile, units;
     const unsigned char *ws;
     const int *expo;
     int *err;
+};
+
+// Epilogue warps per quarter of the lanes.  Three leave 128 registers a thread (512^2 x 538 z transform:
+// 1.21 ms; four: 1.32 ms, two: 1.45 ms); half spectra wait for their even frequencies' integers from L2,
+// which a fourth hides (x_inverse of the same field: 1.45 against 1.79 ms).
+template <int MODE>
+struct Epi {
+    static constexpr int kQ = MODE == kC2R ? 4 : 3;
+    static constexpr int kThreads = 128 * kQ;
+    static constexpr int kLoadWarp = kThreads / 32, kMmaWarp = kLoadWarp + 1;
+    static constexpr int kBlock = kThreads + 64;
+    static constexpr int kGroups = (kMaxNc / 4 + kQ - 1) / kQ;  // groups of 4 outputs per epilogue warp
 };
 
 // A unit of work: one tile of 64 columns, one parity of the frequency, one chunk of nc outputs.  The
@@ -501,14 +574,10 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
     return w;
 }
 
-// the general form of an output: any exponent, a non-finite column, a further factor
-__device__ __noinline__ double output_general(long long t, int q, int e, double post) {
-    const double v = scaled_double(t, q);
-    return e >= kNaN ? __longlong_as_double(0x7ff8000000000000ll) : v * post;
-}
-
 template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
+__global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
+    constexpr int kLoadWarp = Epi<MODE>::kLoadWarp, kMmaWarp = Epi<MODE>::kMmaWarp, kEpiQ = Epi<MODE>::kQ,
+                  kGroups = Epi<MODE>::kGroups;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned long long bars[2 * 8 + 2];
     __shared__ unsigned s_tmem;
@@ -527,7 +596,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
             mbar_init(empty + 8 * i, 1);
         }
         mbar_init(accfull, 1);
-        mbar_init(accempty, kEpi);
+        mbar_init(accempty, Epi<MODE>::kThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -543,21 +612,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
     const int nit = (MODE == kC2R ? 4 : 2) * a.ks;  // steps of a unit: cosine list, sine list (of each parity)
     if (warp == kLoadWarp) {
         if (lane == 0) {
-            int it = 0;  // steps issued so far, over all units
+            int it = 0, st = 0, ph = 1;  // steps issued so far, their stage and the phase its buffer is free after
             bool ok = true;
             for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit w = unit_of<MODE>(a, u);
                 const unsigned char *A = a.ws + (((size_t)w.job * a.ntile + w.lt) * 4 + 2 * w.par) * a.ks * kAStage;
                 const unsigned char *B = a.job[w.job].mat + ((size_t)w.par * 2 * a.nchunk + w.chunk) * a.ks * b_bytes;
+                int ks = 0;
                 for (int i = 0; i < nit; i++, it++) {
-                    const int st = it % a.nstage, round = it / a.nstage;
-                    if (round && !mbar_wait(empty + 8 * st, (round - 1) & 1, ab)) { ok = false; break; }
-                    const int list = i / a.ks;
+                    if (it >= a.nstage && !mbar_wait(empty + 8 * st, ph, ab)) { ok = false; break; }
                     const unsigned dst = smem_u32(smem) + st * stage_bytes;
                     mbar_expect(full + 8 * st, stage_bytes);
                     bulk_load(dst, A + (size_t)i * kAStage, kAStage, full + 8 * st);
-                    bulk_load(dst + kAStage, B + ((size_t)list * a.nchunk * a.ks + (i - list * a.ks)) * b_bytes, b_bytes,
-                              full + 8 * st);
+                    bulk_load(dst + kAStage, B, b_bytes, full + 8 * st);
+                    B += b_bytes;
+                    if (++ks == a.ks) {  // the next list's matrix of the same chunk
+                        ks = 0;
+                        B += (size_t)(a.nchunk - 1) * a.ks * b_bytes;
+                    }
+                    if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
             }
             if (!ok)  // giving up: this block's own copies land before it ends
@@ -567,62 +640,56 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
                 }
         }
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
-            // D FP32, A and B bf16, both K-major, N = nc, M = 128
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nc >> 3) << 17) | (8u << 24);
-            int it = 0, lists = 0;
-            bool ok = true;
-            for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x)
-                for (int i = 0; i < nit; i++, it++) {
-                    const int st = it % a.nstage, round = it / a.nstage;
-                    const bool first = i % a.ks == 0;
-                    if (first && lists) {  // the previous list's sums have left tensor memory
-                        ok = mbar_wait(accempty, (lists - 1) & 1, ab);
-                        if (!ok) break;
-                        fence_after();
-                    }
-                    ok = mbar_wait(full + 8 * st, round & 1, ab);
+        // D FP32, A and B bf16, both K-major, N = nc, M = 128
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nc >> 3) << 17) | (8u << 24);
+        const unsigned lead = elect_one();
+        int st = 0, ph = 0, lists = 0;
+        bool ok = true;
+        for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x)
+            for (int list = 0; list < nit && ok; list += a.ks, lists++) {
+                if (lists) {  // the previous list's sums have left tensor memory
+                    ok = __all_sync(~0u, mbar_wait(accempty, (lists - 1) & 1, ab));
                     if (!ok) break;
                     fence_after();
-                    const unsigned sa = smem_u32(smem) + st * stage_bytes, sb = sa + kAStage;
-// neighbours in this order add to different accumulators
+                }
+                for (int i = 0; i < a.ks; i++) {
+                    ok = __all_sync(~0u, mbar_wait(full + 8 * st, ph, ab));
+                    if (!ok) break;
+                    fence_after();
+                    const unsigned sa = smem_u32(smem) + st * stage_bytes;
+                    const unsigned long long da = smem_desc(sa, kLanes * 16, 128), db = smem_desc(sa + kAStage, nc * 16, 128);
+                    const unsigned keep = i != 0;
+                    // neighbours in this order add to different accumulators; address fields count 16 bytes
 #pragma unroll
                     for (int d = 0; d < kDig; d++)
 #pragma unroll
                         for (int j = 0; j < kDig - d; j++) {
                             const int acc = d + j < kLev ? d + j : kLev - 1;
-                            const bool fresh = first && d == 0 && j < kLev;
-                            mma_bf16(tmem + acc * nc, smem_desc(sa + d * (kLanes * 32), kLanes * 16, 128),
-                                     smem_desc(sb + j * (nc * 32), nc * 16, 128), idesc, fresh ? 0u : 1u);
+                            mma_bf16(tmem + acc * nc, da + d * (kLanes * 2), db + j * (nc * 2), idesc,
+                                     d == 0 && j < kLev ? keep : 1u, lead);
                         }
-                    mma_commit(empty + 8 * st);
-                    if ((i + 1) % a.ks == 0) {
-                        mma_commit(accfull);
-                        lists++;
-                    }
+                    mma_commit(empty + 8 * st, lead);
+                    if (i == a.ks - 1) mma_commit(accfull, lead);
+                    if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
-        }
+            }
     } else {
-        // 16 warps: quarter q of the lanes, every fourth group of 4 outputs
-        const int quad = warp & 3, g0 = warp >> 2, ngr = nc / 16;
+        // a warp holds a quarter of the lanes and every kEpiQ-th group of 4 outputs
+        const int quad = warp & 3, g0 = warp >> 2, ngr = (nc / 4 - g0 + kEpiQ - 1) / kEpiQ;
         const int r = quad * 32 + lane;
         const unsigned taddr = tmem + ((unsigned)(quad * 32) << 16);
         long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;  // [nc][128]
-        const int sh = a.sh;
-        const float fsh = (float)(1ull << sh);
-        // the levels of 4 outputs as integers in units of 2^-sh
-        auto gather = [&](int col, long long (&u)[4]) {
-            float l[kLev][4];
+        // the levels of 4 outputs, and those as integers
+        auto fetch = [&](int gi, unsigned (&l)[kLev][4]) {
+            const unsigned at = taddr + (g0 + kEpiQ * gi) * 4;
 #pragma unroll
-            for (int v = 0; v < kLev; v++) tmem_ld4(l[v], taddr + v * nc + col);
-            tmem_wait_ld();
+            for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
+        };
+        auto gather = [&](int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
+            if (__any_sync(~0u, !join_levels(l, u))) {
+                const Four w = join_levels_wide(taddr + (g0 + kEpiQ * gi) * 4, nc);
 #pragma unroll
-            for (int t = 0; t < 4; t++) {
-                const int i0 = __float2int_rn(l[0][t]), i1 = __float2int_rn(l[1][t] * 512.f),
-                          i2 = __float2int_rn(l[2][t] * 262144.f), i3 = __float2int_rn(l[3][t] * 134217728.f),
-                          i4 = __float2int_rn(l[4][t] * 68719476736.f), i5 = __float2int_rn(l[5][t] * fsh);
-                const long long A = (long long)i0 * 262144 + ((long long)i1 * 512 + i2);
-                u[t] = (A << (sh - 18)) + ((long long)i3 * (1 << (sh - 27)) + ((long long)i4 * (1 << (sh - 36)) + i5));
+                for (int t = 0; t < 4; t++) u[t] = w.u[t];
             }
         };
         int lists = 0;
@@ -641,81 +708,129 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm(GemmArgs a) {
                 off = (size_t)w.lt * s.ts + (size_t)r * s.ls;
             }
             const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * kLanes + r];
-            const int q = e - 1022 - 14 - sh + J.expo;
+            // results are t * 2^q: with an exponent 1086 + q - lz, 0 <= lz < 64, that could leave the normal
+            // numbers' a further power of two, times the job's own factor; NaN for a non-finite column
+            const int q = e - 1022 - 14 - kSh + J.expo, qc = max(-1000, min(q, 900));
+            const double fac = e >= kNaN ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(J.post, q - qc);
+            const bool mul = __any_sync(~0u, !(fac == 1.0));
             double *out = (double *)J.out + off;
             const double *add = MODE == kCol && J.add ? (const double *)J.add + off : nullptr;
-            // every result's exponent 1086 + q - lz, 0 <= lz < 64, is a normal number's
-            const bool plain = e < kNaN && q > -1023 && q < 960 && J.post == 1.0;
-            auto value = [&](long long t) { return plain ? plain_double(t, q) : output_general(t, q, e, J.post); };
+            auto value = [&](long long t) {
+                double v = scaled_double(t, qc);
+                // kept behind the branch: a multiplication of every value would bind the loop to the FP64 pipe
+                if (mul) asm volatile("mul.rn.f64 %0, %0, %1;" : "+d"(v) : "d"(fac));
+                return v;
+            };
             for (int par = w.par; par < (MODE == kC2R ? 2 : w.par + 1); par++) {
                 ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
                 if (!ok) break;
                 lists++;
                 fence_after();
-#pragma unroll 1
-                for (int gi = 0; gi < ngr; gi++) {
-                    const int col = (g0 + 4 * gi) * 4;
-                    long long P[4];
-                    gather(col, P);
+                // the next group's loads are in flight while a group is put together
+                unsigned l[2][kLev][4];
+                fetch(0, l[0]);
 #pragma unroll
-                    for (int t = 0; t < 4; t++) Ps[(col + t) * kLanes] = P[t];
-                }
+                for (int gi = 0; gi < kGroups; gi++)
+                    if (gi < ngr) {
+                        tmem_wait(l[gi & 1]);
+                        if (gi + 1 < ngr) fetch(gi + 1, l[(gi + 1) & 1]);
+                        long long P[4];
+                        gather(gi, l[gi & 1], P);
+#pragma unroll
+                        for (int t = 0; t < 4; t++) Ps[((g0 + kEpiQ * gi) * 4 + t) * kLanes] = P[t];
+                    }
                 fence_before();
                 mbar_arrive(accempty);
                 ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
                 if (!ok) break;
                 lists++;
                 fence_after();
-                long long Q[5][4];
+                long long Q[kGroups][4];
 #pragma unroll
-                for (int gi = 0; gi < 5; gi++)
-                    if (gi < ngr) gather((g0 + 4 * gi) * 4, Q[gi]);
+                for (int gi = 0; gi < kGroups; gi++)
+                    if (gi < ngr) {
+                        fetch(gi, l[0]);
+                        tmem_wait(l[0]);
+                        gather(gi, l[0], Q[gi]);
+                    }
                 fence_before();
                 mbar_arrive(accempty);
                 if (!live) continue;
+                // a group's loads, conversions and stores one after another: loads do not move across stores
 #pragma unroll
-                for (int gi = 0; gi < 5; gi++)
+                for (int gi = 0; gi < kGroups; gi++)
                     if (gi < ngr) {
-                        const int col = (g0 + 4 * gi) * 4;
+                        const int col = (g0 + kEpiQ * gi) * 4, j0 = w.chunk * nc + col;
+                        const int left = a.nq[MODE == kC2R ? 0 : par] - j0;  // outputs of this group that exist
+                        long long p[4];
 #pragma unroll
-                        for (int t = 0; t < 4; t++) {
-                            const int j = w.chunk * nc + col + t;
-                            if (j >= a.nq[MODE == kC2R ? 0 : par]) continue;
-                            const long long p = Ps[(col + t) * kLanes], d = Q[gi][t];
-                            if (MODE == kCol) {
-                                const int f = 2 * j + par, f2 = s.n - f;
-                                const long long sd = s.sign > 0 ? d : -d;
-                                if (f < s.nrows) {
-                                    const size_t o = 2 * (size_t)f * s.rs;
-                                    double v = value(p + sd);
-                                    if (add) v += add[o];
-                                    out[o] = v;
+                        for (int t = 0; t < 4; t++) p[t] = Ps[(col + t) * kLanes];
+                        if (MODE == kCol) {
+                            // fields hold fewer than 2^32 elements: 32-bit row offsets
+                            double v[4], v2[4];
+                            const int f0 = 2 * j0 + par;
+                            unsigned o = (unsigned)f0 * s.rs, o2 = (unsigned)(s.n - f0) * s.rs;
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                const long long d = s.sign > 0 ? Q[gi][t] : -Q[gi][t];
+                                v[t] = value(p[t] + d);
+                                v2[t] = value(p[t] - d);
+                            }
+#pragma unroll
+                            for (int t = 0; t < 4; t++, o += 2 * s.rs, o2 -= 2 * s.rs) {
+                                const int f = f0 + 2 * t, f2 = s.n - f;
+                                if (t < left && f < s.nrows) {
+                                    if (add) v[t] += add[2 * (size_t)o];
+                                    out[2 * (size_t)o] = v[t];
                                 }
-                                if (f && f != f2 && f2 < s.nrows) {
-                                    const size_t o = 2 * (size_t)f2 * s.rs;
-                                    double v = value(p - sd);
-                                    if (add) v += add[o];
-                                    out[o] = v;
+                                if (t < left && f && f != f2 && f2 < s.nrows) {
+                                    if (add) v2[t] += add[2 * (size_t)o2];
+                                    out[2 * (size_t)o2] = v2[t];
                                 }
-                            } else if (MODE == kR2C) {
-                                const int f = 2 * j + par;
-                                if (f <= a.m) *(double2 *)(out + 2 * f) = make_double2(value(p), value(-d));
+                            }
+                        } else if (MODE == kR2C) {
+                            double2 v[4];
+#pragma unroll
+                            for (int t = 0; t < 4; t++) v[t] = make_double2(value(p[t]), value(-Q[gi][t]));
+#pragma unroll
+                            for (int t = 0; t < 4; t++) {
+                                const int f = 2 * (j0 + t) + par;
+                                if (t < left && f <= a.m) *(double2 *)(out + 2 * f) = v[t];
+                            }
+                        } else {
+                            // even: A[k] = p - d, A[n/2 - k] = p + d; odd: B[k] = p - d, B[n/2 - k] = -p - d
+                            double *o0 = out + (size_t)j0 * s.rs, *o1 = out + (size_t)(a.m - j0) * s.rs;
+                            const size_t h = (size_t)a.m * s.rs;
+                            if (par == 0) {
+#pragma unroll
+                                for (int t = 0; t < 4; t++) {
+                                    const int j = j0 + t;
+                                    const long long d = Q[gi][t];
+                                    if (t < left) *(long long *)(o0 + (size_t)t * s.rs) = p[t] - d;
+                                    if (t < left && j && 2 * j != a.m) *(long long *)(o1 - (size_t)t * s.rs) = p[t] + d;
+                                }
                             } else {
-                                // even: A[k] = p - d, A[n/2 - k] = p + d; odd: B[k] = p - d, B[n/2 - k] = -p - d
-                                double *o0 = out + (size_t)j * s.rs, *o1 = out + (size_t)(a.m - j) * s.rs;
-                                const bool two = j && 2 * j != a.m;
-                                if (par == 0) {
-                                    *(long long *)o0 = p - d;
-                                    if (two) *(long long *)o1 = p + d;
-                                } else {
-                                    const size_t h = (size_t)a.m * s.rs;
-                                    const long long A = *(const long long *)o0, B = p - d;
-                                    o0[0] = value(A + B);
-                                    o0[h] = value(A - B);
-                                    if (two) {
-                                        const long long A1 = *(const long long *)o1, B1 = -p - d;
-                                        o1[0] = value(A1 + B1);
-                                        o1[h] = value(A1 - B1);
+                                long long A[4], A1[4];
+#pragma unroll
+                                for (int t = 0; t < 4; t++) {
+                                    const int j = j0 + t;
+                                    A[t] = t < left ? *(const long long *)(o0 + (size_t)t * s.rs) : 0;
+                                    A1[t] = t < left && j && 2 * j != a.m ? *(const long long *)(o1 - (size_t)t * s.rs) : 0;
+                                }
+#pragma unroll
+                                for (int t = 0; t < 4; t++) {
+                                    const int j = j0 + t;
+                                    const long long d = Q[gi][t], B = p[t] - d, B1 = -p[t] - d;
+                                    const double v0 = value(A[t] + B), v1 = value(A[t] - B);
+                                    const double v2 = value(A1[t] + B1), v3 = value(A1[t] - B1);
+                                    double *q0 = o0 + (size_t)t * s.rs, *q1 = o1 - (size_t)t * s.rs;
+                                    if (t < left) {
+                                        q0[0] = v0;
+                                        q0[h] = v1;
+                                    }
+                                    if (t < left && j && 2 * j != a.m) {
+                                        q1[0] = v2;
+                                        q1[h] = v3;
                                     }
                                 }
                             }
@@ -993,7 +1108,6 @@ void fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int 
     g.nq[1] = D.nq[1];
     g.nchunk = D.nchunk;
     g.nc = D.nc;
-    g.sh = D.sh;
     g.err = S->err_dev;
 }
 
@@ -1016,7 +1130,7 @@ void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     g.units = g.ntile * (MODE == kC2R ? 1 : 2) * D.nchunk * nj;
     const size_t smem = (size_t)g.nstage * stage + psize;
     cudaFuncSetAttribute(k_gemm<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_gemm<MODE><<<std::min(g.units, 152u), kGemmThreads, smem, P.stream>>>(g);
+    k_gemm<MODE><<<std::min(g.units, 152u), Epi<MODE>::kBlock, smem, P.stream>>>(g);
 }
 
 template <typename K>
