@@ -59,23 +59,73 @@ __global__ void k_narrow(const double2 *src, float2 *dst, size_t n) {
         dst[q] = make_float2((float)src[q].x, (float)src[q].y);
 }
 
-// float-float <-> FP64 fields of the nl_fp32 form (in place allowed: both are 16 bytes a
-// complex element), once per field per fused_step call, on the FP64 pipe (1.07 and 0.80 ms a
-// 512^2 x 538 field; splits by integer operations on the bit patterns measured no faster, their
-// fallback for magnitudes outside the float range diverging within warps).
-__global__ void k_d2q(const double2 *src, ffc *dst, size_t n) {
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const double2 v = src[q];
-        ffc r;
-        r.x = ff_from_double(v.x);
-        r.y = ff_from_double(v.y);
-        dst[q] = r;
+// float-float <-> FP64 fields of the nl_fp32 form (in place allowed: both are 16 bytes a complex
+// element), once per field per fused_step call.  On the FP64 pipe a 512^2 x 538 field took 1.07 and
+// 0.80 ms; on the bit patterns the copy is bound by memory.  The ranges taken so hold every value whose
+// pair is within the normal floats; zeros are apart, and what is left goes through FP64 arithmetic.
+
+// the pair of a double: its value rounded to 24 bits, and the rounded rest
+__device__ __forceinline__ ff ff_of(double v) {
+    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+    const int e = (int)((h >> 20) & 0x7ff);
+    const unsigned sign = h & 0x80000000u;
+    if (e >= 897 && e <= 1086) {  // 2^-126 <= |v| < 2^64
+        const unsigned f = __funnelshift_l(l, h, 3) & 0x7fffffu, rest = l & 0x1fffffffu;
+        const unsigned up = (rest + 0x0fffffffu + (f & 1u)) >> 29;  // to nearest, ties to even
+        const unsigned hi = (((unsigned)(e - 896) << 23) | f) + up;
+        const float r = __int2float_rn((int)rest - (int)(up << 29));  // times 2^(e - 1075)
+        const float lo = (r * __uint_as_float((unsigned)(e - 1075 + 64 + 127) << 23)) * 5.421010862427522e-20f;  // 2^-64
+        return ff(__uint_as_float(hi | sign), __uint_as_float(__float_as_uint(lo) ^ sign));
+    }
+    if (((h & 0x7fffffffu) | l) == 0) return ff(__uint_as_float(sign), 0.f);
+    return ff_from_double(v);
+}
+
+// the double nearest to a pair
+__device__ __forceinline__ double double_of(ff v) {
+    float s, r;
+    two_sum(v.hi, v.lo, s, r);
+    const unsigned b = __float_as_uint(s), f = b & 0x7fffffu;
+    const int e = (int)((b >> 23) & 0xff);
+    // r as an integer in units of 2^-52 of s's leading bit, signed as s
+    const float t = (r * 1.8446744073709552e19f) * __uint_as_float((unsigned)(242 - e) << 23);  // 2^64, 2^(115 - e)
+    if (e >= 1 && e <= 200 && (f || t * s >= 0.f)) {
+        const int q = (int)b < 0 ? -__float2int_rn(t) : __float2int_rn(t);
+        const long long m = ((long long)f << 29) + q;
+        const unsigned long long d = ((unsigned long long)(unsigned)(e + 896) << 52) + (unsigned long long)m;
+        return __longlong_as_double((long long)(d | ((unsigned long long)(b & 0x80000000u) << 32)));
+    }
+    return s == 0.f ? __hiloint2double((int)(b & 0x80000000u), 0) : ff_to_double(v);
+}
+
+constexpr int kConvert = 4;  // elements a thread has in flight
+__global__ void __launch_bounds__(256) k_d2q(const double2 *src, ffc *dst, size_t n) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += kConvert * step) {
+        double2 v[kConvert];
+#pragma unroll
+        for (int i = 0; i < kConvert; i++)
+            if (q + i * step < n) v[i] = src[q + i * step];
+#pragma unroll
+        for (int i = 0; i < kConvert; i++)
+            if (q + i * step < n) {
+                ffc r;
+                r.x = ff_of(v[i].x);
+                r.y = ff_of(v[i].y);
+                dst[q + i * step] = r;
+            }
     }
 }
-__global__ void k_q2d(const ffc *src, double2 *dst, size_t n) {
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-        const ffc v = src[q];
-        dst[q] = make_double2(ff_to_double(v.x), ff_to_double(v.y));
+__global__ void __launch_bounds__(256) k_q2d(const ffc *src, double2 *dst, size_t n) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += kConvert * step) {
+        float4 v[kConvert];
+#pragma unroll
+        for (int i = 0; i < kConvert; i++)
+            if (q + i * step < n) v[i] = *(const float4 *)(src + q + i * step);
+#pragma unroll
+        for (int i = 0; i < kConvert; i++)
+            if (q + i * step < n) dst[q + i * step] = make_double2(double_of(ff(v[i].x, v[i].y)), double_of(ff(v[i].z, v[i].w)));
     }
 }
 
