@@ -138,7 +138,9 @@ static int launch_x(Plan &P, const XArgs &a, int nf, bool r2c) {
     const dim3 grid(cdiv(a.nrows * P.ny, rb), 1, nf);
     const double rows = (double)a.nrows * P.ny;
     const double bytes = nf * rows * ((double)P.nxh * P.elt() + (double)P.nx * P.rel());
-    const int fst = fast_x(P, a, nf, r2c, bytes);
+    int fst;
+    if constexpr (is_f64<T>) fst = tc_x(P, a, nf, r2c, bytes);
+    else fst = fast_x(P, a, nf, r2c, bytes);
     if (fst != kNoFast) return fst;
     if (r2c) {
         set_smem(k_x_r2c<T, GenericFFT<T>>, sm);

@@ -29,6 +29,12 @@
 
 namespace sg {
 
+#define SG_TRY(x)                  \
+    do {                           \
+        int _st = (x);             \
+        if (_st != OK) return _st; \
+    } while (0)
+
 namespace {
 
 constexpr int kDig = 7;             // digits of data and matrix
@@ -80,7 +86,6 @@ struct TcState {
     size_t expo_count = 0;
     double *phys = nullptr;       // physical rows of the nonlinear term's x pass, one range of tiles
     size_t phys_tiles = 0;        // tiles of it per field
-    double2 *ext = nullptr;       // continuation rows of kMaxF fields
     int *err = nullptr, *err_dev = nullptr;  // host-mapped: set by a kernel that gave up a wait
 };
 
@@ -246,6 +251,8 @@ __device__ __forceinline__ double scaled_double(long long t, int q) {
 struct DigArgs {
     TcShape s;
     TcJob job[kTcMaxJobs];
+    const double *dir;      // FC-Gram matrix (s.next rows, column-major) and its matching points
+    int oz;
     int m, K, ks;
     unsigned tile0, ntile;  // tiles [tile0, tile0 + ntile) of every job
     unsigned char *ws;
@@ -395,23 +402,33 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
     constexpr int kParts = kLanes / LW, kCols = LW / 2;
     const unsigned lt = blockIdx.x / kParts;
     const int lane0 = (blockIdx.x % kParts) * LW;
-    const int n0 = J.ext ? s.n - s.next : s.n;  // rows below n0 come from the field
+    const int n0 = s.n - s.next;  // rows below n0 come from the field, the others from the continuation
     if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
     {
         const int cc = threadIdx.x % kCols;
         const unsigned c = (a.tile0 + lt) * 64 + lane0 / 2 + cc;
         const bool live = c < s.ncol;
-        const size_t off = live ? col_offset(s, c) : 0;
-        const double2 *in = J.in + off, *ext = J.ext ? J.ext + off : nullptr;
+        const double2 *in = J.in + (live ? col_offset(s, c) : 0);
         double2 *dst = (double2 *)smem + cc;
-        for (int row = threadIdx.x / kCols; row < s.n; row += kDigThreads / kCols) {
-            if (live) cp_async<16>(dst + row * kCols, row < n0 ? in + (size_t)row * s.rs : ext + (size_t)(row - n0) * s.es);
+        for (int row = threadIdx.x / kCols; row < n0; row += kDigThreads / kCols) {
+            if (live) cp_async<16>(dst + row * kCols, in + (size_t)row * s.rs);
             else dst[row * kCols] = make_double2(0.0, 0.0);
         }
         async_commit();
         async_wait();
     }
     __syncthreads();
+    if (s.next) {  // FC-Gram continuation (src/fftp/fftp.fpp:755-773), FP64, beside other blocks' integer work
+        const int C = s.next, d = a.oz, l = threadIdx.x % LW;
+        double *x = (double *)smem + l;
+        for (int i = threadIdx.x / LW; i < C; i += kDigThreads / LW) {
+            double v = __ldg(a.dir + i) * x[(n0 - d) * LW] + __ldg(a.dir + (C - 1 - i)) * x[(d - 1) * LW];
+            for (int j = 1; j < d; j++)
+                v = v + __ldg(a.dir + i + C * j) * x[(n0 - d + j) * LW] + __ldg(a.dir + (C - 1 - i) + C * j) * x[(d - 1 - j) * LW];
+            x[(n0 + i) * LW] = v;
+        }
+        __syncthreads();
+    }
     if (J.deriv) digits_body<true, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
     else digits_body<false, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
 }
@@ -442,11 +459,14 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits_real(DigArgs a, const
             dst[k * LW + l] = (u0 * d0 + u1 * d1 + u2 * d2) * scale;
         }
     } else {
-        const unsigned r0 = (a.tile0 + lt) * kLanes + lane0;
-        for (int i = threadIdx.x; i < s.n * LW; i += kDigThreads) {
-            const int l = i / s.n, k = i - l * s.n;
-            dst[k * LW + l] = r0 + l < s.ncol ? __ldg((const double *)J.in + (size_t)(r0 + l) * s.n + k) : 0.0;
-        }
+        // neighbouring threads read neighbouring rows (whose lines the next k find in L1), so that the writes
+        // to shared memory stay off one bank
+        const int l = threadIdx.x % LW;
+        const unsigned row = (a.tile0 + lt) * kLanes + lane0 + l;
+        const bool live = row < s.ncol;
+        const double *in = (const double *)J.in + (live ? (size_t)row * s.n : 0);
+#pragma unroll 4
+        for (int k = threadIdx.x / LW; k < s.n; k += kDigThreads / LW) dst[k * LW + l] = live ? __ldg(in + k) : 0.0;
     }
     __syncthreads();
     digits_body<false, true, LW>(a, job, dst, s_e, lt, lane0);
@@ -855,33 +875,16 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
     }
 }
 
-// FC-Gram continuation rows (src/fftp/fftp.fpp:755-773) of every column, FP64: a thread per real
-// lane; bound by the FP64 pipe (2 C d multiply-adds a lane).
-struct ContArgs {
-    const double *in[kMaxF];
-    double *ext[kMaxF];
-};
-__global__ void __launch_bounds__(128) k_continuation(Geo g, ContArgs a) {
-    const int C = g.cz, d = g.oz;
-    const size_t ps = 2 * (size_t)g.ny * g.ldx;
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= ps) return;
-    const double *in = a.in[blockIdx.y] + q;
-    double *ext = a.ext[blockIdx.y] + q;
-    double t[kMaxOz], b[kMaxOz];
-#pragma unroll
-    for (int j = 0; j < kMaxOz; j++)
-        if (j < d) {
-            t[j] = in[(size_t)(g.nzp - d + j) * ps];
-            b[j] = in[(size_t)(d - 1 - j) * ps];
-        }
-    for (int i = 0; i < C; i++) {
-        double x = __ldg(g.dir + i) * t[0] + __ldg(g.dir + (C - 1 - i)) * b[0];
-#pragma unroll
-        for (int j = 1; j < kMaxOz; j++)
-            if (j < d) x = x + __ldg(g.dir + i + C * j) * t[j] + __ldg(g.dir + (C - 1 - i) + C * j) * b[j];
-        ext[(size_t)i * ps] = x;
-    }
+// physical rows from tiles [tile][x][128 rows] to a field [row][x]
+__global__ void __launch_bounds__(256) k_untile(const double *tiles, double *out, int n, unsigned rows) {
+    __shared__ double t[32][33];
+    const unsigned r0 = blockIdx.x * 32, x0 = blockIdx.y * 32;
+    const double *src = tiles + (size_t)(r0 / kLanes) * n * kLanes + r0 % kLanes;
+    for (unsigned i = threadIdx.y; i < 32; i += 8)
+        if (x0 + i < (unsigned)n) t[i][threadIdx.x] = src[(size_t)(x0 + i) * kLanes + threadIdx.x];
+    __syncthreads();
+    for (unsigned i = threadIdx.y; i < 32; i += 8)
+        if (r0 + i < rows && x0 + threadIdx.x < (unsigned)n) out[(size_t)(r0 + i) * n + x0 + threadIdx.x] = t[threadIdx.x][i];
 }
 
 // ------------------------------------------------------------------ tables
@@ -1098,6 +1101,8 @@ void fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int 
     d.m = g.m = D.m;
     d.K = D.K;
     d.ks = g.ks = D.ks;
+    d.dir = P.geo.dir;
+    d.oz = P.oz;
     d.tile0 = g.tile0 = t0;
     d.ntile = g.ntile = nt;
     d.ws = S->ws;
@@ -1175,6 +1180,23 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
     return check_launch(name);
 }
 
+// Buffer of physical rows in tiles ([field][tile][x][128 rows]), sized for the 15 fields of the nonlinear
+// term's x pass over one range of tiles; its address is fixed like the digits'.
+static int phys_rows(Plan &P) {
+    TcState *S = P.tc;
+    if (S->phys) return OK;
+    const size_t per = 4ull * dims(P.nx).ks * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const size_t all = ((size_t)P.nzp * P.ny + kLanes - 1) / kLanes, t = std::min(all, std::max<size_t>(cap / kTcMaxJobs, 1));
+    if (cudaMalloc(&S->phys, t * 15 * P.nx * kLanes * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        S->phys = nullptr;
+        set_error("out of device memory (physical rows)");
+        return ERR_OOM;
+    }
+    S->phys_tiles = t;
+    return OK;
+}
+
 // gradre / advect between the y passes (pseudospec_hd.f90:209-319, pseudospec_phd.f90:23-113): the
 // velocity and the derivatives of components [c0, c1) to physical rows, the products, and back, in
 // ranges of tiles whose physical rows ([field][tile][x][128 rows]) stay in a buffer of the plan.
@@ -1196,17 +1218,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
     const size_t per = 4ull * D.ks * kAStage, ptile = (size_t)n * kLanes;
     const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
-    const unsigned alltiles = ((unsigned)P.nzp * P.ny + kLanes - 1) / kLanes;
-    if (!S->phys) {  // sized for four components; its address is fixed like the digits'
-        const size_t t = std::min<size_t>(alltiles, std::max<size_t>(cap / kTcMaxJobs, 1));
-        if (cudaMalloc(&S->phys, t * 15 * ptile * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            S->phys = nullptr;
-            set_error("out of device memory (physical rows)");
-            return ERR_OOM;
-        }
-        S->phys_tiles = t;
-    }
+    SG_TRY(phys_rows(P));
     const unsigned tstep = (unsigned)std::min<size_t>(S->phys_tiles, tiles);
     const size_t fstride = S->phys_tiles * ptile;
     const int lw = digit_lanes(n);
@@ -1272,40 +1284,11 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
     return check_launch("x_nonlinear");
 }
 
-int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf) {
-    TcState *S = state(P);
-    const size_t rows = (size_t)P.cz * P.ny * P.ldx;
-    if (!S->ext && cudaMalloc(&S->ext, kMaxF * rows * sizeof(double2)) != cudaSuccess) {
-        cudaGetLastError();
-        S->ext = nullptr;
-        set_error("out of device memory (continuation rows)");
-        return ERR_OOM;
-    }
-    ContArgs a{};
-    for (int f = 0; f < nf; f++) {
-        a.in[f] = (const double *)in[f];
-        a.ext[f] = (double *)(S->ext + f * rows);
-        ext[f] = S->ext + f * rows;
-    }
-    const size_t per = 2 * (size_t)P.ny * P.ldx;
-    {
-        Launch L(P, "continuation", nf * 8.0 * per * (2 * P.oz + P.cz));
-        k_continuation<<<dim3((unsigned)((per + 127) / 128), nf), 128, 0, P.stream>>>(P.geo, a);
-    }
-    return check_launch("continuation");
-}
-
-#define SG_TRY(x)                  \
-    do {                           \
-        int _st = (x);             \
-        if (_st != OK) return _st; \
-    } while (0)
-
 // FP64 passes over the digit-product transforms (tcdft.cu).  They serve every even length of 32 to
 // 550: at all of them they are faster than the FP64 Stockham engine, which the FP64 pipe bounds.
 // kNoFast: a form that they do not take (another length, a scale on part of the rows).
 static int tc_add(Plan &P, TcJob *jobs, int *nj, int n, double factor, const void *in, void *out, const void *add,
-                  int deriv, const double2 *ext) {
+                  int deriv) {
     int st = OK;
     const TcSet *set = tc_set(P, n, factor, &st);
     if (!set) return st;
@@ -1314,7 +1297,6 @@ static int tc_add(Plan &P, TcJob *jobs, int *nj, int n, double factor, const voi
     j.in = (const double2 *)in;
     j.out = (double2 *)out;
     j.add = (const double2 *)add;
-    j.ext = ext;
     j.deriv = deriv;
     tc_job_set(j, set);
     return OK;
@@ -1325,7 +1307,7 @@ static TcShape tc_z_shape(const Plan &P, int sign, int nrows) {
     s.n = P.nz;
     s.sign = sign;
     s.nrows = nrows;
-    s.ncol = s.w = s.s = s.rs = s.es = (unsigned)P.ny * P.ldx;
+    s.ncol = s.w = s.s = s.rs = (unsigned)P.ny * P.ldx;
     return s;
 }
 
@@ -1336,22 +1318,85 @@ int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes) {
     int nj = 0;
     // derivatives first: out0 may alias in
     for (int f = 0; f < nf; f++)
-        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, P.Dkz * sc, a.in[f], a.out1[f], nullptr, 1, nullptr));
+        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, P.Dkz * sc, a.in[f], a.out1[f], nullptr, 1));
     for (int f = 0; f < nf; f++)
-        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, sc, a.in[f], a.out0[f], a.add[f], 0, nullptr));
+        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.nz, sc, a.in[f], a.out0[f], a.add[f], 0));
     return tc_run(P, tc_z_shape(P, +1, a.nrows), jobs, nj, "z_inverse", bytes);
 }
 
 int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
     if (!tc_length_ok(P.nz) || a.in_scale != 1.0) return kNoFast;
-    const double2 *ext[kMaxF];
-    SG_TRY(tc_continuation(P, a.in, ext, nf));
     TcJob jobs[kTcMaxJobs];
     int nj = 0;
-    for (int f = 0; f < nf; f++) SG_TRY(tc_add(P, jobs, &nj, P.nz, 1.0, a.in[f], a.out[f], nullptr, 0, ext[f]));
+    for (int f = 0; f < nf; f++) SG_TRY(tc_add(P, jobs, &nj, P.nz, 1.0, a.in[f], a.out[f], nullptr, 0));
     TcShape s = tc_z_shape(P, -1, P.nz);
     s.next = P.cz;
     return tc_run(P, s, jobs, nj, "z_forward", bytes);
+}
+
+// Rows of fields: real rows to half spectra (r2c) and back.  Back they go through tiles whose writes are
+// coalesced (written row by row, 256^2 x 282 took 439 us instead of 251 and 61 for the copy).  Shorter rows
+// stay with the Stockham engine (half spectra to rows at 64^2 x 90: 33 us against 47; at 128^2 x 154 121
+// against 112, at 256^2 x 282 758 against 420).
+int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
+    if (!tc_length_ok(P.nx) || P.nx < 96) return kNoFast;
+    SG_TRY(workspace(P));
+    if (!r2c) SG_TRY(phys_rows(P));
+    SG_TRY(tc_status(P));
+    TcState *S = P.tc;
+    int st = OK;
+    const TcSet *set = tc_set(P, P.nx, a.scale, &st, !r2c);
+    if (!set) return st;
+    const Dims D = dims(P.nx);
+    const size_t per = 4ull * D.ks * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const unsigned rows = (unsigned)a.nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
+    const unsigned tstep = (unsigned)std::min<size_t>(tiles, r2c ? cap : std::min(cap, 15 * S->phys_tiles));
+    const int lw = digit_lanes(P.nx);
+    const char *name = r2c ? "x_r2c" : "x_c2r";
+    for (int f = 0; f < nf; f++)
+        for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
+            const unsigned nt = std::min(tstep, tiles - t0);
+            TcShape s{};
+            s.n = P.nx;
+            s.ncol = rows;
+            s.rs = r2c ? 1 : P.ldx;
+            s.ls = r2c ? 2 * P.ldx : 1;
+            s.ts = (size_t)kLanes * (r2c ? s.ls : P.nx);
+            TcJob J{};
+            J.in = (const double2 *)a.in[f];
+            J.out = r2c ? (double2 *)((double *)a.out[f] + t0 * s.ts) : (double2 *)S->phys;
+            tc_job_set(J, set);
+            DigArgs d{};
+            GemmArgs g{};
+            fill_args(P, D, s, &J, 1, t0, nt, d, g);
+            const size_t blocks = (size_t)nt * (kLanes / lw);
+            const dim3 grid((unsigned)blocks, digit_split(D, lw, blocks), 1);
+            const double share = bytes * nt / ((double)tiles * nf);
+            {
+                Launch L(P, "digits", share * 0.5 + (double)nt * per);
+                if (r2c) {
+                    const size_t sm = (size_t)P.nx * lw * sizeof(double);
+                    with_smem(lw == 32 ? k_digits_real<32, false> : k_digits_real<16, false>, sm)
+                        <<<grid, kDigThreads, sm, P.stream>>>(d, nullptr, 0, 1.0);
+                } else {
+                    const size_t sm = (size_t)(D.m + 1) * (lw + 1) * sizeof(double2);
+                    with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm)<<<grid, kDigThreads, sm, P.stream>>>(d);
+                }
+            }
+            g.s.rs = r2c ? 1 : kLanes;
+            {
+                Launch L(P, name, share);
+                if (r2c) launch_gemm<kR2C>(P, D, g, 1);
+                else launch_gemm<kC2R>(P, D, g, 1);
+            }
+            if (!r2c) {
+                const unsigned left = std::min(rows - t0 * kLanes, nt * kLanes);
+                Launch L(P, "untile", 16.0 * left * P.nx);
+                k_untile<<<dim3((left + 31) / 32, (P.nx + 31) / 32), dim3(32, 8), 0, P.stream>>>(
+                    S->phys, (double *)a.out[f] + (size_t)t0 * kLanes * P.nx, P.nx, left);
+            }
+        }
+    return check_launch(name);
 }
 
 int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes) {
@@ -1359,9 +1404,9 @@ int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes) {
     TcJob jobs[kTcMaxJobs];
     int nj = 0;
     for (int f = 0; f < nf; f++)
-        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, P.Dky * a.scale, a.in[f], a.out1[f], nullptr, 1, nullptr));
+        if (a.out1[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, P.Dky * a.scale, a.in[f], a.out1[f], nullptr, 1));
     for (int f = 0; f < nf; f++)
-        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, a.scale, a.in[f], a.out0[f], nullptr, 0, nullptr));
+        if (a.out0[f]) SG_TRY(tc_add(P, jobs, &nj, P.ny, a.scale, a.in[f], a.out0[f], nullptr, 0));
     TcShape s{};
     s.n = P.ny;
     s.sign = a.sign;
@@ -1377,7 +1422,6 @@ void tc_free(Plan &P) {
     for (auto &e : P.tc->sets) cudaFree(e.second.mat);
     if (P.tc->ws) cudaFree(P.tc->ws);
     if (P.tc->expo) cudaFree(P.tc->expo);
-    if (P.tc->ext) cudaFree(P.tc->ext);
     if (P.tc->phys) cudaFree(P.tc->phys);
     if (P.tc->err) cudaFreeHost(P.tc->err);
     delete P.tc;
@@ -1388,7 +1432,6 @@ unsigned long long tc_bytes(const Plan &P) {
     if (!P.tc) return 0;
     unsigned long long b = P.tc->ws_bytes + P.tc->expo_count * sizeof(int);
     b += (unsigned long long)P.tc->phys_tiles * 15 * P.nx * kLanes * sizeof(double);
-    if (P.tc->ext) b += (unsigned long long)kMaxF * P.cz * P.ny * P.ldx * sizeof(double2);
     for (const auto &e : P.tc->sets) b += e.second.bytes;
     return b;
 }

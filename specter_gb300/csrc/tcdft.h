@@ -8,6 +8,7 @@ namespace sg {
 struct ZInvArgs;
 struct ZFwdArgs;
 struct YArgs;
+struct XArgs;
 struct XNLArgs;
 
 constexpr int kTcMaxJobs = 16;  // transforms per launch
@@ -19,7 +20,6 @@ struct TcJob {
     const double2 *in;
     double2 *out;
     const double2 *add;   // added to the result when not null (same layout as out)
-    const double2 *ext;   // rows [n - next, n) of the input come from here when not null
     const unsigned char *mat;  // matrix digits of the table set
     int deriv, expo;      // expo: power of two of the set's factor
     double post;          // further factor applied to the result (1: none)
@@ -28,9 +28,8 @@ struct TcJob {
 // Columns: column c of a launch is at element (c / w) * s + c % w of a field, c in [0, ncol).
 struct TcShape {
     int n, sign, nrows;         // nrows: rows of the result that are written
-    int next;                   // rows taken from ext
+    int next;                   // rows [n - next, n) of the input are the FC-Gram continuation (0: none)
     unsigned ncol, w, s, rs;    // rs: row stride of in and out
-    unsigned es;                // row stride of ext (its columns are laid out as the field's)
     // transforms of rows: ncol rows; row r of tile t (128 rows) starts at t * ts + r * ls of the output
     unsigned ls;
     size_t ts;
@@ -48,10 +47,8 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
 int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes);
 int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes);
 int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes);
+int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes);
 int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes);
-// continuation rows of FC-Gram columns of nf <= kMaxF fields, in a buffer of the plan:
-// ext[f][(i * ny + ky) * ldx + kx], i < cz
-int tc_continuation(Plan &P, const void *const in[], const double2 *ext[], int nf);
 void tc_free(Plan &P);
 unsigned long long tc_bytes(const Plan &P);
 // non-zero when a kernel of the plan gave up a wait (checked after synchronising)

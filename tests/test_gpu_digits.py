@@ -57,6 +57,27 @@ def test_xy_round_trip(ny):
     assert np.linalg.norm(o.download() / (16 * ny) - r) < TOL * np.linalg.norm(r)
 
 
+@pytest.mark.parametrize("nx", [94, 96, 98, 130, 254, 256, 512, 550])
+def test_x_rows(nx):
+    p = plan(nx, 6, 36)  # 216 rows: the second tile of 128 is not full
+    rng = np.random.default_rng(nx)
+    r = rng.standard_normal(p.rshape)
+    r[3, 2] *= 1e-200
+    r[4, 1] = 0
+    f, c, o = p.field(api.REAL, data=r), p.field(), p.field(api.REAL)
+    api.fftp2d_real_to_complex_xy(p, f, c)
+    want = np.fft.rfft2(r).transpose(2, 1, 0)
+    assert np.linalg.norm(c.download() - want) < TOL * np.linalg.norm(want)
+    # any half spectrum: the imaginary parts of frequencies 0 and nx/2 do not count (of the y transform's
+    # results, as of irfft's input)
+    a = rng.standard_normal(p.sshape) + 1j * rng.standard_normal(p.sshape)
+    c.upload(a)
+    api.fftp2d_complex_to_real_xy(p, c, o)
+    y = np.fft.ifft(a.transpose(2, 1, 0), axis=1) * 6
+    want = np.fft.irfft(y, n=nx, axis=2) * nx
+    assert np.linalg.norm(o.download() - want) < TOL * np.linalg.norm(want)
+
+
 def test_non_finite_and_denormal_columns():
     p = plan(8, 4, 58)
     rng = np.random.default_rng(0)
