@@ -79,13 +79,13 @@ static int wall_check_static(Plan &P, const void *a, const void *b, double *bot,
     double2 *bcA = (double2 *)base, *bcB = bcA + kWallSlots;
     double *partial = base + 2 * 2 * kWallSlots, *result = partial + 2 * kStaticBlocks;
     const double2 *wtw = (const double2 *)P.dwtw;
-    const dim3 grid(cdiv(P.nxh, 64), P.ny);
+    const dim3 grid(cdiv(P.nxh, 32), P.ny), block(32, kWallSlices);
     const double col = (double)P.nz * P.ny * P.nxh * (double)P.elt();  // one field read
     if (cudaMemsetAsync(result, 0, 2 * sizeof(double), P.stream) != cudaSuccess) return check_launch("bouncheck_z_static clear");
-    { Launch L_(P, "wall_eval", col); k_wall_eval<T><<<grid, 64, 0, P.stream>>>(P.geo, (const C2<T> *)a, 1.0, wtw, bcA, 0); }
+    { Launch L_(P, "wall_eval", col); k_wall_eval<T><<<grid, block, 0, P.stream>>>(P.geo, (const C2<T> *)a, 1.0, wtw, bcA, 0); }
     if (int st = check_launch("bouncheck_z_static wall_eval")) return st;
     if (b) {
-        { Launch L_(P, "wall_eval", col); k_wall_eval<T><<<grid, 64, 0, P.stream>>>(P.geo, (const C2<T> *)b, 1.0, wtw, bcB, 0); }
+        { Launch L_(P, "wall_eval", col); k_wall_eval<T><<<grid, block, 0, P.stream>>>(P.geo, (const C2<T> *)b, 1.0, wtw, bcB, 0); }
         if (int st = check_launch("bouncheck_z_static wall_eval")) return st;
     }
     { Launch L_(P, "reduce_walls", 64.0 * P.nxh * P.ny); k_reduce_walls<<<kStaticBlocks, kThreads, 0, P.stream>>>(P.geo, bcA, b ? bcB : nullptr, partial); }

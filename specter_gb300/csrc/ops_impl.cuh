@@ -7,6 +7,7 @@
 #include "kernels.cuh"
 #include "kernels_elem.cuh"
 #include "ops.h"
+#include "stage_f64.h"
 #include "tcdft.h"
 
 namespace sg {
@@ -189,8 +190,8 @@ static int scratch(Plan &P, int n, void **out) {
 
 // sum block partials on the host in a fixed order (deterministic)
 static int finish_reduce(Plan &P, int nblocks, int per, double *out) {
-    std::vector<double> h((size_t)nblocks * per);
-    if (cudaMemcpyAsync(h.data(), P.dred, h.size() * sizeof(double), cudaMemcpyDeviceToHost, P.stream) != cudaSuccess ||
+    double *h = P.hred;  // pinned: nred doubles
+    if (cudaMemcpyAsync(h, P.dred, (size_t)nblocks * per * sizeof(double), cudaMemcpyDeviceToHost, P.stream) != cudaSuccess ||
         cudaStreamSynchronize(P.stream) != cudaSuccess)
         return check_launch("reduce");
     for (int j = 0; j < per; j++) {
@@ -384,8 +385,10 @@ template <typename T> int Ops<T>::energy(Plan &P, const void *a, const void *b, 
     } else if (kin == 0) {
         SG_TRY(curlk(P, b, c, S[3], 1));
         SG_TRY(curlk(P, a, c, S[4], 2));
-        const void *in[3] = {S[3], S[4], S[4]};
-        SG_TRY(zinv_scratch<T>(P, in, 3, S));
+        // the y-curl enters twice: transformed once
+        const void *in[2] = {S[3], S[4]};
+        SG_TRY(zinv_scratch<T>(P, in, 2, S));
+        S[2] = S[1];
         r.nf = 3;
     } else if (kin == 2) {
         SG_TRY(curlk(P, b, c, S[3], 1));
@@ -412,6 +415,27 @@ template <typename T> int Ops<T>::energy(Plan &P, const void *a, const void *b, 
 template <typename T> int Ops<T>::helicity(Plan &P, const void *a, const void *b, const void *c, double *out) {
     void *S[6];
     SG_TRY(scratch(P, 6, S));
+    if constexpr (is_f64<T>) {
+        // the curl of the transformed velocity and its z derivatives: five transforms instead of six, and no
+        // curl fields
+        ZInvArgs z{};
+        const void *v[3] = {a, b, c};
+        for (int i = 0; i < 3; i++) {
+            z.in[i] = v[i];
+            z.out0[i] = S[i];
+            z.out1[i] = i < 2 ? S[3 + i] : nullptr;
+        }
+        z.nrows = P.nzp;
+        z.scale = 1.0;
+        SG_TRY(launch_z_inverse<T>(P, z, 3));
+        RedArgs r{};
+        r.mode = 2; r.z1 = P.nzp; r.nf = 5;
+        for (int i = 0; i < 5; i++) r.f[i] = S[i];
+        double s;
+        SG_TRY(reduce<T>(P, r, &s));
+        *out = s * (inv_n2(P) / (double)(P.nz - P.cz));
+        return OK;
+    }
     SG_TRY(curlk(P, b, c, S[3], 1));
     SG_TRY(curlk(P, a, c, S[4], 2));
     SG_TRY(curlk(P, a, b, S[5], 3));
@@ -510,7 +534,7 @@ static double2 *plan_bc(Plan &P, int i) { return (double2 *)P.scratch_field(kScr
 
 template <typename T>
 static int wall_eval(Plan &P, const void *in, double scale, double2 *bc, int neg) {
-    { Launch L_(P, "wall_eval", cplx_rows(P, P.nz)); k_wall_eval<T><<<dim3(cdiv(P.nxh, 64), P.ny), 64, 0, P.stream>>>(P.geo, F<T>(in), scale, plan_wtw(P), bc, neg); }
+    { Launch L_(P, "wall_eval", cplx_rows(P, P.nz)); k_wall_eval<T><<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, kWallSlices), 0, P.stream>>>(P.geo, F<T>(in), scale, plan_wtw(P), bc, neg); }
     return check_launch("wall_eval");
 }
 
@@ -539,6 +563,22 @@ template <typename T> int Ops<T>::sol_project(Plan &P, void *a, void *b, void *c
     SG_TRY(scratch(P, 3, S));
     double2 *bc = plan_bc(P, 0), *coef = plan_bc(P, 1);
     if (!bc || !coef) { set_error("out of device memory"); return ERR_OOM; }
+    if constexpr (is_f64<T>) {
+        // the Poisson solve with the wall sums, and the profiles from tables of exponentials
+        if (bctarget == 1) {
+            SG_TRY(f64_poisson(P, a, b, c, d, nullptr, coef));
+            SG_TRY(f64_profile(P, coef, S[1], S[2]));
+            ZInvArgs z{};
+            z.in[0] = d; z.out0[0] = d; z.add[0] = S[1];
+            z.nrows = P.nz; z.scale_rows = P.nz; z.scale = 1.0 / (double)P.nz;
+            SG_TRY(launch_z_inverse<T>(P, z, 1));
+            ZFwdArgs f{};
+            f.in[0] = S[1]; f.out[0] = S[1]; f.in[1] = S[2]; f.out[1] = S[2]; f.in_scale = 1.0;
+            SG_TRY(launch_z_forward<T>(P, f, 2));
+            { Launch L_(P, "proj_sub", 8.0 * cplx_rows(P, P.nz)); k_proj_sub<T><<<elem_blocks(P, P.nz), kThreads, 0, P.stream>>>(P.geo, F<T>(a), F<T>(b), F<T>(c), F<T>(S[1]), F<T>(S[2])); }
+            return check_launch("proj_sub");
+        }
+    }
     { Launch L_(P, "poisson", 8.0 * cplx_rows(P, P.nz)); k_poisson<T><<<elem_blocks(P, P.nz), kThreads, 0, P.stream>>>(P.geo, F<T>(a), F<T>(b), F<T>(c), F<T>(d), F<T>(S[0]), bctarget); }
     SG_TRY(check_launch("poisson"));
     SG_TRY(wall_eval<T>(P, S[0], 1.0, bc, bctarget == 0));

@@ -338,7 +338,7 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
         cudaMemcpy(p->dwtwq, wq.data(), wq.size() * sizeof(ff), cudaMemcpyHostToDevice);
         G.wtwq = p->dwtwq;
     }
-    cudaMallocHost(&p->hred, sizeof(double) * 64);
+    cudaMallocHost(&p->hred, sizeof(double) * p->nred);
     if (cudaGetLastError() != cudaSuccess) { set_error("CUDA error during plan creation"); plan_destroy(p); return ERR_CUDA; }
     *out = p;
     return OK;

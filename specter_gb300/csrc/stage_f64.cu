@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(32 * kSlices) k_stage_poisson(Geo g, double2 *
 // 512^2 x 513); with z = (32 i + j) dz, exp(-kh z) is the product of two table entries, and
 // exp(kh (z - Lz)) is the same read from the other wall.  A block holds 32 columns.
 constexpr int kProfJ = 32;
-__global__ void __launch_bounds__(256) k_stage_profile(Geo g, const double2 *coef, double2 *pr, double dz) {
+// With `deriv` also the profile's z derivative, and then all nz rows (those above nzp one by one).
+__global__ void __launch_bounds__(256) k_stage_profile(Geo g, const double2 *coef, double2 *prof, double2 *deriv, double dz) {
     extern __shared__ double tab[];  // [32 + ni][32 columns]: exp(-kh j dz), then exp(-kh 32 i dz)
     const int c = threadIdx.x, kx = blockIdx.x * 32 + c, ky = blockIdx.y;
     const bool on = kx < g.nxh;
@@ -161,15 +162,24 @@ __global__ void __launch_bounds__(256) k_stage_profile(Geo g, const double2 *coe
     if (!on) return;
     const double2 c1 = coef[2 * col], c2 = coef[2 * col + 1];
     auto ex = [&](int z) { return tab[(z % kProfJ) * 32 + c] * tab[(kProfJ + z / kProfJ) * 32 + c]; };
-    for (int z = threadIdx.y; z < g.nzp; z += blockDim.y) {
-        double2 v;
+    const int rows = deriv ? g.nz : g.nzp;
+    for (int z = threadIdx.y; z < rows; z += blockDim.y) {
+        const size_t q = fidx<double>(g, z, ky, kx);
         if (kx == 0 && ky == 0) {
-            v = make_double2(c1.x * g.z[z], 0.0);
-        } else {
-            const double e1 = ex(g.nzp - 1 - z), e2 = ex(z);
-            v = make_double2(c1.x * e1 + c2.x * e2, c1.y * e1 + c2.y * e2);
+            prof[q] = make_double2(c1.x * g.z[z] + c2.x, 0.0);
+            if (deriv) deriv[q] = make_double2(c1.x, 0.0);
+            continue;
         }
-        pr[fidx<double>(g, z, ky, kx)] = v;
+        double e1, e2;
+        if (z < g.nzp) {
+            e1 = ex(g.nzp - 1 - z);
+            e2 = ex(z);
+        } else {
+            e1 = exp(kh * (g.z[z] - g.Lz));
+            e2 = exp(-(kh * g.z[z]));
+        }
+        prof[q] = make_double2(c1.x * e1 + c2.x * e2, c1.y * e1 + c2.y * e2);
+        if (deriv) deriv[q] = make_double2(kh * (c1.x * e1 - c2.x * e2), kh * (c1.y * e1 - c2.y * e2));
     }
 }
 
@@ -217,6 +227,22 @@ int elem_blocks(const Plan &P) {
 }  // namespace
 
 bool f64_stage_ok(const Plan &P) { return tc_length_ok(P.nz); }
+
+int f64_poisson(Plan &P, void *vx, void *vy, void *vz, void *d, void *th, double2 *coef) {
+    const double field = (double)P.nz * P.ny * P.nxh * 16.0;
+    Launch L(P, "stage_poisson", (7.0 + (th ? 2.0 : 0.0)) * field);
+    k_stage_poisson<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, kSlices), 0, P.stream>>>(
+        P.geo, (double2 *)vx, (double2 *)vy, (double2 *)vz, (double2 *)d, (double2 *)th, coef);
+    return check_launch("poisson");
+}
+
+int f64_profile(Plan &P, const double2 *coef, void *prof, void *deriv) {
+    Launch L(P, "stage_profile", (deriv ? 2.0 * P.nz : (double)P.nzp) * P.ny * P.nxh * 16.0);
+    const size_t sm = (size_t)(kProfJ + cdiv(P.nzp, kProfJ)) * 32 * sizeof(double);
+    if (sm > 40 * 1024) cudaFuncSetAttribute(k_stage_profile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_stage_profile<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, 8), sm, P.stream>>>(P.geo, coef, (double2 *)prof, (double2 *)deriv, P.dz);
+    return check_launch("profile");
+}
 
 int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], const void *const cold[4],
               void *const vout[4], void *pr, void *const E[2]) {
@@ -287,16 +313,8 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
     }
     SG_TRY(forward(trip, nt));
     const bool trip2 = bouss && !rot;
-    {
-        Launch L(P, "stage_poisson", (7.0 + (trip2 ? 2.0 : 0.0)) * field);
-        k_stage_poisson<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, kSlices), 0, P.stream>>>(P.geo, x, y, w, (double2 *)d,
-                                                                                      trip2 ? th : nullptr, coef);
-    }
-    {
-        Launch L(P, "stage_profile", mixed);
-        const size_t sm = (size_t)(kProfJ + cdiv(P.nzp, kProfJ)) * 32 * sizeof(double);
-        k_stage_profile<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, 8), sm, P.stream>>>(P.geo, coef, (double2 *)pr, P.dz);
-    }
+    SG_TRY(f64_poisson(P, x, y, w, d, trip2 ? th : nullptr, coef));
+    SG_TRY(f64_profile(P, coef, pr, nullptr));
     {
         void *in[2] = {d, th}, *out[2] = {pr, th};
         const void *add[2] = {pr, nullptr};
