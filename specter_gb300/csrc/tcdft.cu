@@ -334,20 +334,26 @@ __device__ __forceinline__ int value_exponent(double v, int k) {
 // that it writes whole 16-byte rows of core matrices.  REAL: lanes are real rows; else lanes are the
 // real and imaginary parts of columns.
 template <bool DERIV, bool REAL, int LW>
-__device__ __forceinline__ void digits_body(const DigArgs &a, int job, const double *tile_s, int *s_e, unsigned lt,
+__device__ __forceinline__ void digits_body(const DigArgs &a, int job, double *tile_s, int *s_e, unsigned lt,
                                             int lane0) {
     const int n = a.s.n, m = a.m;
     const int l = threadIdx.x % LW, part = REAL ? 0 : l & 1, lane = lane0 + l;
-    const double *x = tile_s + l;
+    double *xd = tile_s + l;
+    long long *x = (long long *)xd;
     int emax = 0;
+    // rows as wavenumbers: r for r < m, r - n above
     for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW)
-        emax = max(emax, value_exponent<DERIV>(x[row * LW], row < m ? row : row - n));
+        emax = max(emax, value_exponent<DERIV>(xd[row * LW], row < m ? row : row - n));
     atomicMax(&s_e[REAL ? l : l & ~1], emax);
     __syncthreads();
     emax = s_e[REAL ? l : l & ~1];
     if (emax == 0) emax = 1023;  // a column of zeros: any exponent
     if (blockIdx.y == 0 && threadIdx.x < LW) a.expo[((size_t)job * a.ntile + lt) * kLanes + lane] = emax;
     if (emax >= kNaN) emax = 0x7ff;  // a non-finite column's digits are not used
+    // to integers in place, each value once (both parities of the frequency read it)
+    for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW)
+        x[row * LW] = fixed_point<DERIV>(xd[row * LW], row < m ? row : row - n, emax);
+    __syncthreads();
     unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage;
     // effective part: multiplying by i moves real data to imaginary lanes and imaginary data, negated,
     // to real lanes; so does the sine list of a complex transform
@@ -366,16 +372,9 @@ __device__ __forceinline__ void digits_body(const DigArgs &a, int job, const dou
                 c[t] = w[t] = 0;
                 if (k >= a.K) continue;
                 const bool self = k == 0 || 2 * k == m;
-                // row r as a wavenumber: r for r < m, r - n above
-                long long x0 = fixed_point<DERIV>(x[k * LW], k, emax);
-                long long x1 = fixed_point<DERIV>(x[(k + m) * LW], k - m, emax);
-                long long x2 = 0, x3 = 0;
-                if (!self) {
-                    x2 = fixed_point<DERIV>(x[(m - k) * LW], m - k, emax);
-                    x3 = fixed_point<DERIV>(x[(n - k) * LW], -k, emax);
-                }
-                if (par) { x1 = -x1; x3 = -x3; }
-                long long E = x0 + x1, E2 = x2 + x3;
+                const long long x0 = x[k * LW], x1 = x[(k + m) * LW];
+                const long long x2 = self ? 0 : x[(m - k) * LW], x3 = self ? 0 : x[(n - k) * LW];
+                long long E = par ? x0 - x1 : x0 + x1, E2 = par ? x2 - x3 : x2 + x3;
                 if (flip) { E = -E; E2 = -E2; }
                 // even: cos gets E + E', sin E - E'; odd: cos O - O', sin O + O'
                 if (par) E2 = -E2;
@@ -393,7 +392,7 @@ __device__ __forceinline__ void digits_body(const DigArgs &a, int job, const dou
 
 // Columns: LW = 16 keeps three blocks on an SM at n = 538 (69 KB), LW = 32 at up to half of that.
 template <int LW>
-__global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
+__global__ void __launch_bounds__(kDigThreads, 4) k_digits(DigArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_e[LW];
     const TcShape &s = a.s;
@@ -429,15 +428,15 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits(DigArgs a) {
         }
         __syncthreads();
     }
-    if (J.deriv) digits_body<true, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
-    else digits_body<false, false, LW>(a, job, (const double *)smem, s_e, lt, lane0);
+    if (J.deriv) digits_body<true, false, LW>(a, job, (double *)smem, s_e, lt, lane0);
+    else digits_body<false, false, LW>(a, job, (double *)smem, s_e, lt, lane0);
 }
 
 // Real rows.  PROD: the rows are sums of products of physical rows in tiles [k][128 lanes] (the
 // nonlinear term: sum over i of phys[i] * phys[J.deriv + i], times scale); else they come from a
 // field's rows.
 template <int LW, bool PROD>
-__global__ void __launch_bounds__(kDigThreads, 3) k_digits_real(DigArgs a, const double *phys, size_t fstride, double scale) {
+__global__ void __launch_bounds__(kDigThreads, 4) k_digits_real(DigArgs a, const double *phys, size_t fstride, double scale) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ int s_e[LW];
     const TcShape &s = a.s;
@@ -576,7 +575,7 @@ struct Epi {
 // until the same thread has B.  The MMAs (operand reads from shared memory: (128 + nc) * 32 bytes each) and the
 // integer work of the epilogue bound it.
 struct Unit {
-    int job, par, chunk;
+    int job, par, chunk, cols;  // cols: outputs of the chunk that exist
     unsigned lt;
 };
 template <int MODE>
@@ -588,6 +587,7 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
         u /= 2;
     }
     w.chunk = u % a.nchunk;
+    w.cols = min(a.nc, a.nq[MODE == kC2R ? 0 : w.par] - w.chunk * a.nc);
     u /= a.nchunk;
     w.lt = u % a.ntile;
     w.job = u / a.ntile;
@@ -661,11 +661,12 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
         }
     } else if (warp == kMmaWarp) {
         // D FP32, A and B bf16, both K-major, N = nc, M = 128
-        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nc >> 3) << 17) | (8u << 24);
+        const unsigned idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
         const unsigned lead = elect_one();
         int st = 0, ph = 0, lists = 0;
         bool ok = true;
-        for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x)
+        for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
+            const unsigned idesc = idesc0 | ((unsigned)((unit_of<MODE>(a, u).cols + 15) / 16 * 2) << 17);  // N / 8
             for (int list = 0; list < nit && ok; list += a.ks, lists++) {
                 if (lists) {  // the previous list's sums have left tensor memory
                     ok = __all_sync(~0u, mbar_wait(accempty, (lists - 1) & 1, ab));
@@ -693,9 +694,10 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
                     if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
             }
+        }
     } else {
         // a warp holds a quarter of the lanes and every kEpiQ-th group of 4 outputs
-        const int quad = warp & 3, g0 = warp >> 2, ngr = (nc / 4 - g0 + kEpiQ - 1) / kEpiQ;
+        const int quad = warp & 3, g0 = warp >> 2;
         const int r = quad * 32 + lane;
         const unsigned taddr = tmem + ((unsigned)(quad * 32) << 16);
         long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;  // [nc][128]
@@ -717,6 +719,8 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
         for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
             const Unit w = unit_of<MODE>(a, u);
             const TcJob &J = a.job[w.job];
+            // this warp's groups (at least one: what it reads beyond the outputs is not stored)
+            const int ngr = max(1, ((w.cols + 3) / 4 - g0 + kEpiQ - 1) / kEpiQ);
             bool live;
             size_t off;  // of this lane's column or row in the output
             if (MODE == kCol) {
