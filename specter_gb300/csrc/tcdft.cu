@@ -186,7 +186,7 @@ __device__ __forceinline__ size_t col_offset(const TcShape &s, unsigned c) {
 // 2^kSh, rounded) is an integer that an addition of 1.5 * 2^23 leaves in the low mantissa bits while it
 // is below 2^22, as sums of signed digits nearly always are; level 0 goes up to 2^24 and hands what is
 // below its multiples of 4 down to level 1.  False where a level was too large.  (Conversion instructions
-// would run at 16 a clock: 4400 clocks a list against 2500.)
+// would run at 16 a clock: six a value are 3800 clocks a list of 80 outputs, as long as a product of n = 256.)
 __device__ __forceinline__ bool join_levels(const unsigned (&l)[kLev][4], long long (&u)[4]) {
     constexpr unsigned kB4 = 0x4C400000u, kB = 0x4B400000u;  // 1.5 * 2^25, 1.5 * 2^23
     constexpr unsigned long long kOff = ((unsigned long long)kB4 << (kSh + 2)) + ((unsigned long long)kB << (kSh - 9)) +
@@ -243,8 +243,8 @@ __device__ __forceinline__ double scaled_double(long long t, int q) {
     const int lz = __clz((int)(uh ? uh : ul)) + (uh ? 0 : 32);
     const unsigned long long mant = ((u << (lz - 1)) + 0x200) >> 10;
     const unsigned hi = (unsigned)(mant >> 32) + ((unsigned)(1085 + q - lz) << 20);
-    const double v = __hiloint2double((int)(hi | ((unsigned)(sg >> 32) & 0x80000000u)), (int)(unsigned)mant);
-    return u ? v : 0.0;
+    // zero has a zero mantissa: its exponent goes as well
+    return __hiloint2double((int)(lz == 64 ? 0u : hi | ((unsigned)(sg >> 32) & 0x80000000u)), (int)(unsigned)mant);
 }
 
 // ------------------------------------------------------------------ digits
@@ -553,17 +553,14 @@ struct GemmArgs {
     int *err;
 };
 
-// Epilogue warps per quarter of the lanes.  Three leave 128 registers a thread (512^2 x 538 z transform:
-// 1.21 ms; four: 1.32 ms, two: 1.45 ms); half spectra wait for their even frequencies' integers from L2,
-// which a fourth hides (x_inverse of the same field: 1.45 against 1.79 ms).
-template <int MODE>
-struct Epi {
-    static constexpr int kQ = MODE == kC2R ? 4 : 3;
-    static constexpr int kThreads = 128 * kQ;
-    static constexpr int kLoadWarp = kThreads / 32, kMmaWarp = kLoadWarp + 1;
-    static constexpr int kBlock = kThreads + 64;
-    static constexpr int kGroups = (kMaxNc / 4 + kQ - 1) / kQ;  // groups of 4 outputs per epilogue warp
-};
+// Epilogue warps per quarter of the lanes: the more there are, the better they hide one another's latencies,
+// until the registers of a thread (80 with five) no longer hold its sine products.  z transform of 512^2 x 538
+// and half spectra to rows of 512 x 512 x 538, ms, with three, four, five, six, seven:
+// 1.15 1.13 1.10 1.13 1.13 and 1.03 1.13 0.97 1.03 1.00.
+constexpr int kEpiQ = 5;
+constexpr int kEpiThreads = 128 * kEpiQ, kLoadWarp = kEpiThreads / 32, kMmaWarp = kLoadWarp + 1;
+constexpr int kGemmBlock = kEpiThreads + 64;
+constexpr int kGroups = (kMaxNc / 4 + kEpiQ - 1) / kEpiQ;  // groups of 4 outputs per epilogue warp
 
 // A unit of work: one tile of 64 columns, one parity of the frequency, one chunk of nc outputs.  The
 // data digits are the M = 128 rows (64 columns x real, imaginary), the matrix digits the N = nc columns
@@ -594,10 +591,9 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
     return w;
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
-    constexpr int kLoadWarp = Epi<MODE>::kLoadWarp, kMmaWarp = Epi<MODE>::kMmaWarp, kEpiQ = Epi<MODE>::kQ,
-                  kGroups = Epi<MODE>::kGroups;
+// ADD: jobs may have a field to add (each value's branch costs 5 to 12 %, so launches without one do without).
+template <int MODE, bool ADD>
+__global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned long long bars[2 * 8 + 2];
     __shared__ unsigned s_tmem;
@@ -616,7 +612,7 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
             mbar_init(empty + 8 * i, 1);
         }
         mbar_init(accfull, 1);
-        mbar_init(accempty, Epi<MODE>::kThreads);
+        mbar_init(accempty, kEpiThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -662,12 +658,15 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
     } else if (warp == kMmaWarp) {
         // D FP32, A and B bf16, both K-major, N = nc, M = 128
         const unsigned idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
+        // sine lists of forward transforms with A negated (bit 13)
+        const unsigned neg = MODE == kR2C || (MODE == kCol && s.sign < 0) ? 1u << 13 : 0u;
         const unsigned lead = elect_one();
         int st = 0, ph = 0, lists = 0;
         bool ok = true;
         for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
             const unsigned idesc = idesc0 | ((unsigned)((unit_of<MODE>(a, u).cols + 15) / 16 * 2) << 17);  // N / 8
             for (int list = 0; list < nit && ok; list += a.ks, lists++) {
+                const unsigned id = idesc | (lists & 1 ? neg : 0u);
                 if (lists) {  // the previous list's sums have left tensor memory
                     ok = __all_sync(~0u, mbar_wait(accempty, (lists - 1) & 1, ab));
                     if (!ok) break;
@@ -686,7 +685,7 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
 #pragma unroll
                         for (int j = 0; j < kDig - d; j++) {
                             const int acc = d + j < kLev ? d + j : kLev - 1;
-                            mma_bf16(tmem + acc * nc, da + d * (kLanes * 2), db + j * (nc * 2), idesc,
+                            mma_bf16(tmem + acc * nc, da + d * (kLanes * 2), db + j * (nc * 2), id,
                                      d == 0 && j < kLev ? keep : 1u, lead);
                         }
                     mma_commit(empty + 8 * st, lead);
@@ -700,7 +699,9 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
         const int quad = warp & 3, g0 = warp >> 2;
         const int r = quad * 32 + lane;
         const unsigned taddr = tmem + ((unsigned)(quad * 32) << 16);
-        long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;  // [nc][128]
+        // [nc][128], and at least 4 kEpiQ outputs: every warp's first group has a place.  (Tensor memory has it
+        // too: 5 nc + 4 kEpiQ columns are fewer than 6 nc, or than the 128 of nc = 16.)
+        long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;
         // the levels of 4 outputs, and those as integers
         auto fetch = [&](int gi, unsigned (&l)[kLev][4]) {
             const unsigned at = taddr + (g0 + kEpiQ * gi) * 4;
@@ -736,30 +737,29 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
             // numbers' a further power of two, times the job's own factor; NaN for a non-finite column
             const int q = e - 1022 - 14 - kSh + J.expo, qc = max(-1000, min(q, 900));
             const double fac = e >= kNaN ? __longlong_as_double(0x7ff8000000000000ll) : scalbn(J.post, q - qc);
-            const bool mul = __any_sync(~0u, !(fac == 1.0));
+            const bool more = __any_sync(~0u, !(fac == 1.0));
             double *out = (double *)J.out + off;
-            const double *add = MODE == kCol && J.add ? (const double *)J.add + off : nullptr;
-            auto value = [&](long long t) {
-                double v = scaled_double(t, qc);
-                // kept behind the branch: a multiplication of every value would bind the loop to the FP64 pipe
-                if (mul) asm volatile("mul.rn.f64 %0, %0, %1;" : "+d"(v) : "d"(fac));
-                return v;
+            auto value = [&](long long t) { return scaled_double(t, qc); };
+            const double *add = ADD && J.add ? (const double *)J.add + off : nullptr;  // may be the output itself
+            auto plus = [&](double v, double b) {
+                // behind a branch: a multiplication of every value would bind the loop to the FP64 pipe
+                if (more) asm volatile("mul.rn.f64 %0, %0, %1;" : "+d"(v) : "d"(fac));
+                return v + b;
             };
             for (int par = w.par; par < (MODE == kC2R ? 2 : w.par + 1); par++) {
+                __syncwarp();  // lanes without a column skip the output below
                 ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
                 if (!ok) break;
                 lists++;
                 fence_after();
-                // the next group's loads are in flight while a group is put together
-                unsigned l[2][kLev][4];
-                fetch(0, l[0]);
+                unsigned l[kLev][4];
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
                     if (gi < ngr) {
-                        tmem_wait(l[gi & 1]);
-                        if (gi + 1 < ngr) fetch(gi + 1, l[(gi + 1) & 1]);
+                        fetch(gi, l);
+                        tmem_wait(l);
                         long long P[4];
-                        gather(gi, l[gi & 1], P);
+                        gather(gi, l, P);
 #pragma unroll
                         for (int t = 0; t < 4; t++) Ps[((g0 + kEpiQ * gi) * 4 + t) * kLanes] = P[t];
                     }
@@ -773,9 +773,9 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
                     if (gi < ngr) {
-                        fetch(gi, l[0]);
-                        tmem_wait(l[0]);
-                        gather(gi, l[0], Q[gi]);
+                        fetch(gi, l);
+                        tmem_wait(l);
+                        gather(gi, l, Q[gi]);
                     }
                 fence_before();
                 mbar_arrive(accempty);
@@ -796,26 +796,25 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
                             unsigned o = (unsigned)f0 * s.rs, o2 = (unsigned)(s.n - f0) * s.rs;
 #pragma unroll
                             for (int t = 0; t < 4; t++) {
-                                const long long d = s.sign > 0 ? Q[gi][t] : -Q[gi][t];
-                                v[t] = value(p[t] + d);
-                                v2[t] = value(p[t] - d);
+                                v[t] = value(p[t] + Q[gi][t]);
+                                v2[t] = value(p[t] - Q[gi][t]);
                             }
 #pragma unroll
                             for (int t = 0; t < 4; t++, o += 2 * s.rs, o2 -= 2 * s.rs) {
                                 const int f = f0 + 2 * t, f2 = s.n - f;
                                 if (t < left && f < s.nrows) {
-                                    if (add) v[t] += add[2 * (size_t)o];
+                                    if (ADD && add) v[t] = plus(v[t], add[2 * (size_t)o]);
                                     out[2 * (size_t)o] = v[t];
                                 }
                                 if (t < left && f && f != f2 && f2 < s.nrows) {
-                                    if (add) v2[t] += add[2 * (size_t)o2];
+                                    if (ADD && add) v2[t] = plus(v2[t], add[2 * (size_t)o2]);
                                     out[2 * (size_t)o2] = v2[t];
                                 }
                             }
                         } else if (MODE == kR2C) {
                             double2 v[4];
 #pragma unroll
-                            for (int t = 0; t < 4; t++) v[t] = make_double2(value(p[t]), value(-Q[gi][t]));
+                            for (int t = 0; t < 4; t++) v[t] = make_double2(value(p[t]), value(Q[gi][t]));
 #pragma unroll
                             for (int t = 0; t < 4; t++) {
                                 const int f = 2 * (j0 + t) + par;
@@ -860,6 +859,33 @@ __global__ void __launch_bounds__(Epi<MODE>::kBlock, 1) k_gemm(GemmArgs a) {
                             }
                         }
                     }
+                if (more && !(ADD && add) && (MODE != kC2R || par == 1)) {
+                    // a factor that is no power of two, results beyond the normal numbers, non-finite columns: in a
+                    // pass of its own over this thread's outputs (a branch at each value costs every launch 5 to 12 %)
+                    auto finish = [&](size_t o) { out[o] *= fac; };
+                    for (int gi = 0; gi < ngr; gi++)
+#pragma unroll
+                        for (int t = 0; t < 4; t++) {
+                            const int j = w.chunk * nc + (g0 + kEpiQ * gi) * 4 + t, f = 2 * j + par, f2 = s.n - f;
+                            if (j >= a.nq[MODE == kC2R ? 0 : par]) break;
+                            if (MODE == kCol) {
+                                if (f < s.nrows) finish(2 * ((size_t)f * s.rs));
+                                if (f && f != f2 && f2 < s.nrows) finish(2 * ((size_t)f2 * s.rs));
+                            } else if (MODE == kR2C) {
+                                if (f <= a.m) {
+                                    finish(2 * f);
+                                    finish(2 * f + 1);
+                                }
+                            } else {
+                                finish((size_t)j * s.rs);
+                                finish((size_t)(a.m + j) * s.rs);
+                                if (j && 2 * j != a.m) {
+                                    finish((size_t)(a.m - j) * s.rs);
+                                    finish((size_t)(2 * a.m - j) * s.rs);
+                                }
+                            }
+                        }
+                }
             }
         }
     }
@@ -1134,12 +1160,15 @@ int digit_split(const Dims &D, int lw, size_t blocks) {
 
 template <int MODE>
 void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
-    const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)D.nc * kLanes * 8;
+    const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)std::max(D.nc, 4 * kEpiQ) * kLanes * 8;
     g.nstage = std::min(8, (int)((226 * 1024 - psize) / stage));
     g.units = g.ntile * (MODE == kC2R ? 1 : 2) * D.nchunk * nj;
     const size_t smem = (size_t)g.nstage * stage + psize;
-    cudaFuncSetAttribute(k_gemm<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_gemm<MODE><<<std::min(g.units, 152u), Epi<MODE>::kBlock, smem, P.stream>>>(g);
+    bool add = false;
+    for (int j = 0; j < nj; j++) add = add || g.job[j].add;
+    const auto k = MODE == kCol && add ? k_gemm<MODE, MODE == kCol> : k_gemm<MODE, false>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k<<<std::min(g.units, 152u), kGemmBlock, smem, P.stream>>>(g);
 }
 
 template <typename K>
