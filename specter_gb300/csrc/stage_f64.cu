@@ -8,6 +8,7 @@
 // rotbouss_rkstep2.f90, vboundary.f90:67-151, boundary_mod.fpp:197-402).  The elementwise kernels are
 // bound by the FP64 pipe (about 25 operations a point each), so factors that the components share are
 // formed once a point.
+#include "chain.h"
 #include "fast.h"
 #include "kernels_elem.cuh"
 #include "stage_f64.h"
@@ -38,6 +39,7 @@ struct UpdateArgs {
     int nc, rot;
 };
 __global__ void __launch_bounds__(256) k_stage_update(Geo g, UpdateArgs a) {
+    chain_wait();
     SG_ELEMS_BEGIN(g, 0, g.nz)
         const double kxv = g.kx[kx], kyv = g.ky[ky], kzv = g.kz[z];
         const double k2 = kxv * kxv + kyv * kyv + kzv * kzv;
@@ -67,6 +69,7 @@ __global__ void __launch_bounds__(256) k_stage_update(Geo g, UpdateArgs a) {
 // no-slip walls of vx, vy from the previous pressure (k_noslip) and theta = 0 at the walls
 __global__ void __launch_bounds__(64) k_stage_walls(Geo g, double2 *vx, double2 *vy, double2 *th, const double2 *pr, double tmp,
                                                     WallVel vb) {
+    chain_wait();
     const int kx = blockIdx.x * blockDim.x + threadIdx.x, ky = blockIdx.y;
     if (kx >= g.nxh) return;
     for (int w = 0; w < 2; w++) {
@@ -92,6 +95,7 @@ __global__ void __launch_bounds__(32 * kSlices) k_stage_poisson(Geo g, double2 *
     __shared__ double4 red[kSlices][32];
     const int kx = blockIdx.x * 32 + threadIdx.x, ky = blockIdx.y;
     const bool on = kx < g.nxh;
+    chain_wait();
     double4 w = make_double4(0, 0, 0, 0);
     if (on) {
         const double kxv = g.kx[kx], kyv = g.ky[ky], kh2 = kxv * kxv + kyv * kyv, fxy = th ? g.fx[kx] * g.fy[ky] : 0.0;
@@ -159,6 +163,7 @@ __global__ void __launch_bounds__(256) k_stage_profile(Geo g, const double2 *coe
         tab[t * 32 + c] = exp(-(kh * z));
     }
     __syncthreads();
+    chain_wait();
     if (!on) return;
     const double2 c1 = coef[2 * col], c2 = coef[2 * col + 1];
     auto ex = [&](int z) { return tab[(z % kProfJ) * 32 + c] * tab[(kProfJ + z / kProfJ) * 32 + c]; };
@@ -187,9 +192,10 @@ __global__ void __launch_bounds__(256) k_stage_profile(Geo g, const double2 *coe
 // b = kh (c1 E1 - c2 E2), vx -= i kx p, vy -= i ky p, vz -= b (boundary_mod.fpp:385-399, :635-675)
 __global__ void __launch_bounds__(256) k_stage_correct(Geo g, double2 *vx, double2 *vy, double2 *vz, const double2 *E1,
                                                        const double2 *E2, const double2 *coef) {
+    chain_wait();
     SG_ELEMS_BEGIN(g, 0, g.nz)
         const size_t col = (size_t)ky * g.nxh + kx;
-        const double2 c1 = __ldg(coef + 2 * col), c2 = __ldg(coef + 2 * col + 1);
+        const double2 c1 = coef[2 * col], c2 = coef[2 * col + 1];
         double2 p, b;
         if (kx == 0 && ky == 0) {  // profile c1.x z, its derivative c1.x (E2 is the spectrum of 1)
             const double2 e1 = E1[q], e2 = E2[q];
@@ -208,6 +214,7 @@ __global__ void __launch_bounds__(256) k_stage_correct(Geo g, double2 *vx, doubl
 
 // theta's c2r / r2c round trip leaves the kx = 0 and kx = nx/2 columns Hermitian over (ky, -ky)
 __global__ void __launch_bounds__(128) k_stage_herm(Geo g, double2 *th) {
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, sel = blockIdx.y;
     const int h = g.ny / 2 + 1;
     if (i >= h * g.nzp) return;
@@ -231,7 +238,7 @@ bool f64_stage_ok(const Plan &P) { return tc_length_ok(P.nz); }
 int f64_poisson(Plan &P, void *vx, void *vy, void *vz, void *d, void *th, double2 *coef) {
     const double field = (double)P.nz * P.ny * P.nxh * 16.0;
     Launch L(P, "stage_poisson", (7.0 + (th ? 2.0 : 0.0)) * field);
-    k_stage_poisson<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, kSlices), 0, P.stream>>>(
+    chain(k_stage_poisson, dim3(cdiv(P.nxh, 32), P.ny), dim3(32, kSlices), 0, P.stream, 
         P.geo, (double2 *)vx, (double2 *)vy, (double2 *)vz, (double2 *)d, (double2 *)th, coef);
     return check_launch("poisson");
 }
@@ -240,7 +247,7 @@ int f64_profile(Plan &P, const double2 *coef, void *prof, void *deriv) {
     Launch L(P, "stage_profile", (deriv ? 2.0 * P.nz : (double)P.nzp) * P.ny * P.nxh * 16.0);
     const size_t sm = (size_t)(kProfJ + cdiv(P.nzp, kProfJ)) * 32 * sizeof(double);
     if (sm > 40 * 1024) cudaFuncSetAttribute(k_stage_profile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_stage_profile<<<dim3(cdiv(P.nxh, 32), P.ny), dim3(32, 8), sm, P.stream>>>(P.geo, coef, (double2 *)prof, (double2 *)deriv, P.dz);
+    chain(k_stage_profile, dim3(cdiv(P.nxh, 32), P.ny), dim3(32, 8), sm, P.stream, P.geo, coef, (double2 *)prof, (double2 *)deriv, P.dz);
     return check_launch("profile");
 }
 
@@ -276,7 +283,7 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
         a.nc = nc;
         a.rot = rot;
         Launch L(P, "stage_update", 4.0 * nc * field);
-        k_stage_update<<<elem_blocks(P), 256, 0, P.stream>>>(P.geo, a);
+        chain(k_stage_update, elem_blocks(P), 256, 0, P.stream, P.geo, a);
     }
     // wall round trips of vx, vy (no slip) and theta (zero walls): rows above nzp are rebuilt by the
     // continuation
@@ -309,7 +316,7 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
     {
         const WallVel vb{sp.vzsta[0], sp.vzsta[1], sp.vzend[0], sp.vzend[1]};
         Launch L(P, "walls", 8.0 * P.ny * P.nxh * 16.0);
-        k_stage_walls<<<dim3(cdiv(P.nxh, 64), P.ny), 64, 0, P.stream>>>(P.geo, x, y, bouss ? th : nullptr, (const double2 *)pr, tmp, vb);
+        chain(k_stage_walls, dim3(cdiv(P.nxh, 64), P.ny), 64, 0, P.stream, P.geo, x, y, bouss ? th : nullptr, (const double2 *)pr, tmp, vb);
     }
     SG_TRY(forward(trip, nt));
     const bool trip2 = bouss && !rot;
@@ -322,12 +329,12 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
     }
     {
         Launch L(P, "stage_correct", 8.0 * field);
-        k_stage_correct<<<elem_blocks(P), 256, 0, P.stream>>>(P.geo, x, y, w, (const double2 *)E[0], (const double2 *)E[1], coef);
+        chain(k_stage_correct, elem_blocks(P), 256, 0, P.stream, P.geo, x, y, w, (const double2 *)E[0], (const double2 *)E[1], coef);
     }
     if (trip2) {
         {
             Launch L(P, "theta_herm", 4.0 * P.ny * P.nzp * 16.0);
-            k_stage_herm<<<dim3(cdiv((P.ny / 2 + 1) * P.nzp, 128), 2), 128, 0, P.stream>>>(P.geo, th);
+            chain(k_stage_herm, dim3(cdiv((P.ny / 2 + 1) * P.nzp, 128), 2), 128, 0, P.stream, P.geo, th);
         }
         void *f[1] = {th};
         SG_TRY(forward(f, 1));

@@ -23,6 +23,7 @@
 
 #include <cuda_bf16.h>
 
+#include "chain.h"
 #include "fast.h"
 #include "ops.h"
 #include "tcdft.h"
@@ -403,6 +404,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) k_digits(DigArgs a) {
     const int lane0 = (blockIdx.x % kParts) * LW;
     const int n0 = s.n - s.next;  // rows below n0 come from the field, the others from the continuation
     if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
+    chain_wait();
     {
         const int cc = threadIdx.x % kCols;
         const unsigned c = (a.tile0 + lt) * 64 + lane0 / 2 + cc;
@@ -446,6 +448,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) k_digits_real(DigArgs a, const
     const unsigned lt = blockIdx.x / kParts;
     const int lane0 = (blockIdx.x % kParts) * LW;
     if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
+    chain_wait();
     double *dst = (double *)smem;
     if (PROD) {
         const int l = threadIdx.x % LW;
@@ -465,7 +468,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) k_digits_real(DigArgs a, const
         const bool live = row < s.ncol;
         const double *in = (const double *)J.in + (live ? (size_t)row * s.n : 0);
 #pragma unroll 4
-        for (int k = threadIdx.x / LW; k < s.n; k += kDigThreads / LW) dst[k * LW + l] = live ? __ldg(in + k) : 0.0;
+        for (int k = threadIdx.x / LW; k < s.n; k += kDigThreads / LW) dst[k * LW + l] = live ? in[k] : 0.0;
     }
     __syncthreads();
     digits_body<false, true, LW>(a, job, dst, s_e, lt, lane0);
@@ -529,6 +532,7 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits_half(DigArgs a) {
     const int lane0 = (blockIdx.x % kParts) * LW;
     const unsigned r0 = (a.tile0 + lt) * kLanes + lane0;
     if (threadIdx.x < LW) s_e[threadIdx.x] = 0;
+    chain_wait();
     double2 *dst = (double2 *)smem;  // [frequency][LW + 1]: the odd stride keeps the row writes off one bank
     for (int i = threadIdx.x; i < H * LW; i += kDigThreads) {
         const int l = i / H, f = i - l * H;
@@ -623,6 +627,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
     fence_before();
     __syncthreads();
     fence_after();
+    chain_wait();
     const unsigned tmem = s_tmem;
     volatile int *ab = &s_abort;
     const int nit = (MODE == kC2R ? 4 : 2) * a.ks;  // steps of a unit: cosine list, sine list (of each parity)
@@ -908,6 +913,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
 // physical rows from tiles [tile][x][128 rows] to a field [row][x]
 __global__ void __launch_bounds__(256) k_untile(const double *tiles, double *out, int n, unsigned rows) {
     __shared__ double t[32][33];
+    chain_wait();
     const unsigned r0 = blockIdx.x * 32, x0 = blockIdx.y * 32;
     const double *src = tiles + (size_t)(r0 / kLanes) * n * kLanes + r0 % kLanes;
     for (unsigned i = threadIdx.y; i < 32; i += 8)
@@ -1168,7 +1174,8 @@ void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     for (int j = 0; j < nj; j++) add = add || g.job[j].add;
     const auto k = MODE == kCol && add ? k_gemm<MODE, MODE == kCol> : k_gemm<MODE, false>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<std::min(g.units, 152u), kGemmBlock, smem, P.stream>>>(g);
+    if (g.units <= 152) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
+    else k<<<152, kGemmBlock, smem, P.stream>>>(g);
 }
 
 template <typename K>
@@ -1203,7 +1210,7 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
             const double share = (double)nt * jstep / ((double)tiles * njobs);
             {
                 Launch L(P, "digits", share * bytes * 0.5 + (double)nt * jstep * per);
-                with_smem(lw == 32 ? k_digits<32> : k_digits<16>, dsm)<<<grid, kDigThreads, dsm, P.stream>>>(d);
+                chain(with_smem(lw == 32 ? k_digits<32> : k_digits<16>, dsm), grid, kDigThreads, dsm, P.stream, d);
             }
             {
                 Launch L(P, name, share * bytes);
@@ -1280,8 +1287,8 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
         {
             const size_t sm = (size_t)(D.m + 1) * (lw + 1) * sizeof(double2);
             Launch L(P, "digits", share * nin / (nin + nc) + (double)nt * nin * per);
-            with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm)
-                <<<dim3((unsigned)blocks, digit_split(D, lw, blocks * nin), nin), kDigThreads, sm, P.stream>>>(d);
+            chain(with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm),
+                  dim3((unsigned)blocks, digit_split(D, lw, blocks * nin), nin), kDigThreads, sm, P.stream, d);
         }
         g.s.rs = kLanes;
         g.s.ls = 1;
@@ -1305,9 +1312,9 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
         {
             const size_t sm = (size_t)n * lw * sizeof(double);
             Launch L(P, "products", (double)nt * (nin * ptile * 8.0 + nc * per));
-            with_smem(lw == 32 ? k_digits_real<32, true> : k_digits_real<16, true>, sm)
-                <<<dim3((unsigned)blocks, digit_split(D, lw, blocks * nc), nc), kDigThreads, sm, P.stream>>>(
-                    d2, S->phys, fstride, scale);
+            chain(with_smem(lw == 32 ? k_digits_real<32, true> : k_digits_real<16, true>, sm),
+                  dim3((unsigned)blocks, digit_split(D, lw, blocks * nc), nc), kDigThreads, sm, P.stream, d2, S->phys, fstride,
+                  scale);
         }
         {
             Launch L(P, "x_forward", share * nc / (nin + nc) + (double)nt * nc * per);
@@ -1409,11 +1416,11 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
                 Launch L(P, "digits", share * 0.5 + (double)nt * per);
                 if (r2c) {
                     const size_t sm = (size_t)P.nx * lw * sizeof(double);
-                    with_smem(lw == 32 ? k_digits_real<32, false> : k_digits_real<16, false>, sm)
-                        <<<grid, kDigThreads, sm, P.stream>>>(d, nullptr, 0, 1.0);
+                    chain(with_smem(lw == 32 ? k_digits_real<32, false> : k_digits_real<16, false>, sm), grid, kDigThreads, sm,
+                          P.stream, d, nullptr, 0, 1.0);
                 } else {
                     const size_t sm = (size_t)(D.m + 1) * (lw + 1) * sizeof(double2);
-                    with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm)<<<grid, kDigThreads, sm, P.stream>>>(d);
+                    chain(with_smem(lw == 32 ? k_digits_half<32> : k_digits_half<16>, sm), grid, kDigThreads, sm, P.stream, d);
                 }
             }
             g.s.rs = r2c ? 1 : kLanes;
@@ -1425,8 +1432,7 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
             if (!r2c) {
                 const unsigned left = std::min(rows - t0 * kLanes, nt * kLanes);
                 Launch L(P, "untile", 16.0 * left * P.nx);
-                k_untile<<<dim3((left + 31) / 32, (P.nx + 31) / 32), dim3(32, 8), 0, P.stream>>>(
-                    S->phys, (double *)a.out[f] + (size_t)t0 * kLanes * P.nx, P.nx, left);
+                chain(k_untile, dim3((left + 31) / 32, (P.nx + 31) / 32), dim3(32, 8), 0, P.stream, S->phys, (double *)a.out[f] + (size_t)t0 * kLanes * P.nx, P.nx, left);
             }
         }
     return check_launch(name);
