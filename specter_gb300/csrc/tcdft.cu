@@ -596,27 +596,33 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
 }
 
 // ADD: jobs may have a field to add (each value's branch costs 5 to 12 %, so launches without one do without).
-template <int MODE, bool ADD>
+// NACC: sets of accumulators in tensor memory, used by the lists in turn.  With two, a list's MMAs run while
+// the sums of the one before are read; lengths below 128 leave room for it (2 * kLev * 32 columns), and their
+// lists are as short as that read: half spectra to rows of 96 x 96 x 122, 91 -> 80 us, of 64 x 64 x 90, 45 -> 40 us.
+// (As a run-time choice it costs longer lengths 5 to 14 %.)
+template <int MODE, bool ADD, int NACC>
 __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ unsigned long long bars[2 * 8 + 2];
+    __shared__ unsigned long long bars[2 * 8 + 4];
     __shared__ unsigned s_tmem;
     __shared__ int s_abort;
     const TcShape &s = a.s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nc = a.nc;
     const unsigned b_bytes = kDig * nc * 32, stage_bytes = kAStage + b_bytes;
-    const unsigned full = smem_u32(bars), empty = full + 8 * 8, accfull = full + 16 * 8, accempty = accfull + 8;
+    const unsigned full = smem_u32(bars), empty = full + 8 * 8, accfull = full + 16 * 8, accempty = accfull + 16;
     unsigned tcols = 32;
-    while (tcols < (unsigned)(kLev * nc)) tcols *= 2;
+    while (tcols < (unsigned)(NACC * kLev * nc)) tcols *= 2;
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int i = 0; i < a.nstage; i++) {
             mbar_init(full + 8 * i, 1);
             mbar_init(empty + 8 * i, 1);
         }
-        mbar_init(accfull, 1);
-        mbar_init(accempty, kEpiThreads);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(accfull + 8 * i, 1);
+            mbar_init(accempty + 8 * i, kEpiThreads);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -672,11 +678,13 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
             const unsigned idesc = idesc0 | ((unsigned)((unit_of<MODE>(a, u).cols + 15) / 16 * 2) << 17);  // N / 8
             for (int list = 0; list < nit && ok; list += a.ks, lists++) {
                 const unsigned id = idesc | (lists & 1 ? neg : 0u);
-                if (lists) {  // the previous list's sums have left tensor memory
-                    ok = __all_sync(~0u, mbar_wait(accempty, (lists - 1) & 1, ab));
+                const int set = lists % NACC;
+                if (lists >= NACC) {  // the set's previous sums have left tensor memory
+                    ok = __all_sync(~0u, mbar_wait(accempty + 8 * set, ((lists / NACC) - 1) & 1, ab));
                     if (!ok) break;
                     fence_after();
                 }
+                const unsigned tm = tmem + set * kLev * nc;
                 for (int i = 0; i < a.ks; i++) {
                     ok = __all_sync(~0u, mbar_wait(full + 8 * st, ph, ab));
                     if (!ok) break;
@@ -690,11 +698,11 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
 #pragma unroll
                         for (int j = 0; j < kDig - d; j++) {
                             const int acc = d + j < kLev ? d + j : kLev - 1;
-                            mma_bf16(tmem + acc * nc, da + d * (kLanes * 2), db + j * (nc * 2), id,
+                            mma_bf16(tm + acc * nc, da + d * (kLanes * 2), db + j * (nc * 2), id,
                                      d == 0 && j < kLev ? keep : 1u, lead);
                         }
                     mma_commit(empty + 8 * st, lead);
-                    if (i == a.ks - 1) mma_commit(accfull, lead);
+                    if (i == a.ks - 1) mma_commit(accfull + 8 * set, lead);
                     if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
             }
@@ -708,19 +716,32 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
         // too: 5 nc + 4 kEpiQ columns are fewer than 6 nc, or than the 128 of nc = 16.)
         long long *Ps = (long long *)(smem + a.nstage * stage_bytes) + r;
         // the levels of 4 outputs, and those as integers
+        unsigned tset = taddr;  // of the list's set of accumulators
         auto fetch = [&](int gi, unsigned (&l)[kLev][4]) {
-            const unsigned at = taddr + (g0 + kEpiQ * gi) * 4;
+            const unsigned at = tset + (g0 + kEpiQ * gi) * 4;
 #pragma unroll
             for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
         };
         auto gather = [&](int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
             if (__any_sync(~0u, !join_levels(l, u))) {
-                const Four w = join_levels_wide(taddr + (g0 + kEpiQ * gi) * 4, nc);
+                const Four w = join_levels_wide(tset + (g0 + kEpiQ * gi) * 4, nc);
 #pragma unroll
                 for (int t = 0; t < 4; t++) u[t] = w.u[t];
             }
         };
         int lists = 0;
+        auto take = [&] {  // the next list's sums are there
+            const int set = lists % NACC;
+            tset = taddr + set * kLev * nc;
+            if (!__all_sync(~0u, mbar_wait(accfull + 8 * set, (lists / NACC) & 1, ab))) return false;
+            fence_after();
+            return true;
+        };
+        auto give = [&] {  // and have been read
+            fence_before();
+            mbar_arrive(accempty + 8 * (lists % NACC));
+            lists++;
+        };
         bool ok = true;
         for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
             const Unit w = unit_of<MODE>(a, u);
@@ -753,10 +774,8 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
             };
             for (int par = w.par; par < (MODE == kC2R ? 2 : w.par + 1); par++) {
                 __syncwarp();  // lanes without a column skip the output below
-                ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
+                ok = take();
                 if (!ok) break;
-                lists++;
-                fence_after();
                 unsigned l[kLev][4];
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
@@ -768,12 +787,9 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
 #pragma unroll
                         for (int t = 0; t < 4; t++) Ps[((g0 + kEpiQ * gi) * 4 + t) * kLanes] = P[t];
                     }
-                fence_before();
-                mbar_arrive(accempty);
-                ok = __all_sync(~0u, mbar_wait(accfull, lists & 1, ab));
+                give();
+                ok = take();
                 if (!ok) break;
-                lists++;
-                fence_after();
                 long long Q[kGroups][4];
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
@@ -782,8 +798,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                         tmem_wait(l);
                         gather(gi, l, Q[gi]);
                     }
-                fence_before();
-                mbar_arrive(accempty);
+                give();
                 if (!live) continue;
                 // a group's loads, conversions and stores one after another: loads do not move across stores
 #pragma unroll
@@ -1172,7 +1187,9 @@ void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     const size_t smem = (size_t)g.nstage * stage + psize;
     bool add = false;
     for (int j = 0; j < nj; j++) add = add || g.job[j].add;
-    const auto k = MODE == kCol && add ? k_gemm<MODE, MODE == kCol> : k_gemm<MODE, false>;
+    const bool two = 2 * kLev * D.nc <= 512;
+    const auto k = MODE == kCol && add ? (two ? k_gemm<MODE, MODE == kCol, 2> : k_gemm<MODE, MODE == kCol, 1>)
+                                       : (two ? k_gemm<MODE, false, 2> : k_gemm<MODE, false, 1>);
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (g.units <= 152) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
     else k<<<152, kGemmBlock, smem, P.stream>>>(g);
