@@ -53,17 +53,28 @@ constexpr int kNaN = 0x40000000;    // exponent of a column that holds a non-fin
 // what a launch transforms: complex columns; real rows to half spectra; half spectra to real rows
 enum { kCol = 0, kR2C = 1, kC2R = 2 };
 
+// Steps of 16 values in the four lists: `first` for the cosine list of the even frequencies (K = m/2 + 1
+// values), `rest` for each of the others, one step less where m is a multiple of 32 (they hold m/2 values;
+// 64^3: 5 steps instead of 8, 128^3: 9 of 12, 512^3: 33 of 36).
+struct Steps {
+    int first, rest;
+    __host__ __device__ int of(int list) const { return list ? rest : first; }
+    __host__ __device__ int before(int list) const { return list ? first + (list - 1) * rest : 0; }
+    __host__ __device__ int all() const { return first + 3 * rest; }
+};
 struct Dims {
-    int n, m, K, ks, nq[2], nchunk, nc;
+    int n, m, K, nq[2], nchunk, nc;
+    Steps ks;
 };
 Dims dims(int n) {
     Dims d;
     d.n = n;
     d.m = n / 2;
     d.K = d.m / 2 + 1;
-    d.ks = (d.K + 15) / 16;
     d.nq[0] = d.m / 2 + 1;
     d.nq[1] = (d.m + 1) / 2;
+    d.ks.first = (d.nq[0] + 15) / 16;
+    d.ks.rest = (d.nq[1] + 15) / 16;
     const int np = (d.nq[0] + 15) / 16 * 16;
     d.nchunk = (np + kMaxNc - 1) / kMaxNc;
     d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
@@ -254,7 +265,8 @@ struct DigArgs {
     TcJob job[kTcMaxJobs];
     const double *dir;      // FC-Gram matrix (s.next rows, column-major) and its matching points
     int oz;
-    int m, K, ks;
+    int m, K;
+    Steps ks;
     unsigned tile0, ntile;  // tiles [tile0, tile0 + ntile) of every job
     unsigned char *ws;
     int *expo;              // [job][ntile][128 lanes]
@@ -355,17 +367,17 @@ __device__ __forceinline__ void digits_body(const DigArgs &a, int job, double *t
     for (int row = threadIdx.x / LW; row < n; row += kDigThreads / LW)
         x[row * LW] = fixed_point<DERIV>(xd[row * LW], row < m ? row : row - n, emax);
     __syncthreads();
-    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage;
+    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * a.ks.all() * kAStage;
     // effective part: multiplying by i moves real data to imaginary lanes and imaginary data, negated,
     // to real lanes; so does the sine list of a complex transform
     const int epart = DERIV ? part ^ 1 : part;
     const int row0 = DERIV ? lane ^ 1 : lane, row1 = REAL ? lane : row0 ^ 1;
     const bool flip = DERIV && part == 1;
-    const size_t st = (size_t)a.ks * kAStage;
-    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks; g += gridDim.y * (kDigThreads / LW)) {
+    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks.first; g += gridDim.y * (kDigThreads / LW)) {
         unsigned char *d = tb + (size_t)(g >> 1) * kAStage + (size_t)(g & 1) * kLanes * 16;
+        const bool rest = g < 2 * a.ks.rest;  // else the first list alone goes on
 #pragma unroll 1
-        for (int par = 0; par < 2; par++) {  // even frequencies: x[k] + x[k+m]; odd: x[k] - x[k+m]
+        for (int par = 0; par < (rest ? 2 : 1); par++) {  // even frequencies: x[k] + x[k+m]; odd: x[k] - x[k+m]
             long long c[8], w[8];
 #pragma unroll
             for (int t = 0; t < 8; t++) {
@@ -381,12 +393,17 @@ __device__ __forceinline__ void digits_body(const DigArgs &a, int job, double *t
                 if (par) E2 = -E2;
                 c[t] = E + E2;
                 w[t] = E - E2;
-                if (par ? k == 0 : self) w[t] = 0;
+                if (self) w[t] = 0;
                 if (par && 2 * k == m) c[t] = 0;
                 if (epart == 1) w[t] = -w[t];
             }
-            put_digits(d + 2 * par * st + row0 * 16, c);
-            put_digits(d + (2 * par + 1) * st + row1 * 16, w);
+            // the last of the odd sine list (k = m/2) takes the place of k = 0, which has no sine
+            if (par && g == 0 && m % 2 == 0) {
+                const long long O = x[m / 2 * LW] - x[(m / 2 + m) * LW];
+                w[0] = flip != (epart == 1) ? -O : O;
+            }
+            put_digits(d + (size_t)a.ks.before(2 * par) * kAStage + row0 * 16, c);
+            if (rest) put_digits(d + (size_t)a.ks.before(2 * par + 1) * kAStage + row1 * 16, w);
         }
     }
 }
@@ -493,12 +510,12 @@ __device__ __forceinline__ void half_digits(const DigArgs &a, int job, const dou
     if (emax == 0) emax = 1023;
     if (blockIdx.y == 0 && threadIdx.x < LW) a.expo[((size_t)job * a.ntile + lt) * kLanes + lane] = emax;
     if (emax >= kNaN) emax = 0x7ff;
-    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * 4 * a.ks * kAStage + lane * 16;
-    const size_t st = (size_t)a.ks * kAStage;
-    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks; g += gridDim.y * (kDigThreads / LW)) {
+    unsigned char *tb = a.ws + ((size_t)job * a.ntile + lt) * a.ks.all() * kAStage + lane * 16;
+    for (int g = blockIdx.y * (kDigThreads / LW) + threadIdx.x / LW; g < 2 * a.ks.first; g += gridDim.y * (kDigThreads / LW)) {
         unsigned char *d = tb + (size_t)(g >> 1) * kAStage + (size_t)(g & 1) * kLanes * 16;
+        const bool rest = g < 2 * a.ks.rest;  // else the first list alone goes on
 #pragma unroll 1
-        for (int par = 0; par < 2; par++) {
+        for (int par = 0; par < (rest ? 2 : 1); par++) {
             long long c[8], w[8];
 #pragma unroll
             for (int t = 0; t < 8; t++) {
@@ -514,8 +531,8 @@ __device__ __forceinline__ void half_digits(const DigArgs &a, int job, const dou
                 c[t] = end ? re : 2 * re;
                 w[t] = end ? 0 : 2 * im;
             }
-            put_digits(d + 2 * par * st, c);
-            put_digits(d + (2 * par + 1) * st, w);
+            put_digits(d + (size_t)a.ks.before(2 * par) * kAStage, c);
+            if (rest) put_digits(d + (size_t)a.ks.before(2 * par + 1) * kAStage, w);
         }
     }
 }
@@ -550,7 +567,8 @@ __global__ void __launch_bounds__(kDigThreads, 3) k_digits_half(DigArgs a) {
 struct GemmArgs {
     TcShape s;
     TcJob job[kTcMaxJobs];
-    int m, ks, nq[2], nchunk, nc, nstage;  // m = n / 2
+    int m, nq[2], nchunk, nc, nstage;  // m = n / 2
+    Steps ks;
     unsigned tile0, ntile, units;
     const unsigned char *ws;
     const int *expo;
@@ -636,16 +654,20 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
     chain_wait();
     const unsigned tmem = s_tmem;
     volatile int *ab = &s_abort;
-    const int nit = (MODE == kC2R ? 4 : 2) * a.ks;  // steps of a unit: cosine list, sine list (of each parity)
+    constexpr int kLists = MODE == kC2R ? 4 : 2;  // of a unit: cosine list, sine list (of each parity)
     if (warp == kLoadWarp) {
         if (lane == 0) {
             int it = 0, st = 0, ph = 1;  // steps issued so far, their stage and the phase its buffer is free after
             bool ok = true;
             for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit w = unit_of<MODE>(a, u);
-                const unsigned char *A = a.ws + (((size_t)w.job * a.ntile + w.lt) * 4 + 2 * w.par) * a.ks * kAStage;
-                const unsigned char *B = a.job[w.job].mat + ((size_t)w.par * 2 * a.nchunk + w.chunk) * a.ks * b_bytes;
-                int ks = 0;
+                int list = 2 * w.par, left = a.ks.of(list);
+                const unsigned char *A = a.ws + (((size_t)w.job * a.ntile + w.lt) * a.ks.all() + a.ks.before(list)) * kAStage;
+                auto matrix = [&] {
+                    return a.job[w.job].mat + (size_t)(a.ks.before(list) * a.nchunk + w.chunk * a.ks.of(list)) * b_bytes;
+                };
+                const unsigned char *B = matrix();
+                const int nit = a.ks.before(list + kLists) - a.ks.before(list);
                 for (int i = 0; i < nit; i++, it++) {
                     if (it >= a.nstage && !mbar_wait(empty + 8 * st, ph, ab)) { ok = false; break; }
                     const unsigned dst = smem_u32(smem) + st * stage_bytes;
@@ -653,9 +675,9 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                     bulk_load(dst, A + (size_t)i * kAStage, kAStage, full + 8 * st);
                     bulk_load(dst + kAStage, B, b_bytes, full + 8 * st);
                     B += b_bytes;
-                    if (++ks == a.ks) {  // the next list's matrix of the same chunk
-                        ks = 0;
-                        B += (size_t)(a.nchunk - 1) * a.ks * b_bytes;
+                    if (--left == 0) {  // the next list's matrix of the same chunk
+                        left = a.ks.of(++list);
+                        B = matrix();
                     }
                     if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
@@ -675,8 +697,10 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
         int st = 0, ph = 0, lists = 0;
         bool ok = true;
         for (unsigned u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
-            const unsigned idesc = idesc0 | ((unsigned)((unit_of<MODE>(a, u).cols + 15) / 16 * 2) << 17);  // N / 8
-            for (int list = 0; list < nit && ok; list += a.ks, lists++) {
+            const Unit w = unit_of<MODE>(a, u);
+            const unsigned idesc = idesc0 | ((unsigned)((w.cols + 15) / 16 * 2) << 17);  // N / 8
+            for (int list = 0; list < kLists && ok; list++, lists++) {
+                const int ks = a.ks.of(2 * w.par + list);
                 const unsigned id = idesc | (lists & 1 ? neg : 0u);
                 const int set = lists % NACC;
                 if (lists >= NACC) {  // the set's previous sums have left tensor memory
@@ -685,7 +709,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                     fence_after();
                 }
                 const unsigned tm = tmem + set * kLev * nc;
-                for (int i = 0; i < a.ks; i++) {
+                for (int i = 0; i < ks; i++) {
                     ok = __all_sync(~0u, mbar_wait(full + 8 * st, ph, ab));
                     if (!ok) break;
                     fence_after();
@@ -702,7 +726,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                                      d == 0 && j < kLev ? keep : 1u, lead);
                         }
                     mma_commit(empty + 8 * st, lead);
-                    if (i == a.ks - 1) mma_commit(accfull + 8 * set, lead);
+                    if (i == ks - 1) mma_commit(accfull + 8 * set, lead);
                     if (++st == a.nstage) { st = 0; ph ^= 1; }
                 }
             }
@@ -940,22 +964,22 @@ __global__ void __launch_bounds__(256) k_untile(const double *tiles, double *out
 
 // ------------------------------------------------------------------ tables
 // digits [angle][7] of factor * cos, factor * sin at 2 pi t / n -> the matrices of one set
-__global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, int K, int ks, int nq0, int nq1, int nchunk,
+__global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, int K, Steps ks, int nq0, int nq1, int nchunk,
                            int nc, int half) {
-    const long long total = 4ll * nchunk * ks * 16 * nc;
+    const long long total = (long long)nchunk * ks.all() * 16 * nc;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
-        const int kk = (int)(q % 16), col = (int)(q / 16 % nc);
-        long long t = q / 16 / nc;
-        const int step = (int)(t % ks);
-        t /= ks;
-        const int chunk = (int)(t % nchunk), list = (int)(t / nchunk % 2), par = (int)(t / nchunk / 2);
-        const int k = 16 * step + kk, j = chunk * nc + col;
+        const int kk = (int)(q % 16), col = (int)(q / 16 % nc), t = (int)(q / 16 / nc);  // [list][chunk][step][col][kk]
+        const int set = t < nchunk * ks.first ? 0 : 1 + (t - nchunk * ks.first) / (nchunk * ks.rest);
+        const int r = t - nchunk * ks.before(set), chunk = r / ks.of(set), step = r % ks.of(set);
+        const int list = set % 2, par = set / 2;
+        int k = 16 * step + kk;
+        const int j = chunk * nc + col;
+        if (!half && set == 3 && n % 4 == 0) k = k == 0 ? n / 4 : k == n / 4 ? K : k;  // as the digits have it
         // the K side runs over points and the N side over frequencies, the other way about for half spectra
         const int pt = half ? j : k, fq = half ? k : j;
         const bool on = pt < K && fq < (par ? nq1 : nq0);
         const int ang = on ? (int)((long long)(2 * fq + par) * pt % n) : 0;
-        __nv_bfloat16 *dst = mat + (((long long)(par * 2 + list) * nchunk + chunk) * ks + step) * (kDig * 16 * nc) +
-                             (kk / 8) * (nc * 8) + col * 8 + kk % 8;
+        __nv_bfloat16 *dst = mat + (long long)t * (kDig * 16 * nc) + (kk / 8) * (nc * 8) + col * 8 + kk % 8;
         for (int i = 0; i < kDig; i++)
             dst[(long long)i * nc * 16] = on ? dig[((long long)list * n + ang) * kDig + i] : __float2bfloat16(0.f);
     }
@@ -1077,7 +1101,7 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
             const int i = (int)(q % kDig);
             h[(size_t)l * n * kDig + q] = __float2bfloat16(ldexpf((float)(l ? ds[q] : dc[q]), -9 * i));
         }
-    set.bytes = 4ull * D.nchunk * D.ks * kDig * 32 * D.nc;
+    set.bytes = (size_t)D.nchunk * D.ks.all() * kDig * 32 * D.nc;
     __nv_bfloat16 *dig = nullptr;
     if (cudaMalloc(&set.mat, set.bytes) != cudaSuccess || cudaMalloc(&dig, h.size() * 2) != cudaSuccess) {
         cudaGetLastError();
@@ -1110,7 +1134,7 @@ static int workspace(Plan &P) {
                             ((size_t)P.nz * P.ny + kLanes - 1) / kLanes};
     for (int i = 0; i < 3; i++) {
         if (!tc_length_ok(len[i])) continue;
-        const size_t per = 4ull * dims(len[i]).ks * kAStage;
+        const size_t per = (size_t)dims(len[i]).ks.all() * kAStage;
         size_t t = cols[i] * jobs[i];
         t = std::min(t, std::max<size_t>((2ull << 30) / per, kTcMaxJobs));
         want = std::max(want, t * per);
@@ -1173,7 +1197,7 @@ int digit_lanes(int n) { return n <= 300 ? 32 : 16; }
 // Small launches split a tile's lists over blocks (each reads its columns itself) until there are two
 // blocks per SM.
 int digit_split(const Dims &D, int lw, size_t blocks) {
-    const int rounds = (2 * D.ks * lw + kDigThreads - 1) / kDigThreads;
+    const int rounds = (2 * D.ks.first * lw + kDigThreads - 1) / kDigThreads;
     int split = 1;
     while (split < rounds && blocks * split < 304) split++;
     return split;
@@ -1208,7 +1232,7 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
     if (int st = tc_status(P)) return st;
     TcState *S = P.tc;
     const Dims D = dims(s.n);
-    const size_t per = 4ull * D.ks * kAStage;
+    const size_t per = (size_t)D.ks.all() * kAStage;
     const unsigned tiles = (s.ncol + 63) / 64;
     const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     // all jobs at once when they fit, else job by job in ranges of tiles
@@ -1242,7 +1266,7 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
 static int phys_rows(Plan &P) {
     TcState *S = P.tc;
     if (S->phys) return OK;
-    const size_t per = 4ull * dims(P.nx).ks * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const size_t per = (size_t)dims(P.nx).ks.all() * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const size_t all = ((size_t)P.nzp * P.ny + kLanes - 1) / kLanes, t = std::min(all, std::max<size_t>(cap / kTcMaxJobs, 1));
     if (cudaMalloc(&S->phys, t * 15 * P.nx * kLanes * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
@@ -1272,7 +1296,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
     const TcSet *fwd = dinv ? tc_set(P, n, 1.0, &st, false) : nullptr;
     if (!fwd) return st;
     const Dims D = dims(n);
-    const size_t per = 4ull * D.ks * kAStage, ptile = (size_t)n * kLanes;
+    const size_t per = (size_t)D.ks.all() * kAStage, ptile = (size_t)n * kLanes;
     const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
     SG_TRY(phys_rows(P));
@@ -1405,7 +1429,7 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
     const TcSet *set = tc_set(P, P.nx, a.scale, &st, !r2c);
     if (!set) return st;
     const Dims D = dims(P.nx);
-    const size_t per = 4ull * D.ks * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const size_t per = (size_t)D.ks.all() * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)a.nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
     const unsigned tstep = (unsigned)std::min<size_t>(tiles, r2c ? cap : std::min(cap, 15 * S->phys_tiles));
     const int lw = digit_lanes(P.nx);
