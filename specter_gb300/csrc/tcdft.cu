@@ -1416,11 +1416,13 @@ int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
 }
 
 // Rows of fields: real rows to half spectra (r2c) and back.  Back they go through tiles whose writes are
-// coalesced (written row by row, 256^2 x 282 took 439 us instead of 251 and 61 for the copy).  Shorter rows
-// stay with the Stockham engine (half spectra to rows at 64^2 x 90: 33 us against 47; at 128^2 x 154 121
-// against 112, at 256^2 x 282 758 against 420).
+// coalesced (written row by row, 256^2 x 282 took 439 us instead of 251 and 61 for the copy).  A few short
+// rows stay with the Stockham engine, one launch instead of two or three (whole transforms to physical
+// space, Stockham against digits, us: 32 x 32 x 58 33 and 38, 64 x 64 x 90 60 and 51, 32 x 128 x 154 107 and 78,
+// 64 x 192 x 282 338 and 195).
+constexpr unsigned kFewRows = 16 * kLanes;
 int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
-    if (!tc_length_ok(P.nx) || P.nx < 96) return kNoFast;
+    if (!tc_length_ok(P.nx) || (P.nx < 96 && (unsigned)a.nrows * P.ny < kFewRows)) return kNoFast;
     SG_TRY(workspace(P));
     if (!r2c) SG_TRY(phys_rows(P));
     SG_TRY(tc_status(P));

@@ -78,6 +78,25 @@ def test_x_rows(nx):
     assert np.linalg.norm(o.download() - want) < TOL * np.linalg.norm(want)
 
 
+# short rows, on both sides of the number of rows from which they are digit products (2048)
+@pytest.mark.parametrize("nx", [32, 34, 64, 94])
+@pytest.mark.parametrize("ny", [56, 58])
+def test_short_x_rows(nx, ny):
+    p = plan(nx, ny, 36)
+    rng = np.random.default_rng(nx + ny)
+    r = rng.standard_normal(p.rshape)
+    f, c, o = p.field(api.REAL, data=r), p.field(), p.field(api.REAL)
+    api.fftp2d_real_to_complex_xy(p, f, c)
+    want = np.fft.rfft2(r).transpose(2, 1, 0)
+    assert np.linalg.norm(c.download() - want) < TOL * np.linalg.norm(want)
+    a = rng.standard_normal(p.sshape) + 1j * rng.standard_normal(p.sshape)
+    c.upload(a)
+    api.fftp2d_complex_to_real_xy(p, c, o)
+    y = np.fft.ifft(a.transpose(2, 1, 0), axis=1) * ny
+    want = np.fft.irfft(y, n=nx, axis=2) * nx
+    assert np.linalg.norm(o.download() - want) < TOL * np.linalg.norm(want)
+
+
 def test_non_finite_and_denormal_columns():
     p = plan(8, 4, 58)
     rng = np.random.default_rng(0)
