@@ -467,7 +467,7 @@ def extra_forms(api, initial, cfg, local, form, line, peak, caps):
     line["fp64"] = {"value": round(v64, 2), "unit": UNIT, "ms_per_step": round(ms64 / 2, 3), "steps": 2,
                     "roofline_hbm": {"stage_model_gbs": round(model64, 1), "peak": peak, "frac": round(model64 / peak, 4)},
                     "roofline_fp64": {"model_fft_tflops": round(flops64, 3), "peak_tflops": round(fpeak, 3),
-                                      "peak_kind": "measured FP64 DGEMM (torch.matmul 8192^3)",
+                                      "peak_kind": "measured FP64 DGEMM (torch.matmul 8192^3); above 1: the transforms run as exact digit products on the tensor cores",
                                       "frac": round(flops64 / fpeak, 4)},
                     "kernels_ms_per_step": {k: round(v[1] / 2, 2)
                                             for k, v in sorted(rep64.items(), key=lambda kv: -kv[1][1])[:6]}}

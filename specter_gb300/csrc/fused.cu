@@ -191,7 +191,7 @@ static int harmonic_spectra(Plan &P, void *E1, void *E2) {
 }
 
 // Plain FP64 solvers run the stage of stage_f64.cu where the z length has digit-product transforms; the
-// column kernels on the FP64 Stockham engine serve the others (211 against 37 ms an RK2 step of
+// column kernels on the FP64 Stockham engine serve the others (211 against 25 ms an RK2 step of
 // Rayleigh-Benard convection at 256^2 x 257).
 static bool plain_f64(const Plan &P, const StageParams &sp) { return P.prec == FP64 && !sp.nl_fp32 && f64_stage_ok(P); }
 
