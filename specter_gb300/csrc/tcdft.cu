@@ -27,6 +27,7 @@
 #include "fast.h"
 #include "ops.h"
 #include "tcdft.h"
+#include "tcranges.h"
 
 namespace sg {
 
@@ -1172,9 +1173,13 @@ int tc_status(const Plan &P) {
 namespace {
 
 // One range of tiles of one set of jobs: arguments of the digit and of the product kernels.
-void fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int nj, unsigned t0, unsigned nt, DigArgs &d,
+int fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int nj, unsigned t0, unsigned nt, DigArgs &d,
                GemmArgs &g) {
     TcState *S = P.tc;
+    if ((size_t)nj * nt * D.ks.all() * kAStage > S->ws_bytes || (size_t)nj * nt * kLanes > S->expo_count) {
+        set_error("digit workspace too small for a launch");
+        return ERR_STATE;
+    }
     d.s = g.s = s;
     for (int j = 0; j < nj; j++) d.job[j] = g.job[j] = jobs[j];
     d.m = g.m = D.m;
@@ -1193,6 +1198,7 @@ void fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int 
     g.nchunk = D.nchunk;
     g.nc = D.nc;
     g.err = S->err_dev;
+    return OK;
 }
 
 // lanes per digit block: three blocks on an SM
@@ -1239,27 +1245,26 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
     const size_t per = (size_t)D.ks.all() * kAStage;
     const unsigned tiles = (s.ncol + 63) / 64;
     const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
-    // all jobs at once when they fit, else job by job in ranges of tiles
-    const int jstep = (size_t)tiles * njobs <= cap ? njobs : 1;
-    const unsigned tstep = jstep == njobs ? tiles : (unsigned)std::min<size_t>(tiles, cap);
+    const TcRange range = tc_range(njobs, tiles, cap);
     const int lw = digit_lanes(s.n);
     const size_t dsm = (size_t)s.n * lw * 8;
-    for (int j0 = 0; j0 < njobs; j0 += jstep)
-        for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
-            const unsigned nt = std::min(tstep, tiles - t0);
+    for (int j0 = 0; j0 < njobs; j0 += range.jobs)
+        for (unsigned t0 = 0; t0 < tiles; t0 += range.tiles) {
+            const int nj = std::min(range.jobs, njobs - j0);
+            const unsigned nt = std::min(range.tiles, tiles - t0);
             DigArgs d{};
             GemmArgs g{};
-            fill_args(P, D, s, jobs + j0, jstep, t0, nt, d, g);
+            SG_TRY(fill_args(P, D, s, jobs + j0, nj, t0, nt, d, g));
             const size_t blocks = (size_t)nt * (kLanes / lw);
-            const dim3 grid((unsigned)blocks, digit_split(D, lw, blocks * jstep), jstep);
-            const double share = (double)nt * jstep / ((double)tiles * njobs);
+            const dim3 grid((unsigned)blocks, digit_split(D, lw, blocks * nj), nj);
+            const double share = (double)nt * nj / ((double)tiles * njobs);
             {
-                Launch L(P, "digits", share * bytes * 0.5 + (double)nt * jstep * per);
+                Launch L(P, "digits", share * bytes * 0.5 + (double)nt * nj * per);
                 chain(with_smem(lw == 32 ? k_digits<32> : k_digits<16>, dsm), grid, kDigThreads, dsm, P.stream, d);
             }
             {
                 Launch L(P, name, share * bytes);
-                launch_gemm<kCol>(P, D, g, jstep);
+                launch_gemm<kCol>(P, D, g, nj);
             }
         }
     return check_launch(name);
@@ -1304,7 +1309,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
     const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
     SG_TRY(phys_rows(P));
-    const unsigned tstep = (unsigned)std::min<size_t>(S->phys_tiles, tiles);
+    const unsigned tstep = tc_range(1, tiles, S->phys_tiles).tiles;
     const size_t fstride = S->phys_tiles * ptile;
     const int lw = digit_lanes(n);
     for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
@@ -1328,7 +1333,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
         s.rs = P.ldx;
         DigArgs d{};
         GemmArgs g{};
-        fill_args(P, D, s, jobs, nin, t0, nt, d, g);
+        SG_TRY(fill_args(P, D, s, jobs, nin, t0, nt, d, g));
         {
             const size_t sm = (size_t)(D.m + 1) * (lw + 1) * sizeof(double2);
             Launch L(P, "digits", share * nin / (nin + nc) + (double)nt * nin * per);
@@ -1353,7 +1358,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
         s.ts = (size_t)kLanes * s.ls;
         DigArgs d2{};
         GemmArgs g2{};
-        fill_args(P, D, s, jobs, nc, t0, nt, d2, g2);
+        SG_TRY(fill_args(P, D, s, jobs, nc, t0, nt, d2, g2));
         {
             const size_t sm = (size_t)n * lw * sizeof(double);
             Launch L(P, "products", (double)nt * (nin * ptile * 8.0 + nc * per));
@@ -1437,7 +1442,7 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
     const Dims D = dims(P.nx);
     const size_t per = (size_t)D.ks.all() * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)a.nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
-    const unsigned tstep = (unsigned)std::min<size_t>(tiles, r2c ? cap : std::min(cap, 15 * S->phys_tiles));
+    const unsigned tstep = tc_range(1, tiles, r2c ? cap : std::min(cap, 15 * S->phys_tiles)).tiles;
     const int lw = digit_lanes(P.nx);
     const char *name = r2c ? "x_r2c" : "x_c2r";
     for (int f = 0; f < nf; f++)
@@ -1455,7 +1460,7 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
             tc_job_set(J, set);
             DigArgs d{};
             GemmArgs g{};
-            fill_args(P, D, s, &J, 1, t0, nt, d, g);
+            SG_TRY(fill_args(P, D, s, &J, 1, t0, nt, d, g));
             const size_t blocks = (size_t)nt * (kLanes / lw);
             const dim3 grid((unsigned)blocks, digit_split(D, lw, blocks), 1);
             const double share = bytes * nt / ((double)tiles * nf);
