@@ -15,6 +15,8 @@
 #include <cstring>
 #include <vector>
 
+#include "smem.h"
+
 namespace sg {
 
 // first member of every record: where the instance's blocks start in the batched grid, and the
@@ -44,8 +46,8 @@ struct Batch {
 template <class Rec, class Kern>
 void batch_launch_impl(Kern kern, const void *recs, int n, int blocks, size_t smem, int threads, cudaStream_t s,
                        bool setup_only) {
-    if (setup_only) {  // always: the kernel's static shared memory counts against the default 48 KB too
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (setup_only) {
+        allow_smem(kern, smem);
         return;
     }
     kern<<<blocks, threads, smem, s>>>((const Rec *)recs, n);

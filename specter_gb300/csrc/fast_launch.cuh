@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "fast.h"
+#include "smem.h"
 
 namespace sg {
 namespace {
@@ -25,11 +26,6 @@ int stage_tile(void *const out0[], void *const out1[], int nf, int L, int n) {
     for (int f = 0; f < nf; f++) two |= (out0[f] && out1[f]) ? 1 : 0;
     if (!two) return 0;
     return pick((size_t)L * sizeof(float2)) == pick(((size_t)L + n) * sizeof(float2)) ? 1 : 0;
-}
-
-template <typename K>
-void smem_attr(K kern, size_t bytes) {
-    if (bytes > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 struct Scope {
@@ -62,7 +58,7 @@ int zinv(Plan &P, const ZInvArgs &a0, int nf, double bytes) {
         return OK;
     }
     auto k = (kFixed && tk == 8) ? k_z_inverse<float, E, kFixed ? 8 : 0> : k_z_inverse<float, E>;
-    smem_attr(k, sm);
+    allow_smem(k, sm);
     Scope s(P, "z_inverse", bytes);
     k<<<dim3(cdiv(P.nxh, tk), P.ny, nf), kThreads, sm, P.stream>>>(P.geo, P.tz4.d, a.prepared(), tk);
     return done("z_inverse");
@@ -73,7 +69,7 @@ int zfwd(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
     using E = FourStep<float, L1, L2>;
     const int tk = P.capped(pick((size_t)P.tz4.d.L * sizeof(float2)), Plan::kTileZ);
     const size_t sm = (size_t)P.tz4.d.L * tk * sizeof(float2);
-    smem_attr(k_z_forward<float, E>, sm);
+    allow_smem(k_z_forward<float, E>, sm);
     Scope s(P, "z_forward", bytes);
     k_z_forward<float, E><<<dim3(cdiv(P.nxh, tk), P.ny, nf), kThreads, sm, P.stream>>>(P.geo, P.tz4.d, a.prepared(), tk);
     return done("z_forward");
@@ -97,7 +93,7 @@ int ypass(Plan &P, const YArgs &a0, int nf, int nplanes, double bytes) {
         return OK;
     }
     auto k = (kFixed && tk == 16) ? k_y_pass_t<float, E, kFixed ? 16 : 0> : k_y_pass_t<float, E, 0>;
-    smem_attr(k, sm);
+    allow_smem(k, sm);
     Scope s(P, a.sign < 0 ? "y_forward" : "y_inverse", bytes);
     k<<<dim3(cdiv(P.nxh, tk), nplanes, nf), kThreads, sm, P.stream>>>(P.geo, P.ty4.d, a.prepared(), tk);
     return done("y_pass");
@@ -113,11 +109,11 @@ int xpass(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
     const size_t sm = x_pass_elems<E>(P.tx4.d, P.nxh, rb) * sizeof(float2);
     const dim3 grid(cdiv(a.nrows * P.ny, rb), 1, nf);
     if (r2c) {
-        smem_attr(k_x_r2c<float, E>, sm);
+        allow_smem(k_x_r2c<float, E>, sm);
         Scope s(P, "x_r2c", bytes);
         k_x_r2c<float, E><<<grid, kThreads, sm, P.stream>>>(P.geo, P.tx4.d, a.prepared(), rb);
     } else {
-        smem_attr(k_x_c2r<float, E>, sm);
+        allow_smem(k_x_c2r<float, E>, sm);
         Scope s(P, "x_c2r", bytes);
         k_x_c2r<float, E><<<grid, kThreads, sm, P.stream>>>(P.geo, P.tx4.d, a.prepared(), rb);
     }
@@ -149,7 +145,7 @@ int xnl(Plan &P, const XNLArgs &a, double bytes) {
     }
     const size_t sm = (fixed ? x_nl_pipe_elems(P.nxh, P.H, rb) : x_nl_elems<E>(P.tx4.d, P.nxh, P.H, rb)) * sizeof(float2);
     auto k = fixed ? k_x_nonlinear<float, E, kFixed ? 8 : 0> : k_x_nonlinear<float, E>;
-    smem_attr(k, sm);
+    allow_smem(k, sm);
     Scope s(P, "x_nonlinear", bytes);
     k<<<dim3(cdiv(a.nrows * P.ny, rb)), kThreads, sm, P.stream>>>(P.geo, P.tx4.d, a.prepared(), rb);
     return done("x_nonlinear");

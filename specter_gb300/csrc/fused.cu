@@ -4,6 +4,7 @@
 #include "fused.h"
 #include "fast.h"
 #include "fused_launch.cuh"
+#include "smem.h"
 #include "stage_f64.h"
 
 namespace sg {
@@ -174,7 +175,7 @@ static int harmonic_spectra(Plan &P, void *E1, void *E2) {
     else {
         const size_t sm = 2 * (size_t)t->d.L * tk * es;
         auto k = k_z_forward<double, GenericFFT<double>>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(cdiv(P.nxh, tk), P.ny, 2), kThreads, sm, P.stream>>>(P.geo, t->d, a, tk);
         if (P.prec != FP64) {
             k_narrow<<<152 * 8, 256, 0, P.stream>>>(p1, (float2 *)E1, n);

@@ -5,6 +5,7 @@
 
 #include "ffzoom.cuh"
 #include "fused_kernels.cuh"
+#include "smem.h"
 
 namespace sg {
 
@@ -69,25 +70,25 @@ int launch_fused(Plan &P, const typename E::Desc &fd, const FusedArgs &a, int wh
     P.prof_begin(name, bytes);
     if (which == kFusedVelocity) {
         auto k = k_fused_velocity<T, E>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(cdiv(P.nxh, tk), P.ny), E::wide_threads(tk), sm, P.stream>>>(P.geo, fd, a.prepared(), tk);
     } else if (which == kFusedVComp) {
         auto k = (FIX && tk == FIX) ? k_fused_vcomp<T, E, FIX> : k_fused_vcomp<T, E>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(cdiv(P.nxh, tk), P.ny, 3), E::kColThreads, sm, P.stream>>>(P.geo, fd, a.prepared(), tk);
     } else if (which == kFusedVProj) {
         // the projection holds three components, so at the same cap it runs half the width of
         // the other column kernels: its own fixed-width copy at FIX / 2
         auto k = (FIX && tk == FIX) ? k_fused_vproj<T, E, FIX> : (FIX && tk == FIX / 2) ? k_fused_vproj<T, E, FIX / 2> : k_fused_vproj<T, E>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(cdiv(P.nxh, tk), P.ny), E::kColThreads, sm, P.stream>>>(P.geo, fd, a.prepared(), tk);
     } else if (which == kFusedTheta) {
         auto k = (FIX && tk == FIX) ? k_fused_theta<T, E, FIX> : k_fused_theta<T, E>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(cdiv(P.nxh, tk), P.ny), E::kColThreads, sm, P.stream>>>(P.geo, fd, a.prepared(), tk);
     } else {
         auto k = k_theta_herm<T, E>;
-        if (sm > 40 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        allow_smem(k, sm);
         k<<<dim3(P.ny, 2), E::kColThreads, sm, P.stream>>>(P.geo, fd, a.prepared());
     }
     P.prof_end();

@@ -7,6 +7,7 @@
 #include "kernels.cuh"
 #include "kernels_elem.cuh"
 #include "ops.h"
+#include "smem.h"
 #include "stage_f64.h"
 #include "tcdft.h"
 
@@ -38,13 +39,6 @@ static int pick_tile(size_t per_col_bytes) {
     for (int t : {16, 8, 4, 2, 1})
         if (per_col_bytes * t <= kSmemBudget) return t;
     return 0;
-}
-
-// Opt in to more than the default 48 KB per block early: kernels that run the FC-Gram
-// continuation also hold a small static array (fc_continuation), which counts against it.
-template <typename K>
-static void set_smem(K kern, size_t bytes) {
-    if (bytes > 40 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 static int elem_blocks(const Plan &P, int rows) {
@@ -85,7 +79,7 @@ static int launch_z_inverse(Plan &P, const ZInvArgs &a0, int nf) {
     if constexpr (is_f64<T>) fst = tc_z_inverse(P, a, nf, bytes);
     else fst = fast_z_inverse(P, a, nf, bytes);
     if (fst != kNoFast) return fst;
-    set_smem(k_z_inverse<T, GenericFFT<T>>, sm);
+    allow_smem(k_z_inverse<T, GenericFFT<T>>, sm);
     Launch L(P, "z_inverse", bytes);
     k_z_inverse<T, GenericFFT<T>><<<dim3(cdiv(P.nxh, tk), P.ny, nf), kThreads, sm, P.stream>>>(P.geo, P.tz.d, a.prepared(), tk);
     return check_launch("z_inverse");
@@ -102,7 +96,7 @@ static int launch_z_forward(Plan &P, const ZFwdArgs &a, int nf) {
     if constexpr (is_f64<T>) fst = tc_z_forward(P, a, nf, bytes);
     else fst = fast_z_forward(P, a, nf, bytes);
     if (fst != kNoFast) return fst;
-    set_smem(k_z_forward<T, GenericFFT<T>>, sm);
+    allow_smem(k_z_forward<T, GenericFFT<T>>, sm);
     Launch L(P, "z_forward", bytes);
     k_z_forward<T, GenericFFT<T>><<<dim3(cdiv(P.nxh, tk), P.ny, nf), kThreads, sm, P.stream>>>(P.geo, P.tz.d, a.prepared(), tk);
     return check_launch("z_forward");
@@ -122,7 +116,7 @@ static int launch_y(Plan &P, const YArgs &a0, int nf, int nplanes) {
     if constexpr (is_f64<T>) fst = tc_y(P, a, nf, nplanes, bytes);
     else fst = fast_y(P, a, nf, nplanes, bytes);
     if (fst != kNoFast) return fst;
-    set_smem(k_y_pass_t<T, GenericFFT<T>, 0>, sm);
+    allow_smem(k_y_pass_t<T, GenericFFT<T>, 0>, sm);
     Launch L(P, a.sign < 0 ? "y_forward" : "y_inverse", bytes);
     k_y_pass_t<T, GenericFFT<T>, 0><<<dim3(cdiv(P.nxh, tk), nplanes, nf), kThreads, sm, P.stream>>>(P.geo, P.ty.d, a.prepared(), tk);
     return check_launch("y_pass");
@@ -144,11 +138,11 @@ static int launch_x(Plan &P, const XArgs &a, int nf, bool r2c) {
     else fst = fast_x(P, a, nf, r2c, bytes);
     if (fst != kNoFast) return fst;
     if (r2c) {
-        set_smem(k_x_r2c<T, GenericFFT<T>>, sm);
+        allow_smem(k_x_r2c<T, GenericFFT<T>>, sm);
         Launch L(P, "x_r2c", bytes);
         k_x_r2c<T, GenericFFT<T>><<<grid, kThreads, sm, P.stream>>>(P.geo, P.tx.d, a.prepared(), rb);
     } else {
-        set_smem(k_x_c2r<T, GenericFFT<T>>, sm);
+        allow_smem(k_x_c2r<T, GenericFFT<T>>, sm);
         Launch L(P, "x_c2r", bytes);
         k_x_c2r<T, GenericFFT<T>><<<grid, kThreads, sm, P.stream>>>(P.geo, P.tx.d, a.prepared(), rb);
     }
@@ -171,7 +165,7 @@ static int launch_x_nl(Plan &P, const XNLArgs &a) {
     if constexpr (!is_f64<T>) fst = fast_x_nl(P, a, bytes);
     else fst = tc_x_nonlinear(P, a, bytes);
     if (fst != kNoFast) return fst;
-    set_smem(k_x_nonlinear<T, GenericFFT<T>>, sm);
+    allow_smem(k_x_nonlinear<T, GenericFFT<T>>, sm);
     Launch L(P, "x_nonlinear", bytes);
     k_x_nonlinear<T, GenericFFT<T>><<<dim3(cdiv(a.nrows * P.ny, rb)), kThreads, sm, P.stream>>>(P.geo, P.tx.d, a.prepared(), rb);
     return check_launch("x_nonlinear");

@@ -11,6 +11,7 @@
 #include "chain.h"
 #include "fast.h"
 #include "kernels_elem.cuh"
+#include "smem.h"
 #include "stage_f64.h"
 #include "tcdft.h"
 
@@ -246,7 +247,7 @@ int f64_poisson(Plan &P, void *vx, void *vy, void *vz, void *d, void *th, double
 int f64_profile(Plan &P, const double2 *coef, void *prof, void *deriv) {
     Launch L(P, "stage_profile", (deriv ? 2.0 * P.nz : (double)P.nzp) * P.ny * P.nxh * 16.0);
     const size_t sm = (size_t)(kProfJ + cdiv(P.nzp, kProfJ)) * 32 * sizeof(double);
-    if (sm > 40 * 1024) cudaFuncSetAttribute(k_stage_profile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(k_stage_profile, sm);
     chain(k_stage_profile, dim3(cdiv(P.nxh, 32), P.ny), dim3(32, 8), sm, P.stream, P.geo, coef, (double2 *)prof, (double2 *)deriv, P.dz);
     return check_launch("profile");
 }

@@ -26,6 +26,7 @@
 #include "chain.h"
 #include "fast.h"
 #include "ops.h"
+#include "smem.h"
 #include "tcdft.h"
 #include "tcranges.h"
 
@@ -1224,14 +1225,14 @@ void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     const bool two = 2 * kLev * D.nc <= 512;
     const auto k = MODE == kCol && add ? (two ? k_gemm<MODE, MODE == kCol, 2> : k_gemm<MODE, MODE == kCol, 1>)
                                        : (two ? k_gemm<MODE, false, 2> : k_gemm<MODE, false, 1>);
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k, smem);
     if (g.units <= 152) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
     else k<<<152, kGemmBlock, smem, P.stream>>>(g);
 }
 
 template <typename K>
 K with_smem(K k, size_t bytes) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    allow_smem(k, bytes);
     return k;
 }
 
