@@ -11,6 +11,7 @@
 #include "fused.h"
 #include "handles.h"
 #include "ops.h"
+#include "tcdft.h"
 
 using namespace sg;
 
@@ -150,7 +151,7 @@ int specter_plan_synchronize(specter_plan *plan) {
     CHECK_PLAN(plan);
     cudaError_t e = cudaStreamSynchronize(plan->p->stream);
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return SPECTER_ERR_CUDA; }
-    return SPECTER_OK;
+    return tc_status(*plan->p);
 }
 
 int specter_plan_stream(specter_plan *plan, void **stream) {
@@ -327,7 +328,7 @@ int specter_fields_download(int n, specter_field *const *fields, void *const *ho
         cudaEventRecord(P.xfer_ev[b], P.copy_stream);
     }
     if (cudaStreamSynchronize(P.copy_stream) != cudaSuccess) return check_launch("download");
-    return SPECTER_OK;
+    return tc_status(P);
 }
 
 int specter_field_download(const specter_field *f, void *host) {
@@ -344,7 +345,7 @@ int specter_field_download(const specter_field *f, void *host) {
         if (cudaMemcpyAsync(host, stg, nbytes, cudaMemcpyDeviceToHost, P.stream) != cudaSuccess) return check_launch("download");
     }
     if (cudaStreamSynchronize(P.stream) != cudaSuccess) return check_launch("download");
-    return SPECTER_OK;
+    return tc_status(P);
 }
 
 int specter_field_copy(specter_field *dst, const specter_field *src) {
@@ -672,6 +673,7 @@ int specter_plan_set_option(specter_plan *plan, const char *name, int value) {
     if (!strcmp(name, "ff_pair_proj")) { P.ff_pair_proj = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_pair_cols")) { P.ff_pair_cols = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_zoom")) { P.ff_zoom = value ? 1 : 0; return SPECTER_OK; }
+    if (!strcmp(name, "gave_up")) { *P.gave_up = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_threads")) {
         if (value != 256 && value != 384) { set_error("ff_threads is 256 or 384"); return SPECTER_ERR_ARG; }
         P.ff_threads = value;
@@ -694,7 +696,7 @@ int specter_plan_get_option(specter_plan *plan, const char *name, int *value) {
     const Plan &P = *plan->p;
     const struct { const char *n; int v; } opts[] = {
         {"velocity_split", P.velocity_split}, {"ff_threads", P.ff_threads}, {"ff_engine", P.ff_engine},
-        {"ff_pair_proj", P.ff_pair_proj},     {"ff_pair_cols", P.ff_pair_cols}, {"ff_zoom", P.ff_zoom},
+        {"ff_pair_proj", P.ff_pair_proj},     {"ff_pair_cols", P.ff_pair_cols}, {"ff_zoom", P.ff_zoom}, {"gave_up", *P.gave_up},
         {"tile_cap_z", P.tile_cap[0]},
         {"tile_cap_y", P.tile_cap[1]},        {"tile_cap_x", P.tile_cap[2]},   {"tile_cap_fused", P.tile_cap[3]}};
     for (const auto &o : opts)
@@ -774,6 +776,7 @@ struct specter_graph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaStream_t> streams;  // distinct plan streams of the captured solvers
+    std::vector<specter_plan *> plans;  // and their plans, held
     std::vector<cudaEvent_t> ev;        // one per stream (join at capture, entry at launch)
     cudaEvent_t fork = nullptr, done = nullptr;
     long long kernels = 0;
@@ -790,6 +793,7 @@ int specter_graph_destroy(specter_graph *g) {
     if (g->fork) cudaEventDestroy(g->fork);
     if (g->done) cudaEventDestroy(g->done);
     if (g->root) cudaStreamDestroy(g->root);
+    for (specter_plan *p : g->plans) plan_release(p);
     delete g;
     return SPECTER_OK;
 }
@@ -816,7 +820,10 @@ int specter_graph_create(specter_solver *const *solvers, int n, int nsteps, spec
         cudaStream_t s = solvers[i]->plan->p->stream;
         bool seen = false;
         for (cudaStream_t t : g->streams) seen = seen || t == s;
-        if (!seen) g->streams.push_back(s);
+        if (seen) continue;
+        g->streams.push_back(s);
+        g->plans.push_back(solvers[i]->plan);
+        solvers[i]->plan->refs++;
     }
     cudaStreamCreateWithFlags(&g->root, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming);
@@ -855,8 +862,16 @@ int specter_graph_create(specter_solver *const *solvers, int n, int nsteps, spec
     return SPECTER_OK;
 }
 
+// a replayed step runs no host code of its own: what its kernels gave up is looked at here
+static int graph_status(const specter_graph *g) {
+    for (const specter_plan *p : g->plans)
+        if (int st = tc_status(*p->p)) return st;
+    return SPECTER_OK;
+}
+
 int specter_graph_launch(specter_graph *g) {
     if (!g || !g->exec) { set_error("null graph"); return SPECTER_ERR_ARG; }
+    if (int st = graph_status(g)) return st;
     for (size_t j = 0; j < g->streams.size(); j++) {
         cudaEventRecord(g->ev[j], g->streams[j]);
         cudaStreamWaitEvent(g->root, g->ev[j], 0);
@@ -870,13 +885,13 @@ int specter_graph_launch(specter_graph *g) {
 int specter_graph_synchronize(specter_graph *g) {
     if (!g) { set_error("null graph"); return SPECTER_ERR_ARG; }
     if (cudaStreamSynchronize(g->root) != cudaSuccess) return check_launch("graph synchronize");
-    return SPECTER_OK;
+    return graph_status(g);
 }
 
 int specter_graph_query(specter_graph *g, int *done) {
     if (!g || !done) { set_error("null argument"); return SPECTER_ERR_ARG; }
     const cudaError_t e = cudaStreamQuery(g->root);
-    if (e == cudaSuccess) { *done = 1; return SPECTER_OK; }
+    if (e == cudaSuccess) { *done = 1; return graph_status(g); }
     if (e == cudaErrorNotReady) { cudaGetLastError(); *done = 0; return SPECTER_OK; }
     return check_launch("graph query");
 }

@@ -28,6 +28,7 @@
 #include "handles.h"
 #include "kernels_elem.cuh"
 #include "ops.h"
+#include "tcdft.h"
 
 namespace sg {
 
@@ -99,6 +100,7 @@ static int wall_check_static(Plan &P, const void *a, const void *b, double *bot,
         set_error(std::string("bouncheck_z_static: ") + cudaGetErrorString(cudaGetLastError()));
         return ERR_CUDA;
     }
+    if (int st = tc_status(P)) return st;
     *bot = host[0];
     *top = host[1];
     return OK;

@@ -188,6 +188,7 @@ static int finish_reduce(Plan &P, int nblocks, int per, double *out) {
     if (cudaMemcpyAsync(h, P.dred, (size_t)nblocks * per * sizeof(double), cudaMemcpyDeviceToHost, P.stream) != cudaSuccess ||
         cudaStreamSynchronize(P.stream) != cudaSuccess)
         return check_launch("reduce");
+    SG_TRY(tc_status(P));
     for (int j = 0; j < per; j++) {
         double s = 0.0;
         for (int b = 0; b < nblocks; b++) s += h[(size_t)b * per + j];

@@ -338,7 +338,12 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
         cudaMemcpy(p->dwtwq, wq.data(), wq.size() * sizeof(ff), cudaMemcpyHostToDevice);
         G.wtwq = p->dwtwq;
     }
-    cudaMallocHost(&p->hred, sizeof(double) * p->nred);
+    cudaMallocHost(&p->hred, sizeof(double) * (p->nred + 1));
+    if (p->hred) {
+        p->gave_up = (int *)(p->hred + p->nred);
+        *p->gave_up = 0;
+        cudaHostGetDevicePointer((void **)&p->gave_up_dev, p->gave_up, 0);
+    }
     if (cudaGetLastError() != cudaSuccess) { set_error("CUDA error during plan creation"); plan_destroy(p); return ERR_CUDA; }
     *out = p;
     return OK;

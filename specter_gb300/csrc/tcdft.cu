@@ -100,7 +100,6 @@ struct TcState {
     size_t expo_count = 0;
     double *phys = nullptr;       // physical rows of the nonlinear term's x pass, one range of tiles
     size_t phys_tiles = 0;        // tiles of it per field
-    int *err = nullptr, *err_dev = nullptr;  // host-mapped: set by a kernel that gave up a wait
 };
 
 namespace {
@@ -1146,27 +1145,22 @@ static int workspace(Plan &P) {
         want = std::max(want, t * per);
         tiles = std::max(tiles, t);
     }
-    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * kLanes * sizeof(int)) != cudaSuccess ||
-        cudaHostAlloc(&S->err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer(&S->err_dev, S->err, 0) != cudaSuccess) {
+    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * kLanes * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         if (S->ws) cudaFree(S->ws);
         if (S->expo) cudaFree(S->expo);
-        if (S->err) cudaFreeHost(S->err);
         S->ws = nullptr;
         S->expo = nullptr;
-        S->err = nullptr;
         set_error("out of device memory (digit workspace)");
         return ERR_OOM;
     }
-    *S->err = 0;
     S->ws_bytes = want;
     S->expo_count = tiles * kLanes;
     return OK;
 }
 
 int tc_status(const Plan &P) {
-    if (!P.tc || !P.tc->err || !*(volatile int *)P.tc->err) return OK;
+    if (!*(volatile int *)P.gave_up) return OK;
     set_error("a transform kernel gave up a wait");
     return ERR_CUDA;
 }
@@ -1198,7 +1192,7 @@ int fill_args(Plan &P, const Dims &D, const TcShape &s, const TcJob *jobs, int n
     g.nq[1] = D.nq[1];
     g.nchunk = D.nchunk;
     g.nc = D.nc;
-    g.err = S->err_dev;
+    g.err = P.gave_up_dev;
     return OK;
 }
 
@@ -1515,7 +1509,6 @@ void tc_free(Plan &P) {
     if (P.tc->ws) cudaFree(P.tc->ws);
     if (P.tc->expo) cudaFree(P.tc->expo);
     if (P.tc->phys) cudaFree(P.tc->phys);
-    if (P.tc->err) cudaFreeHost(P.tc->err);
     delete P.tc;
     P.tc = nullptr;
 }

@@ -51,7 +51,9 @@ int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes);
 int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes);
 void tc_free(Plan &P);
 unsigned long long tc_bytes(const Plan &P);
-// non-zero when a kernel of the plan gave up a wait (checked after synchronising)
+// An error when a kernel of the plan gave up a wait: its results are wrong, and so may be whatever was made of
+// them.  Looked at before a transform is queued and wherever the plan's work has been waited for, so that no
+// call that hands out results or reports completion succeeds after it.
 int tc_status(const Plan &P);
 
 }  // namespace sg
