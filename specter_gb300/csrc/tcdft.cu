@@ -7,10 +7,13 @@
 // parts.  Inputs become 62-bit integers against their column's largest value, folded exactly, and
 // split into seven signed 9-bit digits (|d| <= 256, exact in bf16); the matrices are held as seven
 // digits too.  Products of digit i of the data and digit j of the matrix, i + j <= 6, accumulate in
-// FP32 in tensor memory, one accumulator per level i + j (levels 5 and 6 share one).  A level's sums
-// are integers below 2^24 (checked for every matrix when its table is built: levels 0 to 2 for any
-// data), so they are exact whatever the order; what is dropped is below 2^-60 of the column's
-// largest value.  The levels are put together as a 64-bit integer and rounded once to FP64.
+// FP32 in tensor memory, one accumulator per level i + j (levels 5 and 6 share one).  The sums of levels
+// 0 to 2 are integers below 2^24 for any data (checked for every matrix when its table is built), so they are
+// exact whatever the order; those of levels 3 and 4 are, but for data whose digits are in step with the
+// matrix's at lengths above about 400, and such sums are found by their size and made again in integers
+// (mend_outputs).  What is rounded or dropped beyond is below 2^-58 of the column's largest value an input.  The
+// levels are put together as a 64-bit integer and rounded once to FP64.  (Products of floating-point matrices by
+// splitting into parts whose products are exact: Ozaki, Ogita, Oishi and Rump, 2012.)
 //
 // Error against long double, relative L2 (n = 58 .. 538): 5e-17 .. 1.7e-16, a double-precision FFT
 // 1.4e-16 .. 5e-16.
@@ -29,6 +32,7 @@
 #include "smem.h"
 #include "tcdft.h"
 #include "tcranges.h"
+#include "tctables.h"
 
 namespace sg {
 
@@ -40,11 +44,8 @@ namespace sg {
 
 namespace {
 
-constexpr int kDig = 7;             // digits of data and matrix
 constexpr int kLev = 6;             // accumulators (levels 0..4, 5 + 6)
 constexpr int kLanes = 128;         // rows of an MMA: 64 columns, real and imaginary parts
-constexpr int kMaxNc = 80;          // outputs per block: kLev * 80 = 480 of 512 tensor-memory columns
-constexpr int kMaxLen = 550;        // every even length up to here holds the exactness bound of level 2
 constexpr int kAStage = kDig * kLanes * 16 * 2;  // bytes of one 16-deep step of data digits
 constexpr int kDigThreads = 256;
 // Outputs as integers in units of 2^-kSh of the level-0 unit: results are below (n + 2) * sqrt(2) * 2^14
@@ -55,34 +56,6 @@ constexpr int kNaN = 0x40000000;    // exponent of a column that holds a non-fin
 // what a launch transforms: complex columns; real rows to half spectra; half spectra to real rows
 enum { kCol = 0, kR2C = 1, kC2R = 2 };
 
-// Steps of 16 values in the four lists: `first` for the cosine list of the even frequencies (K = m/2 + 1
-// values), `rest` for each of the others, one step less where m is a multiple of 32 (they hold m/2 values;
-// 64^3: 5 steps instead of 8, 128^3: 9 of 12, 512^3: 33 of 36).
-struct Steps {
-    int first, rest;
-    __host__ __device__ int of(int list) const { return list ? rest : first; }
-    __host__ __device__ int before(int list) const { return list ? first + (list - 1) * rest : 0; }
-    __host__ __device__ int all() const { return first + 3 * rest; }
-};
-struct Dims {
-    int n, m, K, nq[2], nchunk, nc;
-    Steps ks;
-};
-Dims dims(int n) {
-    Dims d;
-    d.n = n;
-    d.m = n / 2;
-    d.K = d.m / 2 + 1;
-    d.nq[0] = d.m / 2 + 1;
-    d.nq[1] = (d.m + 1) / 2;
-    d.ks.first = (d.nq[0] + 15) / 16;
-    d.ks.rest = (d.nq[1] + 15) / 16;
-    const int np = (d.nq[0] + 15) / 16 * 16;
-    d.nchunk = (np + kMaxNc - 1) / kMaxNc;
-    d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
-    return d;
-}
-
 }  // namespace
 
 struct TcSet {
@@ -90,6 +63,7 @@ struct TcSet {
     size_t bytes = 0;
     int expo = 0;
     double post = 1.0;
+    float top[2] = {0.f, 0.f};
 };
 
 struct TcState {
@@ -195,6 +169,20 @@ __device__ __forceinline__ size_t col_offset(const TcShape &s, unsigned c) {
     return (size_t)q * s.s + (c - q * s.w);
 }
 
+// Epilogue warps per quarter of the lanes: the more there are, the better they hide one another's latencies,
+// until the registers of a thread (80 with five) no longer hold its sine products.  z transform of 512^2 x 538
+// and half spectra to rows of 512 x 512 x 538, ms, with three, four, five, six, seven:
+// 1.15 1.13 1.10 1.13 1.13 and 1.03 1.13 0.97 1.03 1.00.
+constexpr int kEpiQ = 5;
+constexpr int kEpiThreads = 128 * kEpiQ, kLoadWarp = kEpiThreads / 32, kMmaWarp = kLoadWarp + 1;
+constexpr int kGemmBlock = kEpiThreads + 64;
+constexpr int kGemmSmem = 223 * 1024;  // dynamic shared memory: what the static arrays leave of 227 KB
+constexpr int kGroups = (kMaxNc / 4 + kEpiQ - 1) / kEpiQ;  // groups of 4 outputs per epilogue warp
+
+// Outputs of a thread that its epilogue has left for mend_outputs: bit 16 * (sine list) + 4 * (group of the warp) +
+// (output of the group).
+__shared__ unsigned s_marks[kEpiThreads];
+
 // The levels of four outputs as integers, sum over v of l[v] * 2^kSh.  A level times 2^9v (level 5 times
 // 2^kSh, rounded) is an integer that an addition of 1.5 * 2^23 leaves in the low mantissa bits while it
 // is below 2^22, as sums of signed digits nearly always are; level 0 goes up to 2^24 and hands what is
@@ -226,19 +214,26 @@ __device__ __forceinline__ bool join_levels(const unsigned (&l)[kLev][4], long l
     return (bad & 0xFF800000u) == 0;
 }
 
-// The same for levels of any size, read again from tensor memory.
+// The same for levels of any size, read again from tensor memory.  An output whose level 3 or 4 may have passed 2^24
+// in FP32 (at or above TcJob::top: digits in step with the matrix's; random data is far below) leaves these two
+// out and is marked, from bit `at` on: mend_outputs adds them.
 struct Four {
     long long u[4];
 };
-__device__ __noinline__ Four join_levels_wide(unsigned at, int nc) {
+template <bool MARK>
+__device__ __noinline__ Four join_levels_wide(unsigned tm, int nc, float top3, float top4, int at) {
     unsigned l[kLev][4];
 #pragma unroll
-    for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
+    for (int v = 0; v < kLev; v++) tmem_ld4(l[v], tm + v * nc);
     tmem_wait(l);
     Four r;
 #pragma unroll
     for (int t = 0; t < 4; t++) {
         auto level = [&](int v, float w) { return (long long)__float2int_rn(__uint_as_float(l[v][t]) * w); };
+        if (MARK && (fabsf(__uint_as_float(l[3][t])) * 134217728.f >= top3 || fabsf(__uint_as_float(l[4][t])) * 68719476736.f >= top4)) {
+            s_marks[threadIdx.x] |= 1u << (at + t);
+            l[3][t] = l[4][t] = 0;
+        }
         r.u[t] = (level(0, 1.f) << kSh) + (level(1, 512.f) << (kSh - 9)) + (level(2, 262144.f) << (kSh - 18)) +
                  (level(3, 134217728.f) << (kSh - 27)) + (level(4, 68719476736.f) << (kSh - 36)) +
                  level(5, (float)(1ull << kSh));
@@ -580,15 +575,6 @@ struct GemmArgs {
     int *err;
 };
 
-// Epilogue warps per quarter of the lanes: the more there are, the better they hide one another's latencies,
-// until the registers of a thread (80 with five) no longer hold its sine products.  z transform of 512^2 x 538
-// and half spectra to rows of 512 x 512 x 538, ms, with three, four, five, six, seven:
-// 1.15 1.13 1.10 1.13 1.13 and 1.03 1.13 0.97 1.03 1.00.
-constexpr int kEpiQ = 5;
-constexpr int kEpiThreads = 128 * kEpiQ, kLoadWarp = kEpiThreads / 32, kMmaWarp = kLoadWarp + 1;
-constexpr int kGemmBlock = kEpiThreads + 64;
-constexpr int kGroups = (kMaxNc / 4 + kEpiQ - 1) / kEpiQ;  // groups of 4 outputs per epilogue warp
-
 // A unit of work: one tile of 64 columns, one parity of the frequency, one chunk of nc outputs.  The
 // data digits are the M = 128 rows (64 columns x real, imaginary), the matrix digits the N = nc columns
 // of the MMAs; a pipeline of bulk copies feeds 28 MMAs a 16-deep step.  One block per SM walks over
@@ -618,13 +604,82 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
     return w;
 }
 
+// Adds levels 3 and 4 to the outputs of this thread that join_levels_wide has left without them: summed in integers
+// from the digits, which are exact whatever their size.  Beside the epilogue, whose registers it would cost 4 % of
+// every launch from within.
+template <int MODE>
+__device__ __noinline__ void mend_outputs(const GemmArgs &a, unsigned u, int par, double *out) {
+    const Unit w = unit_of<MODE>(a, u);
+    const TcJob &J = a.job[w.job];
+    const TcShape &s = a.s;
+    const int lane = threadIdx.x & 127, g0 = threadIdx.x >> 7, nc = a.nc;
+    const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * kLanes + lane], q = e - 1022 - 14 - kSh + J.expo;
+    unsigned marks = s_marks[threadIdx.x];
+    s_marks[threadIdx.x] = 0;
+    if (e >= kNaN) return;
+    for (; marks; marks &= marks - 1) {
+        const int bit = __ffs(marks) - 1, sine = bit >> 4, list = 2 * par + sine;
+        const int col = (g0 + kEpiQ * (bit >> 2 & 3)) * 4 + (bit & 3), j = w.chunk * nc + col;
+        if (col >= w.cols) continue;
+        const unsigned char *data = a.ws + (((size_t)w.job * a.ntile + w.lt) * a.ks.all() + a.ks.before(list)) * kAStage + lane * 16;
+        const unsigned char *mat = J.mat + (size_t)(a.ks.before(list) * a.nchunk + w.chunk * a.ks.of(list)) * (kDig * 32 * nc) + col * 16;
+        long long e3 = 0, e4 = 0;
+        for (int k = 0; k < 16 * a.ks.of(list); k++) {
+            const unsigned step = k / 16, half = k / 8 % 2;  // eight values side by side, two such groups a step
+            const unsigned char *pd = data + (size_t)step * kAStage + half * kLanes * 16 + k % 8 * 2;
+            const unsigned char *pm = mat + (size_t)step * (kDig * 32 * nc) + half * nc * 16 + k % 8 * 2;
+            auto digit = [](const unsigned char *p, int i) {  // bf16 in units of 2^-9i
+                const float v = __uint_as_float((unsigned)*(const unsigned short *)p << 16);
+                return __float2int_rn(v * __uint_as_float((unsigned)(127 + 9 * i) << 23));
+            };
+            int x[5], y[5];
+#pragma unroll
+            for (int i = 0; i < 5; i++) {
+                x[i] = digit(pd + i * (kLanes * 32), i);
+                y[i] = digit(pm + i * (nc * 32), i);
+            }
+            e3 += x[0] * y[3] + x[1] * y[2] + x[2] * y[1] + x[3] * y[0];
+            e4 += x[0] * y[4] + x[1] * y[3] + x[2] * y[2] + x[3] * y[1] + x[4] * y[0];
+        }
+        long long t = (e3 << (kSh - 27)) + (e4 << (kSh - 36));
+        if (sine && (MODE == kR2C || (MODE == kCol && s.sign < 0))) t = -t;
+        const double v = scalbn((double)t, q) * J.post;
+        if (MODE == kCol) {
+            const int f = 2 * j + par, f2 = s.n - f;
+            if (f < s.nrows) out[2 * (size_t)f * s.rs] += v;
+            if (f && f != f2 && f2 < s.nrows) out[2 * (size_t)f2 * s.rs] += sine ? -v : v;
+        } else if (MODE == kR2C) {
+            const int f = 2 * j + par;
+            if (f <= a.m) out[2 * f + sine] += v;
+        } else {
+            const bool two = j && 2 * j != a.m;
+            double *o0 = out + (size_t)j * s.rs, *o1 = out + (size_t)(a.m - j) * s.rs;
+            if (par == 0) {  // integers yet
+                *(long long *)o0 += sine ? -t : t;
+                if (two) *(long long *)o1 += t;
+            } else {
+                const size_t h = (size_t)a.m * s.rs;
+                const double b = sine ? -v : v;
+                o0[0] += b;
+                o0[h] -= b;
+                if (two) {
+                    o1[0] -= v;
+                    o1[h] += v;
+                }
+            }
+        }
+    }
+}
+
 // ADD: jobs may have a field to add (each value's branch costs 5 to 12 %, so launches without one do without).
 // NACC: sets of accumulators in tensor memory, used by the lists in turn.  With two, a list's MMAs run while
 // the sums of the one before are read; lengths below 128 leave room for it (2 * kLev * 32 columns), and their
 // lists are as short as that read: half spectra to rows of 96 x 96 x 122, 91 -> 80 us, of 64 x 64 x 90, 45 -> 40 us.
 // (As a run-time choice it costs longer lengths 5 to 14 %.)
-template <int MODE, bool ADD, int NACC>
-__global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
+// MARK: some job has sums that FP32 may not hold (TcJob::top), so outputs may be left to mend_outputs.  At lengths
+// below about 300 hardly any has, and the launches that do without take 2 % less.
+template <int MODE, bool ADD, int NACC, bool MARK>
+__global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ GemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned long long bars[2 * 8 + 4];
     __shared__ unsigned s_tmem;
@@ -751,13 +806,16 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
 #pragma unroll
             for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
         };
-        auto gather = [&](int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
+        auto gather = [&](const TcJob &J, int sine, int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
             if (__any_sync(~0u, !join_levels(l, u))) {
-                const Four w = join_levels_wide(tset + (g0 + kEpiQ * gi) * 4, nc);
+                const unsigned at = tset + (g0 + kEpiQ * gi) * 4;
+                const Four w = MARK ? join_levels_wide<true>(at, nc, J.top[0], J.top[1], 16 * sine + 4 * gi)
+                                    : join_levels_wide<false>(at, nc, 0.f, 0.f, 0);
 #pragma unroll
                 for (int t = 0; t < 4; t++) u[t] = w.u[t];
             }
         };
+        if (MARK) s_marks[threadIdx.x] = 0;
         int lists = 0;
         auto take = [&] {  // the next list's sums are there
             const int set = lists % NACC;
@@ -812,7 +870,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                         fetch(gi, l);
                         tmem_wait(l);
                         long long P[4];
-                        gather(gi, l, P);
+                        gather(J, 0, gi, l, P);
 #pragma unroll
                         for (int t = 0; t < 4; t++) Ps[((g0 + kEpiQ * gi) * 4 + t) * kLanes] = P[t];
                     }
@@ -825,10 +883,13 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                     if (gi < ngr) {
                         fetch(gi, l);
                         tmem_wait(l);
-                        gather(gi, l, Q[gi]);
+                        gather(J, 1, gi, l, Q[gi]);
                     }
                 give();
-                if (!live) continue;
+                if (!live) {
+                    if (MARK) s_marks[threadIdx.x] = 0;  // of what lies beyond the outputs
+                    continue;
+                }
                 // a group's loads, conversions and stores one after another: loads do not move across stores
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
@@ -935,6 +996,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(GemmArgs a) {
                             }
                         }
                 }
+                if (MARK && s_marks[threadIdx.x]) mend_outputs<MODE>(a, u, par, out);
             }
         }
     }
@@ -990,73 +1052,6 @@ __global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, 
     }
 }
 
-// cos and sin of 2 pi t / n for every t from one octant, in long double
-void circle(int n, std::vector<long double> &c, std::vector<long double> &s) {
-    const long double pi = 3.14159265358979323846264338327950288L;
-    c.assign(n, 0.0L);
-    s.assign(n, 0.0L);
-    std::map<int, std::pair<long double, long double>> cache;  // by 8 t / n folded into the first octant
-    for (int t = 0; t < n; t++) {
-        // angle = 2 pi t / n = (pi / 4) (8 t / n): octant o and remainder u = 8 t - o n, in units of pi / (4 n)
-        const int o = 8 * t / n, u = 8 * t - o * n;
-        const int v = o & 1 ? n - u : u;
-        auto it = cache.find(v);
-        if (it == cache.end()) {
-            const long double x = pi * (long double)v / (4.0L * (long double)n);
-            it = cache.insert({v, {cosl(x), sinl(x)}}).first;
-        }
-        long double a = it->second.first, b = it->second.second;
-        switch (o) {
-            case 0: break;
-            case 1: std::swap(a, b); break;
-            case 2: { const long double w = a; a = -b; b = w; break; }
-            case 3: a = -a; break;
-            case 4: a = -a; b = -b; break;
-            case 5: { const long double w = a; a = -b; b = -w; break; }
-            case 6: { const long double w = a; a = b; b = -w; break; }
-            default: b = -b; break;
-        }
-        c[t] = a;
-        s[t] = b;
-    }
-}
-
-void matrix_digits(long double v, int d[kDig]) {
-    const long long V = llrintl(v * 4611686018427387904.0L);  // 2^62
-    unsigned long long bias = 0;
-    for (int i = 1; i < kDig; i++) bias += 256ull << (54 - 9 * i);
-    const unsigned long long w = (unsigned long long)V + bias;
-    d[0] = (int)((long long)w >> 54);
-    for (int i = 1; i < kDig; i++) d[i] = (int)((w >> (54 - 9 * i)) & 511) - 256;
-}
-
-// Levels 0, 1 and 2 of every output's sums stay below 2^24 for any data digits (|d| <= 256).
-bool exact_levels(const Dims &D, bool half, const std::vector<int> &dc, const std::vector<int> &ds) {
-    std::vector<int> ac(D.n, 0), as(D.n, 0);
-    for (int t = 0; t < D.n; t++)
-        for (int i = 0; i < 3; i++) {
-            ac[t] += std::abs(dc[(size_t)t * kDig + i]);
-            as[t] += std::abs(ds[(size_t)t * kDig + i]);
-        }
-    for (int par = 0; par < 2; par++) {
-        const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
-        for (int o = 0; o < no; o++) {
-            // angles (2 f + par) * point: advance by a fixed step from one input to the next
-            const int step = half ? 2 * o % D.n : (2 * o + par) % D.n;
-            int ang = half ? par * o % D.n : 0;
-            long long sc = 0, ss = 0;
-            for (int i = 0; i < ni; i++) {
-                sc += ac[ang];
-                ss += as[ang];
-                ang += step;
-                if (ang >= D.n) ang -= D.n;
-            }
-            if (256 * std::max(sc, ss) > (1ll << 24)) return false;
-        }
-    }
-    return true;
-}
-
 TcState *state(Plan &P) {
     if (!P.tc) P.tc = new TcState();
     return P.tc;
@@ -1070,6 +1065,8 @@ void tc_job_set(TcJob &j, const TcSet *s) {
     j.mat = s->mat;
     j.expo = s->expo;
     j.post = s->post;
+    j.top[0] = s->top[0];
+    j.top[1] = s->top[1];
 }
 
 const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
@@ -1079,32 +1076,18 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     auto it = S->sets.find(key);
     if (it != S->sets.end()) return &it->second;
     const Dims D = dims(n);
-    std::vector<long double> c, s;
-    circle(n, c, s);
     TcSet set;
-    std::vector<int> dc((size_t)n * kDig), ds((size_t)n * kDig);
-    // factor = scale * 2^expo with scale in (1/2, 1]; a smaller scale where the digits of this one miss
-    // the exactness bound, and the plain matrices with a multiplication after them where all do
-    bool ok = false;
-    int ex = 0;
-    double fr = frexp(factor, &ex);
-    if (fr == 0.5) { fr = 1.0; ex -= 1; }
-    for (int t = 0; t < 5 && !ok; t++) {
-        const long double sc = t < 4 ? (long double)fr / (long double)(1 << t) : 1.0L;
-        for (int k = 0; k < n; k++) {
-            matrix_digits(c[k] * sc, &dc[(size_t)k * kDig]);
-            matrix_digits(s[k] * sc, &ds[(size_t)k * kDig]);
-        }
-        set.expo = t < 4 ? ex + t : 0;
-        set.post = t < 4 ? 1.0 : factor;
-        ok = exact_levels(D, half, dc, ds);
-    }
-    if (!ok) { set_error("digit tables: exactness bound"); *status = ERR_SHAPE; return nullptr; }
+    MatrixDigits M;
+    if (!matrix_digits_for(D, factor, half, M)) { set_error("digit tables: exactness bound"); *status = ERR_SHAPE; return nullptr; }
+    set.expo = M.expo;
+    set.post = M.post;
+    set.top[0] = M.top[0];
+    set.top[1] = M.top[1];
     std::vector<__nv_bfloat16> h(2 * (size_t)n * kDig);
     for (int l = 0; l < 2; l++)
         for (size_t q = 0; q < (size_t)n * kDig; q++) {
             const int i = (int)(q % kDig);
-            h[(size_t)l * n * kDig + q] = __float2bfloat16(ldexpf((float)(l ? ds[q] : dc[q]), -9 * i));
+            h[(size_t)l * n * kDig + q] = __float2bfloat16(ldexpf((float)(l ? M.s[q] : M.c[q]), -9 * i));
         }
     set.bytes = (size_t)D.nchunk * D.ks.all() * kDig * 32 * D.nc;
     __nv_bfloat16 *dig = nullptr;
@@ -1211,14 +1194,18 @@ int digit_split(const Dims &D, int lw, size_t blocks) {
 template <int MODE>
 void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     const unsigned stage = kAStage + kDig * D.nc * 32, psize = (unsigned)std::max(D.nc, 4 * kEpiQ) * kLanes * 8;
-    g.nstage = std::min(8, (int)((226 * 1024 - psize) / stage));
+    g.nstage = std::min(8, (int)((kGemmSmem - psize) / stage));
     g.units = g.ntile * (MODE == kC2R ? 1 : 2) * D.nchunk * nj;
     const size_t smem = (size_t)g.nstage * stage + psize;
-    bool add = false;
-    for (int j = 0; j < nj; j++) add = add || g.job[j].add;
-    const bool two = 2 * kLev * D.nc <= 512;
-    const auto k = MODE == kCol && add ? (two ? k_gemm<MODE, MODE == kCol, 2> : k_gemm<MODE, MODE == kCol, 1>)
-                                       : (two ? k_gemm<MODE, false, 2> : k_gemm<MODE, false, 1>);
+    bool add = false, mark = false;
+    for (int j = 0; j < nj; j++) {
+        add = add || g.job[j].add;
+        mark = mark || !(std::isinf(g.job[j].top[0]) && std::isinf(g.job[j].top[1]));
+    }
+    const bool two = 2 * kLev * D.nc <= 512;  // lengths below 128, whose sums are always exact
+    constexpr bool kAdd = MODE == kCol;
+    const auto k = kAdd && add ? (two ? k_gemm<MODE, kAdd, 2, false> : mark ? k_gemm<MODE, kAdd, 1, true> : k_gemm<MODE, kAdd, 1, false>)
+                               : (two ? k_gemm<MODE, false, 2, false> : mark ? k_gemm<MODE, false, 1, true> : k_gemm<MODE, false, 1, false>);
     allow_smem(k, smem);
     if (g.units <= 152) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
     else k<<<152, kGemmBlock, smem, P.stream>>>(g);

@@ -23,6 +23,7 @@ struct TcJob {
     const unsigned char *mat;  // matrix digits of the table set
     int deriv, expo;      // expo: power of two of the set's factor
     double post;          // further factor applied to the result (1: none)
+    float top[2];         // sums of levels 3 and 4 that are smaller are exact (MatrixDigits)
 };
 
 // Columns: column c of a launch is at element (c / w) * s + c % w of a field, c in [0, ncol).

@@ -1,0 +1,165 @@
+// Lengths, matrix digits and exactness bounds of the digit products (tcdft.cu); host code without CUDA.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <cstdlib>
+#include <map>
+#include <utility>
+#include <vector>
+
+#ifdef __CUDACC__
+#define SG_BOTH __host__ __device__
+#else
+#define SG_BOTH
+#endif
+
+namespace sg {
+
+constexpr int kDig = 7;       // digits of data and matrix
+constexpr int kMaxNc = 80;    // outputs per block: six accumulators of 80 are 480 of 512 tensor-memory columns
+constexpr int kMaxLen = 550;  // every even length up to here holds the bounds of matrix_digits_for
+
+// Steps of 16 values in the four lists: `first` for the cosine list of the even frequencies (K = m/2 + 1
+// values), `rest` for each of the others, one step less where m is a multiple of 32 (they hold m/2 values;
+// 64^3: 5 steps instead of 8, 128^3: 9 of 12, 512^3: 33 of 36).
+struct Steps {
+    int first, rest;
+    SG_BOTH int of(int list) const { return list ? rest : first; }
+    SG_BOTH int before(int list) const { return list ? first + (list - 1) * rest : 0; }
+    SG_BOTH int all() const { return first + 3 * rest; }
+};
+struct Dims {
+    int n, m, K, nq[2], nchunk, nc;
+    Steps ks;
+};
+inline Dims dims(int n) {
+    Dims d;
+    d.n = n;
+    d.m = n / 2;
+    d.K = d.m / 2 + 1;
+    d.nq[0] = d.m / 2 + 1;
+    d.nq[1] = (d.m + 1) / 2;
+    d.ks.first = (d.nq[0] + 15) / 16;
+    d.ks.rest = (d.nq[1] + 15) / 16;
+    const int np = (d.nq[0] + 15) / 16 * 16;
+    d.nchunk = (np + kMaxNc - 1) / kMaxNc;
+    d.nc = ((np + d.nchunk - 1) / d.nchunk + 15) / 16 * 16;
+    return d;
+}
+
+// cos and sin of 2 pi t / n for every t from one octant, in long double
+inline void circle(int n, std::vector<long double> &c, std::vector<long double> &s) {
+    const long double pi = 3.14159265358979323846264338327950288L;
+    c.assign(n, 0.0L);
+    s.assign(n, 0.0L);
+    std::map<int, std::pair<long double, long double>> cache;  // by 8 t / n folded into the first octant
+    for (int t = 0; t < n; t++) {
+        // angle = 2 pi t / n = (pi / 4) (8 t / n): octant o and remainder u = 8 t - o n, in units of pi / (4 n)
+        const int o = 8 * t / n, u = 8 * t - o * n;
+        const int v = o & 1 ? n - u : u;
+        auto it = cache.find(v);
+        if (it == cache.end()) {
+            const long double x = pi * (long double)v / (4.0L * (long double)n);
+            it = cache.insert({v, {cosl(x), sinl(x)}}).first;
+        }
+        long double a = it->second.first, b = it->second.second;
+        switch (o) {
+            case 0: break;
+            case 1: std::swap(a, b); break;
+            case 2: { const long double w = a; a = -b; b = w; break; }
+            case 3: a = -a; break;
+            case 4: a = -a; b = -b; break;
+            case 5: { const long double w = a; a = -b; b = -w; break; }
+            case 6: { const long double w = a; a = b; b = -w; break; }
+            default: b = -b; break;
+        }
+        c[t] = a;
+        s[t] = b;
+    }
+}
+
+inline void matrix_digits(long double v, int d[kDig]) {
+    const long long V = llrintl(v * 4611686018427387904.0L);  // 2^62
+    unsigned long long bias = 0;
+    for (int i = 1; i < kDig; i++) bias += 256ull << (54 - 9 * i);
+    const unsigned long long w = (unsigned long long)V + bias;
+    d[0] = (int)((long long)w >> 54);
+    for (int i = 1; i < kDig; i++) d[i] = (int)((w >> (54 - 9 * i)) & 511) - 256;
+}
+
+// Level v of an output is the sum over the list of the products of digit i of the data and digit v - i of the
+// matrix.  The largest absolute sum of the products, over the outputs, that any data digits (|d| <= 256) can make:
+// every partial sum in any order is below it.  For levels 2, 3 and 4 (those above are in all of them).
+inline void level_bounds(const Dims &D, bool half, const std::vector<int> &dc, const std::vector<int> &ds, long long b[3]) {
+    b[0] = b[1] = b[2] = 0;
+    for (int list = 0; list < 2; list++) {
+        const std::vector<int> &d = list ? ds : dc;
+        for (int v = 2; v <= 4; v++) {
+            std::vector<int> a(D.n, 0);
+            for (int t = 0; t < D.n; t++)
+                for (int i = 0; i <= v; i++) a[t] += std::abs(d[(size_t)t * kDig + i]);
+            for (int par = 0; par < 2; par++) {
+                const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
+                for (int o = 0; o < no; o++) {
+                    // angles (2 f + par) * point: advance by a fixed step from one input to the next
+                    const int step = half ? 2 * o % D.n : (2 * o + par) % D.n;
+                    int ang = half ? par * o % D.n : 0;
+                    long long sum = 0;
+                    for (int i = 0; i < ni; i++) {
+                        sum += a[ang];
+                        ang += step;
+                        if (ang >= D.n) ang -= D.n;
+                    }
+                    b[v - 2] = std::max(b[v - 2], 256 * sum);
+                }
+            }
+        }
+    }
+}
+
+// The digits of one matrix set and what of it the sums can trust.
+struct MatrixDigits {
+    std::vector<int> c, s;  // [angle][kDig] of the cosines, of the sines
+    int expo = 0;           // times 2^expo
+    double post = 1.0;      // and times this after the products (1: none)
+    // A sum of level 3 or 4 whose result is below this is exact in FP32, whatever the order of its terms:
+    // had a partial sum passed 2^24, what is left of the bound could not have brought it back below.
+    float top[2] = {0.f, 0.f};
+};
+
+// factor = scale * 2^expo with scale in (1/2, 1]: the matrices hold cosines and sines times scale.  A smaller scale
+// where those digits miss the bounds, and the plain matrices with a multiplication after them where all do.
+// Bounds: level 2 (and so 0 and 1) exact for any data; levels 3 and 4 trusted up to 2^22 at least, the size from
+// which the epilogue looks at them (join_levels).
+inline bool matrix_digits_for(const Dims &D, double factor, bool half, MatrixDigits &m) {
+    std::vector<long double> c, s;
+    circle(D.n, c, s);
+    m.c.resize((size_t)D.n * kDig);
+    m.s.resize((size_t)D.n * kDig);
+    int ex = 0;
+    double fr = std::frexp(factor, &ex);
+    if (fr == 0.5) { fr = 1.0; ex -= 1; }
+    for (int t = 0; t < 5; t++) {
+        const long double sc = t < 4 ? (long double)fr / (long double)(1 << t) : 1.0L;
+        for (int k = 0; k < D.n; k++) {
+            matrix_digits(c[k] * sc, &m.c[(size_t)k * kDig]);
+            matrix_digits(s[k] * sc, &m.s[(size_t)k * kDig]);
+        }
+        m.expo = t < 4 ? ex + t : 0;
+        m.post = t < 4 ? 1.0 : factor;
+        long long b[3];
+        level_bounds(D, half, m.c, m.s, b);
+        if (b[0] > 1 << 24) continue;
+        bool ok = true;
+        for (int v = 0; v < 2; v++) {
+            const long long top = (1ll << 25) - b[v + 1];
+            if (top < 1 << 22) ok = false;
+            m.top[v] = b[v + 1] <= 1 << 24 ? INFINITY : (float)top;
+        }
+        if (ok) return true;
+    }
+    return false;
+}
+
+}  // namespace sg
