@@ -198,7 +198,10 @@ int specter_plan_tile_caps(specter_plan *plan, const int caps[4]);
  * (0/1: on that engine, the projection kernel and the other column kernels run as one 576-thread
  * block per SM or as two 288-thread blocks; the autotuner picks them), "ff_zoom" (1, the default:
  * on that engine the wall round trips are window corrections of the spectrum when C + 2d = 35 and
- * nz + C + 34 <= 576; 0: an inverse and a forward transform each), "gave_up" (1 once a transform
+ * nz + C + 34 <= 576; 0: an inverse and a forward transform each), "digit_room_mb" (FP64
+ * plans, set before their first use: the most MiB that the digits of a launch of transforms may
+ * take, larger launches run in ranges; 0, the default: 2048; -1: no digit transforms, the general
+ * engine, which needs no buffer), "gave_up" (1 once a transform
  * kernel of the plan has given up a wait: from then on every call that transforms, waits for the
  * plan's work or hands out results returns SPECTER_ERR_CUDA; setting it is for tests of that) */
 int specter_plan_set_option(specter_plan *plan, const char *name, int value);

@@ -673,6 +673,11 @@ int specter_plan_set_option(specter_plan *plan, const char *name, int value) {
     if (!strcmp(name, "ff_pair_proj")) { P.ff_pair_proj = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_pair_cols")) { P.ff_pair_cols = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_zoom")) { P.ff_zoom = value ? 1 : 0; return SPECTER_OK; }
+    if (!strcmp(name, "digit_room_mb")) {
+        if (value < -1) { set_error("digit_room_mb is a number of MiB, 0 or -1"); return SPECTER_ERR_ARG; }
+        P.digit_room_mb = value;
+        return SPECTER_OK;
+    }
     if (!strcmp(name, "gave_up")) { *P.gave_up = value ? 1 : 0; return SPECTER_OK; }
     if (!strcmp(name, "ff_threads")) {
         if (value != 256 && value != 384) { set_error("ff_threads is 256 or 384"); return SPECTER_ERR_ARG; }
@@ -696,7 +701,7 @@ int specter_plan_get_option(specter_plan *plan, const char *name, int *value) {
     const Plan &P = *plan->p;
     const struct { const char *n; int v; } opts[] = {
         {"velocity_split", P.velocity_split}, {"ff_threads", P.ff_threads}, {"ff_engine", P.ff_engine},
-        {"ff_pair_proj", P.ff_pair_proj},     {"ff_pair_cols", P.ff_pair_cols}, {"ff_zoom", P.ff_zoom}, {"gave_up", *P.gave_up},
+        {"ff_pair_proj", P.ff_pair_proj},     {"ff_pair_cols", P.ff_pair_cols}, {"ff_zoom", P.ff_zoom}, {"gave_up", *P.gave_up}, {"digit_room_mb", P.digit_room_mb},
         {"tile_cap_z", P.tile_cap[0]},
         {"tile_cap_y", P.tile_cap[1]},        {"tile_cap_x", P.tile_cap[2]},   {"tile_cap_fused", P.tile_cap[3]}};
     for (const auto &o : opts)

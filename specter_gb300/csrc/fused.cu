@@ -6,6 +6,7 @@
 #include "fused_launch.cuh"
 #include "smem.h"
 #include "stage_f64.h"
+#include "tcdft.h"
 
 namespace sg {
 
@@ -17,6 +18,7 @@ struct FusedState {
     void *E[2] = {nullptr, nullptr};  // z spectra of the unit laplace_z profiles, per column
     void *W[3] = {nullptr, nullptr, nullptr};  // split velocity form: updated components
     int nc = 3;
+    bool plain = false;  // the stage of stage_f64.cu
     // nl_fp32 (FP64 plans): the FP32 companion plan of the nonlinear term and the FP32 copy of
     // the stage input it reads
     Plan *nlp = nullptr;
@@ -206,7 +208,8 @@ int fused_create(Plan &P, const StageParams &sp, FusedState **out) {
         ok = ok && cudaMalloc(&fs->X1[i], P.field_bytes()) == cudaSuccess;
         if (sp.ord >= 3) ok = ok && cudaMalloc(&fs->X2[i], P.field_bytes()) == cudaSuccess;
     }
-    const bool columns = !plain_f64(P, sp);  // buffers of the column kernels
+    fs->plain = plain_f64(P, sp) && tc_reserve(P) == OK;
+    const bool columns = !fs->plain;  // buffers of the column kernels
     if (sp.solver == 1 && columns) ok = ok && cudaMalloc(&fs->side, 2 * (size_t)P.ny * P.nzp * P.elt()) == cudaSuccess;  // BOUSS only
     for (int i = 0; i < 2; i++) ok = ok && cudaMalloc(&fs->E[i], P.field_bytes()) == cudaSuccess;
     for (int i = 0; i < 3 && columns; i++) ok = ok && cudaMalloc(&fs->W[i], P.field_bytes()) == cudaSuccess;
@@ -333,7 +336,7 @@ static int run_stage(Plan &P, FusedState *fs, int o, const void *const vin[4], c
                      void *const vout[4], void *pr) {
     const StageParams &sp = fs->sp;
     if constexpr (is_f64<T>)
-        if (plain_f64(P, sp)) return f64_stage(P, sp, o, vin, cold, vout, pr, fs->E);
+        if (fs->plain) return f64_stage(P, sp, o, vin, cold, vout, pr, fs->E);
     const bool bouss = sp.solver >= 1, rot = sp.solver == 2;
     const void *nl[4] = {nullptr, nullptr, nullptr, nullptr};
     int st = OK;

@@ -92,6 +92,7 @@ struct Plan {
     FFTTable tx, ty, tz;      // lengths H = nx/2, ny, nz
     FFT4Table tx4, ty4, tz4;  // four-step tables of the same lengths (FP32 plans)
     TcState *tc = nullptr;    // FP64 plans: digit-product transforms (tcdft.h), built on first use
+    int digit_room_mb = 0;    // limit of their digits' buffer in MiB (0: kRoomMiB of tcdft.cu; -1: no such transforms)
     int *gave_up = nullptr, *gave_up_dev = nullptr;  // pinned, beside hred: set by a kernel that gave up a wait
     cudaStream_t stream = nullptr;
     // host transfers of several fields: copies on their own stream, double-buffered staging

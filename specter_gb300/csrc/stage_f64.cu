@@ -291,6 +291,11 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
     double2 *x = (double2 *)vout[0], *y = (double2 *)vout[1], *w = (double2 *)vout[2], *th = (double2 *)vout[3];
     void *trip[3] = {x, y, th};
     const int nt = bouss ? 3 : 2;
+    auto done = [](int st) {
+        if (st != kNoFast) return st;
+        set_error("no memory for the digit tables (FP64 stage)");
+        return (int)ERR_OOM;
+    };
     auto inverse = [&](void *const in[], void *const out[], const void *const add[], int n) {
         ZInvArgs z{};
         for (int i = 0; i < n; i++) {
@@ -300,7 +305,7 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
         }
         z.nrows = z.scale_rows = P.nzp;
         z.scale = 1.0 / (double)P.nz;
-        return tc_z_inverse(P, z, n, n * (field + mixed));
+        return done(tc_z_inverse(P, z, n, n * (field + mixed)));
     };
     auto forward = [&](void *const f[], int n) {
         ZFwdArgs z{};
@@ -309,7 +314,7 @@ int f64_stage(Plan &P, const StageParams &sp, int o, const void *const vin[4], c
             z.out[i] = f[i];
         }
         z.in_scale = 1.0;
-        return tc_z_forward(P, z, n, n * (field + mixed));
+        return done(tc_z_forward(P, z, n, n * (field + mixed)));
     };
     SG_TRY(inverse(trip, trip, nullptr, nt));
     double tmp = rmp;

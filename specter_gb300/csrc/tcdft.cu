@@ -70,10 +70,14 @@ struct TcState {
     std::map<std::pair<int, double>, TcSet> sets;  // by length (negative: half spectrum to real) and factor
     unsigned char *ws = nullptr;  // digits
     size_t ws_bytes = 0;
+    int ws_jobs = 0;              // of launches of that many transforms
     int *expo = nullptr;          // column exponents of the digits in ws
     size_t expo_count = 0;
-    double *phys = nullptr;       // physical rows of the nonlinear term's x pass, one range of tiles
-    size_t phys_tiles = 0;        // tiles of it per field
+    double *phys = nullptr;       // physical rows in tiles, of one range of tiles of the x passes
+    size_t phys_count = 0, phys_asked = 0;
+    std::vector<void *> kept;     // smaller buffers from before: captured graphs may hold them
+    size_t kept_bytes = 0;
+    size_t tiles(int n) const { return std::min(ws_bytes / ((size_t)dims(n).ks.all() * kAStage), expo_count / kLanes); }
 };
 
 namespace {
@@ -1059,6 +1063,11 @@ TcState *state(Plan &P) {
 
 }  // namespace
 
+static bool capturing(const Plan &P) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(P.stream, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+}
+
 bool tc_length_ok(int n) { return n >= 32 && n <= kMaxLen && n % 2 == 0; }
 
 void tc_job_set(TcJob &j, const TcSet *s) {
@@ -1075,6 +1084,9 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     const std::pair<int, double> key(half ? -n : n, factor);
     auto it = S->sets.find(key);
     if (it != S->sets.end()) return &it->second;
+    *status = kNoFast;  // without memory for the tables, or where none may be allocated
+    if (capturing(P)) return nullptr;
+    *status = OK;
     const Dims D = dims(n);
     TcSet set;
     MatrixDigits M;
@@ -1094,8 +1106,7 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     if (cudaMalloc(&set.mat, set.bytes) != cudaSuccess || cudaMalloc(&dig, h.size() * 2) != cudaSuccess) {
         cudaGetLastError();
         if (set.mat) cudaFree(set.mat);
-        set_error("out of device memory (digit tables)");
-        *status = ERR_OOM;
+        *status = kNoFast;
         return nullptr;
     }
     cudaMemcpyAsync(dig, h.data(), h.size() * 2, cudaMemcpyHostToDevice, P.stream);
@@ -1111,34 +1122,61 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     return &(S->sets[key] = set);
 }
 
-// The digit workspace of a plan has one size for its lifetime (captured graphs hold its address):
-// what its largest axis needs for all its columns, at most 2 GiB; longer launches run in ranges of tiles.
-static int workspace(Plan &P) {
-    TcState *S = state(P);
-    if (S->ws) return OK;
-    size_t want = 0, tiles = 0;
-    const int len[3] = {P.nz, P.ny, P.nx}, jobs[3] = {kTcMaxJobs, kTcMaxJobs, kTcMaxJobs};
+// Room for digits, sized for what the plan's calls use: plans that run single transforms (conversions, output) hold the
+// digits of one, those that run the nonlinear term those of its launches, both up to a limit beyond which launches
+// run in ranges of tiles.  Buffers keep their addresses: one that has become too small stays until the plan's
+// end, for graphs that hold it.
+// The limit, MiB, against an RK2 step of convection, ms: 512^2 x 513 2048: 235, 1024: 240, 512: 249, 128: 312; 256^2 x 257
+// 25.1, 25.7, 27.9, 35.4; 128^2 x 129 (701 MB at most) 4.08, 4.08, 4.09, 4.86.
+constexpr size_t kRoomMiB = 2048;
+
+// bytes and lanes of digits for launches of up to `jobs` transforms (1 or more), in `most` bytes if 16 tiles fit them
+static void room_for(const Plan &P, int jobs, size_t most, size_t *bytes, size_t *lanes) {
+    const int len[3] = {P.nz, P.ny, P.nx}, many[3] = {8, 8, 15};  // of the z and y passes and of the nonlinear x pass
     const size_t cols[3] = {((size_t)P.ny * P.ldx + 63) / 64, ((size_t)P.nz * P.ldx + 63) / 64,
                             ((size_t)P.nz * P.ny + kLanes - 1) / kLanes};
+    *bytes = *lanes = 0;
     for (int i = 0; i < 3; i++) {
         if (!tc_length_ok(len[i])) continue;
         const size_t per = (size_t)dims(len[i]).ks.all() * kAStage;
-        size_t t = cols[i] * jobs[i];
-        t = std::min(t, std::max<size_t>((2ull << 30) / per, kTcMaxJobs));
-        want = std::max(want, t * per);
-        tiles = std::max(tiles, t);
+        const size_t t = std::min(cols[i] * (jobs > 1 ? many[i] : 1), std::max<size_t>(most / per, kTcMaxJobs));
+        *bytes = std::max(*bytes, t * per);
+        *lanes = std::max(*lanes, t * kLanes);
     }
-    if (cudaMalloc(&S->ws, want) != cudaSuccess || cudaMalloc(&S->expo, tiles * kLanes * sizeof(int)) != cudaSuccess) {
+}
+
+// kNoFast: there is no memory for it, or it would have to be allocated during a capture (the general engine needs
+// none)
+static int room(Plan &P, int jobs) {
+    TcState *S = state(P);
+    jobs = jobs > 1 ? kTcMaxJobs : 1;
+    if (P.digit_room_mb < 0) return kNoFast;
+    if (S->ws_jobs >= jobs) return OK;
+    if (capturing(P)) return S->ws ? OK : kNoFast;
+    size_t last = 0;
+    for (size_t most = (size_t)(P.digit_room_mb ? P.digit_room_mb : kRoomMiB) << 20;; most /= 2) {
+        size_t bytes, lanes;
+        room_for(P, jobs, most, &bytes, &lanes);
+        if (bytes == last || (bytes <= S->ws_bytes && lanes <= S->expo_count)) break;  // no smaller, or no gain
+        last = bytes;
+        void *ws = nullptr, *expo = nullptr;
+        if (cudaMalloc(&ws, bytes) == cudaSuccess && cudaMalloc(&expo, lanes * sizeof(int)) == cudaSuccess) {
+            if (S->ws) {
+                S->kept.push_back(S->ws);
+                S->kept.push_back(S->expo);
+                S->kept_bytes += S->ws_bytes + S->expo_count * sizeof(int);
+            }
+            S->ws = (unsigned char *)ws;
+            S->ws_bytes = bytes;
+            S->expo = (int *)expo;
+            S->expo_count = lanes;
+            break;
+        }
         cudaGetLastError();
-        if (S->ws) cudaFree(S->ws);
-        if (S->expo) cudaFree(S->expo);
-        S->ws = nullptr;
-        S->expo = nullptr;
-        set_error("out of device memory (digit workspace)");
-        return ERR_OOM;
+        if (ws) cudaFree(ws);
     }
-    S->ws_bytes = want;
-    S->expo_count = tiles * kLanes;
+    if (!S->ws) return kNoFast;
+    S->ws_jobs = jobs;  // as much of it as there is
     return OK;
 }
 
@@ -1220,14 +1258,12 @@ K with_smem(K k, size_t bytes) {
 }  // namespace
 
 int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes) {
-    if (int st = workspace(P)) return st;
-    if (int st = tc_status(P)) return st;
-    TcState *S = P.tc;
+    SG_TRY(room(P, njobs));
+    SG_TRY(tc_status(P));
     const Dims D = dims(s.n);
     const size_t per = (size_t)D.ks.all() * kAStage;
     const unsigned tiles = (s.ncol + 63) / 64;
-    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
-    const TcRange range = tc_range(njobs, tiles, cap);
+    const TcRange range = tc_range(njobs, tiles, P.tc->tiles(s.n));
     const int lw = digit_lanes(s.n);
     const size_t dsm = (size_t)s.n * lw * 8;
     for (int j0 = 0; j0 < njobs; j0 += range.jobs)
@@ -1252,21 +1288,31 @@ int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *
     return check_launch(name);
 }
 
-// Buffer of physical rows in tiles ([field][tile][x][128 rows]), sized for the 15 fields of the nonlinear
-// term's x pass over one range of tiles; its address is fixed like the digits'.
-static int phys_rows(Plan &P) {
+// Buffer of physical rows in tiles ([field][tile][x][128 rows]) for one range of tiles: one field's, or the 15 of the
+// nonlinear term's x pass.
+static int phys_rows(Plan &P, int fields) {
     TcState *S = P.tc;
-    if (S->phys) return OK;
-    const size_t per = (size_t)dims(P.nx).ks.all() * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
-    const size_t all = ((size_t)P.nzp * P.ny + kLanes - 1) / kLanes, t = std::min(all, std::max<size_t>(cap / kTcMaxJobs, 1));
-    if (cudaMalloc(&S->phys, t * 15 * P.nx * kLanes * sizeof(double)) != cudaSuccess) {
+    const size_t cap = S->tiles(P.nx), all = ((size_t)P.nz * P.ny + kLanes - 1) / kLanes;
+    const size_t t = std::min(all, std::max<size_t>(fields > 1 ? cap / kTcMaxJobs : cap, 1));
+    const size_t one = (size_t)fields * P.nx * kLanes, want = t * one;
+    if (want <= S->phys_asked || capturing(P)) return S->phys_count >= one ? OK : kNoFast;
+    S->phys_asked = want;
+    double *m = nullptr;
+    size_t n = want;
+    while (n > S->phys_count && n >= one && cudaMalloc(&m, n * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
-        S->phys = nullptr;
-        set_error("out of device memory (physical rows)");
-        return ERR_OOM;
+        m = nullptr;
+        n = n / 2 / one * one;
     }
-    S->phys_tiles = t;
-    return OK;
+    if (m) {
+        if (S->phys) {
+            S->kept.push_back(S->phys);
+            S->kept_bytes += S->phys_count * sizeof(double);
+        }
+        S->phys = m;
+        S->phys_count = n;
+    }
+    return S->phys_count >= one ? OK : kNoFast;
 }
 
 // gradre / advect between the y passes (pseudospec_hd.f90:209-319, pseudospec_phd.f90:23-113): the
@@ -1278,21 +1324,22 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
     void *const *out = x.out;
     const int c0 = x.c0, c1 = x.c1, nrows = x.nrows;
     const double scale = x.tmp;
-    if (int st = workspace(P)) return st;
-    if (int st = tc_status(P)) return st;
+    const int n = P.nx, nc = c1 - c0, nin = 3 + 3 * nc;
+    SG_TRY(room(P, nin));
+    SG_TRY(phys_rows(P, 15));
+    SG_TRY(tc_status(P));
     TcState *S = P.tc;
     int st = OK;
-    const int n = P.nx, nc = c1 - c0, nin = 3 + 3 * nc;
     const TcSet *inv = tc_set(P, n, 1.0, &st, true), *dinv = inv ? tc_set(P, n, P.Dkx, &st, true) : nullptr;
     const TcSet *fwd = dinv ? tc_set(P, n, 1.0, &st, false) : nullptr;
     if (!fwd) return st;
     const Dims D = dims(n);
     const size_t per = (size_t)D.ks.all() * kAStage, ptile = (size_t)n * kLanes;
-    const size_t cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
     const unsigned rows = (unsigned)nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
-    SG_TRY(phys_rows(P));
-    const unsigned tstep = tc_range(1, tiles, S->phys_tiles).tiles;
-    const size_t fstride = S->phys_tiles * ptile;
+    const size_t fit = std::min(S->tiles(n) / kTcMaxJobs, S->phys_count / (15 * ptile));
+    if (!fit) return kNoFast;
+    const unsigned tstep = tc_range(1, tiles, fit).tiles;
+    const size_t fstride = tstep * ptile;
     const int lw = digit_lanes(n);
     for (unsigned t0 = 0; t0 < tiles; t0 += tstep) {
         const unsigned nt = std::min(tstep, tiles - t0);
@@ -1414,17 +1461,17 @@ int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
 constexpr unsigned kFewRows = 16 * kLanes;
 int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
     if (!tc_length_ok(P.nx) || (P.nx < 96 && (unsigned)a.nrows * P.ny < kFewRows)) return kNoFast;
-    SG_TRY(workspace(P));
-    if (!r2c) SG_TRY(phys_rows(P));
+    SG_TRY(room(P, 1));
+    if (!r2c) SG_TRY(phys_rows(P, 1));
     SG_TRY(tc_status(P));
     TcState *S = P.tc;
     int st = OK;
     const TcSet *set = tc_set(P, P.nx, a.scale, &st, !r2c);
     if (!set) return st;
     const Dims D = dims(P.nx);
-    const size_t per = (size_t)D.ks.all() * kAStage, cap = std::min(S->ws_bytes / per, S->expo_count / kLanes);
+    const size_t per = (size_t)D.ks.all() * kAStage, cap = S->tiles(P.nx);
     const unsigned rows = (unsigned)a.nrows * P.ny, tiles = (rows + kLanes - 1) / kLanes;
-    const unsigned tstep = tc_range(1, tiles, r2c ? cap : std::min(cap, 15 * S->phys_tiles)).tiles;
+    const unsigned tstep = tc_range(1, tiles, r2c ? cap : std::min(cap, S->phys_count / ((size_t)P.nx * kLanes))).tiles;
     const int lw = digit_lanes(P.nx);
     const char *name = r2c ? "x_r2c" : "x_c2r";
     for (int f = 0; f < nf; f++)
@@ -1490,9 +1537,15 @@ int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes) {
     return tc_run(P, s, jobs, nj, a.sign < 0 ? "y_forward" : "y_inverse", bytes);
 }
 
+int tc_reserve(Plan &P) {
+    SG_TRY(room(P, kTcMaxJobs));
+    return tc_length_ok(P.nx) ? phys_rows(P, 15) : OK;
+}
+
 void tc_free(Plan &P) {
     if (!P.tc) return;
     for (auto &e : P.tc->sets) cudaFree(e.second.mat);
+    for (void *m : P.tc->kept) cudaFree(m);
     if (P.tc->ws) cudaFree(P.tc->ws);
     if (P.tc->expo) cudaFree(P.tc->expo);
     if (P.tc->phys) cudaFree(P.tc->phys);
@@ -1503,7 +1556,7 @@ void tc_free(Plan &P) {
 unsigned long long tc_bytes(const Plan &P) {
     if (!P.tc) return 0;
     unsigned long long b = P.tc->ws_bytes + P.tc->expo_count * sizeof(int);
-    b += (unsigned long long)P.tc->phys_tiles * 15 * P.nx * kLanes * sizeof(double);
+    b += P.tc->kept_bytes + P.tc->phys_count * sizeof(double);
     for (const auto &e : P.tc->sets) b += e.second.bytes;
     return b;
 }

@@ -44,12 +44,15 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half = fals
 void tc_job_set(TcJob &j, const TcSet *s);
 // complex columns
 int tc_run(Plan &P, const TcShape &s, const TcJob *jobs, int njobs, const char *name, double bytes);
-// the passes of kernels.cuh over these transforms; kNoFast (fast.h) for a form that they do not take
+// the passes of kernels.cuh over these transforms; kNoFast (fast.h) for a form that they do not take, and where
+// their buffers or tables are not there and cannot be allocated
 int tc_z_inverse(Plan &P, const ZInvArgs &a, int nf, double bytes);
 int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes);
 int tc_y(Plan &P, const YArgs &a, int nf, int nplanes, double bytes);
 int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes);
 int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes);
+// the buffers of a solver's stage, allocated; kNoFast when there is no memory for them
+int tc_reserve(Plan &P);
 void tc_free(Plan &P);
 unsigned long long tc_bytes(const Plan &P);
 // An error when a kernel of the plan gave up a wait: its results are wrong, and so may be whatever was made of

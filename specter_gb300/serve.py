@@ -113,9 +113,12 @@ class Server:
         self.policy = policy
         self.fill_points = fill_points
         self.per_field = {}  # solver kind -> device bytes per field-sized unit, measured
+        # before that; with the digits of its transforms an FP64 solver holds between 40 and 80 by its grid, so
+        # that the first grid's measurement says little about the next
+        self.fields, self.least = (48.0, 0.0) if precision else (80.0, 80.0)
 
     def _estimate(self, req):
-        return int(self.per_field.get(req.kind, 48.0) * field_bytes(req, self.precision))
+        return int(max(self.per_field.get(req.kind, self.fields), self.least) * field_bytes(req, self.precision))
 
     def _start(self, req, now):
         t_setup = time.perf_counter()

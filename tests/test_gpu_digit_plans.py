@@ -78,3 +78,97 @@ def test_gave_up_is_reported():
     api.set_option(p, "gave_up", 0)
     for c in calls.values():
         c()
+
+
+def room(p, mb):
+    api.set_option(p, "digit_room_mb", mb)
+    return p
+
+
+# Room for a few tiles of digits: the same launches in ranges of tiles, or one transform at a time, bit for bit.
+@pytest.mark.parametrize("nx,ny,nz", [(96, 40, 58), (34, 64, 90), (130, 34, 154)])
+def test_ranges(nx, ny, nz):
+    def run(p):
+        rng = np.random.default_rng(nx)
+        r = p.field(api.REAL, data=rng.standard_normal(p.rshape))
+        f = [p.field(data=rng.standard_normal(p.sshape) + 1j * rng.standard_normal(p.sshape)) for _ in range(4)]
+        o = [p.field() for _ in range(5)]
+        out = []
+        api.fftp3d_real_to_complex(p, r, o[4])
+        api.gradre(p, f[0], f[1], f[2], o[0], o[1], o[2])
+        api.advect(p, f[0], f[1], f[2], f[3], o[3])
+        out += [x.download() for x in o]
+        api.fftp3d_complex_to_real(p, o[4], r)
+        o[4].zero()
+        api.v_imposebc_and_project(p, f[0], f[1], f[2], o[4], 1, 2)
+        return out + [x.download() for x in f + [o[4]]] + [r.download()]
+
+    got, want = run(room(plan(nx, ny, nz), 2)), run(plan(nx, ny, nz))
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("kind", [api.HD, api.BOUSS, api.ROTBOUSS])
+def test_stage_ranges(kind):
+    def run(mb):
+        p = room(plan(96, 40, 90), mb)
+        s = api.Solver(p, kind, ord=2, dt=1e-4, nu=1e-3, kappa=1e-3, omega=(0.1, 0.0, 0.5))
+        rng = np.random.default_rng(1)
+        for f in s.state[:-1]:
+            r = p.field(api.REAL, data=1e-2 * rng.standard_normal(p.rshape))
+            api.fftp3d_real_to_complex(p, r, f)
+        s.step(2)
+        return [f.download() for f in s.state]
+
+    small, large, general = run(2), run(0), run(-1)
+    assert all(np.array_equal(a, b) for a, b in zip(small, large))
+    # against the column kernels on the general engine: rounding times 1e4 (the continuation)
+    assert all(np.linalg.norm(a - b) < 1e-11 * np.linalg.norm(b) for a, b in zip(small, general))
+
+
+# A plan that transforms fields one by one holds the digits of one, not those of the nonlinear term.
+def test_memory_of_single_transforms():
+    p = plan(128, 128, 154)
+    r, c = p.field(api.REAL), p.field()
+    p.synchronize()
+    free = api.device_memory()[0]
+    api.fftp3d_complex_to_real(p, c, r)
+    p.synchronize()
+    assert free - api.device_memory()[0] < 8 * 16 * 72 * 128 * 154
+
+
+# The first transform of a plan inside a stream capture, where nothing can be allocated, and one after it.
+@pytest.mark.parametrize("before", [False, True])
+def test_first_call_captured(before):
+    import torch
+    w = room(plan(16, 4, 58), -1)
+    api.fftp1d_complex_to_real_z(w, w.field())  # its kernel is loaded
+    p = plan(16, 4, 58)
+    rng = np.random.default_rng(2)
+    a = rng.standard_normal(p.sshape) + 1j * rng.standard_normal(p.sshape)
+    f, src = p.field(data=a), p.field(data=a)
+    if before:
+        api.fftp1d_complex_to_real_z(p, f)
+    p.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(p.stream)):
+        f.copy_from(src)
+        api.fftp1d_complex_to_real_z(p, f)
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        want = np.fft.ifft(a, axis=-1) * 58
+        assert np.linalg.norm(f.download() - want) < 2e-15 * np.linalg.norm(want)
+
+
+# What the server reserves for an FP64 request before it has seen one of its kind.
+def test_server_estimate():
+    from specter_gb300 import serve
+    srv = serve.Server(1, precision=0)
+    for kind, nx, ny, nzp in (("HD", 64, 64, 65), ("BOUSS", 128, 64, 129), ("BOUSS", 128, 128, 65), ("HD", 256, 64, 257)):
+        req = serve.Request(0, 0.0, kind, nx, ny, nzp, 1, 1)
+        p, s = serve.make(srv.api, srv.initial, req, 0)
+        s.step(1)
+        p.synchronize()
+        assert api.solver_memory(s) <= srv._estimate(req)
+        s.close()
+        p.close()
