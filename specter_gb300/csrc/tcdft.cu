@@ -60,7 +60,6 @@ enum { kCol = 0, kR2C = 1, kC2R = 2 };
 
 struct TcSet {
     unsigned char *mat = nullptr;
-    size_t bytes = 0;
     int expo = 0;
     double post = 1.0;
     float top[2] = {0.f, 0.f};
@@ -71,12 +70,14 @@ struct TcState {
     unsigned char *ws = nullptr;  // digits
     size_t ws_bytes = 0;
     int ws_jobs = 0;              // of launches of that many transforms
-    int *expo = nullptr;          // column exponents of the digits in ws
+    int *expo = nullptr;          // column exponents of the digits in ws (behind them)
     size_t expo_count = 0;
     double *phys = nullptr;       // physical rows in tiles, of one range of tiles of the x passes
     size_t phys_count = 0, phys_asked = 0;
-    std::vector<void *> kept;     // smaller buffers from before: captured graphs may hold them
+    std::vector<void *> kept;     // tables; and smaller buffers from before, which captured graphs may hold
     size_t kept_bytes = 0;
+    unsigned char *slab = nullptr;  // what is left of the tables' latest block (in kept)
+    size_t slab_left = 0;
     size_t tiles(int n) const { return std::min(ws_bytes / ((size_t)dims(n).ks.all() * kAStage), expo_count / kLanes); }
 };
 
@@ -1034,8 +1035,14 @@ __global__ void __launch_bounds__(256) k_untile(const double *tiles, double *out
 }
 
 // ------------------------------------------------------------------ tables
-// digits [angle][7] of factor * cos, factor * sin at 2 pi t / n -> the matrices of one set
-__global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, int K, Steps ks, int nq0, int nq1, int nchunk,
+// Digits [cos, sin][angle][7] of factor * cos and factor * sin at 2 pi t / n, as an argument of the kernel: a copy
+// would have to wait for the stream or for the host's memory.
+struct AngleDigits {
+    short d[2 * kMaxLen * kDig];
+};
+static_assert(sizeof(AngleDigits) < 32000, "kernel arguments");
+// -> the matrices of one set
+__global__ void k_fill_mat(__nv_bfloat16 *mat, const __grid_constant__ AngleDigits dig, int n, int K, Steps ks, int nq0, int nq1, int nchunk,
                            int nc, int half) {
     const long long total = (long long)nchunk * ks.all() * 16 * nc;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
@@ -1052,7 +1059,8 @@ __global__ void k_fill_mat(__nv_bfloat16 *mat, const __nv_bfloat16 *dig, int n, 
         const int ang = on ? (int)((long long)(2 * fq + par) * pt % n) : 0;
         __nv_bfloat16 *dst = mat + (long long)t * (kDig * 16 * nc) + (kk / 8) * (nc * 8) + col * 8 + kk % 8;
         for (int i = 0; i < kDig; i++)
-            dst[(long long)i * nc * 16] = on ? dig[((long long)list * n + ang) * kDig + i] : __float2bfloat16(0.f);
+            dst[(long long)i * nc * 16] = __float2bfloat16(
+                on ? (float)dig.d[((long long)list * n + ang) * kDig + i] * __uint_as_float((unsigned)(127 - 9 * i) << 23) : 0.f);
     }
 }
 
@@ -1078,6 +1086,27 @@ void tc_job_set(TcJob &j, const TcSet *s) {
     j.top[1] = s->top[1];
 }
 
+// Device memory of tables, cut from blocks: an allocation takes as long as a short transform.
+static unsigned char *table_memory(TcState *S, size_t bytes) {
+    bytes = (bytes + 255) / 256 * 256;
+    if (S->slab_left < bytes) {
+        const size_t block = std::max<size_t>(bytes, 256 * 1024);
+        void *m = nullptr;
+        if (cudaMalloc(&m, block) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        S->kept.push_back(m);
+        S->kept_bytes += block;
+        S->slab = (unsigned char *)m;
+        S->slab_left = block;
+    }
+    unsigned char *p = S->slab;
+    S->slab += bytes;
+    S->slab_left -= bytes;
+    return p;
+}
+
 const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     *status = OK;
     TcState *S = state(P);
@@ -1095,30 +1124,19 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     set.post = M.post;
     set.top[0] = M.top[0];
     set.top[1] = M.top[1];
-    std::vector<__nv_bfloat16> h(2 * (size_t)n * kDig);
-    for (int l = 0; l < 2; l++)
-        for (size_t q = 0; q < (size_t)n * kDig; q++) {
-            const int i = (int)(q % kDig);
-            h[(size_t)l * n * kDig + q] = __float2bfloat16(ldexpf((float)(l ? M.s[q] : M.c[q]), -9 * i));
-        }
-    set.bytes = (size_t)D.nchunk * D.ks.all() * kDig * 32 * D.nc;
-    __nv_bfloat16 *dig = nullptr;
-    if (cudaMalloc(&set.mat, set.bytes) != cudaSuccess || cudaMalloc(&dig, h.size() * 2) != cudaSuccess) {
-        cudaGetLastError();
-        if (set.mat) cudaFree(set.mat);
+    AngleDigits h;
+    for (size_t q = 0; q < (size_t)n * kDig; q++) {
+        h.d[q] = (short)M.c[q];
+        h.d[(size_t)n * kDig + q] = (short)M.s[q];
+    }
+    set.mat = table_memory(S, (size_t)D.nchunk * D.ks.all() * kDig * 32 * D.nc);
+    if (!set.mat) {
         *status = kNoFast;
         return nullptr;
     }
-    cudaMemcpyAsync(dig, h.data(), h.size() * 2, cudaMemcpyHostToDevice, P.stream);
-    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, dig, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc,
+    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, h, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc,
                                             half ? 1 : 0);
-    const cudaError_t e = cudaStreamSynchronize(P.stream);  // the host digits go out of scope
-    cudaFree(dig);
-    if (e != cudaSuccess || (*status = check_launch("digit tables"))) {
-        cudaFree(set.mat);
-        if (!*status) *status = ERR_CUDA;
-        return nullptr;
-    }
+    if ((*status = check_launch("digit tables"))) return nullptr;
     return &(S->sets[key] = set);
 }
 
@@ -1159,21 +1177,19 @@ static int room(Plan &P, int jobs) {
         room_for(P, jobs, most, &bytes, &lanes);
         if (bytes == last || (bytes <= S->ws_bytes && lanes <= S->expo_count)) break;  // no smaller, or no gain
         last = bytes;
-        void *ws = nullptr, *expo = nullptr;
-        if (cudaMalloc(&ws, bytes) == cudaSuccess && cudaMalloc(&expo, lanes * sizeof(int)) == cudaSuccess) {
+        void *ws = nullptr;
+        if (cudaMalloc(&ws, bytes + lanes * sizeof(int)) == cudaSuccess) {
             if (S->ws) {
                 S->kept.push_back(S->ws);
-                S->kept.push_back(S->expo);
                 S->kept_bytes += S->ws_bytes + S->expo_count * sizeof(int);
             }
             S->ws = (unsigned char *)ws;
             S->ws_bytes = bytes;
-            S->expo = (int *)expo;
+            S->expo = (int *)(S->ws + bytes);
             S->expo_count = lanes;
             break;
         }
         cudaGetLastError();
-        if (ws) cudaFree(ws);
     }
     if (!S->ws) return kNoFast;
     S->ws_jobs = jobs;  // as much of it as there is
@@ -1544,10 +1560,8 @@ int tc_reserve(Plan &P) {
 
 void tc_free(Plan &P) {
     if (!P.tc) return;
-    for (auto &e : P.tc->sets) cudaFree(e.second.mat);
     for (void *m : P.tc->kept) cudaFree(m);
     if (P.tc->ws) cudaFree(P.tc->ws);
-    if (P.tc->expo) cudaFree(P.tc->expo);
     if (P.tc->phys) cudaFree(P.tc->phys);
     delete P.tc;
     P.tc = nullptr;
@@ -1557,7 +1571,6 @@ unsigned long long tc_bytes(const Plan &P) {
     if (!P.tc) return 0;
     unsigned long long b = P.tc->ws_bytes + P.tc->expo_count * sizeof(int);
     b += P.tc->kept_bytes + P.tc->phys_count * sizeof(double);
-    for (const auto &e : P.tc->sets) b += e.second.bytes;
     return b;
 }
 

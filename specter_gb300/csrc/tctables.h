@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
-#include <map>
 #include <utility>
 #include <vector>
 
@@ -53,17 +52,17 @@ inline void circle(int n, std::vector<long double> &c, std::vector<long double> 
     const long double pi = 3.14159265358979323846264338327950288L;
     c.assign(n, 0.0L);
     s.assign(n, 0.0L);
-    std::map<int, std::pair<long double, long double>> cache;  // by 8 t / n folded into the first octant
+    std::vector<std::pair<long double, long double>> cache(n + 1, {2.0L, 0.0L});  // by 8 t / n folded into the first octant
     for (int t = 0; t < n; t++) {
         // angle = 2 pi t / n = (pi / 4) (8 t / n): octant o and remainder u = 8 t - o n, in units of pi / (4 n)
         const int o = 8 * t / n, u = 8 * t - o * n;
         const int v = o & 1 ? n - u : u;
-        auto it = cache.find(v);
-        if (it == cache.end()) {
+        auto &it = cache[v];
+        if (it.first > 1.0L) {
             const long double x = pi * (long double)v / (4.0L * (long double)n);
-            it = cache.insert({v, {cosl(x), sinl(x)}}).first;
+            it = {cosl(x), sinl(x)};
         }
-        long double a = it->second.first, b = it->second.second;
+        long double a = it.first, b = it.second;
         switch (o) {
             case 0: break;
             case 1: std::swap(a, b); break;
@@ -92,30 +91,37 @@ inline void matrix_digits(long double v, int d[kDig]) {
 // matrix.  The largest absolute sum of the products, over the outputs, that any data digits (|d| <= 256) can make:
 // every partial sum in any order is below it.  For levels 2, 3 and 4 (those above are in all of them).
 inline void level_bounds(const Dims &D, bool half, const std::vector<int> &dc, const std::vector<int> &ds, long long b[3]) {
-    b[0] = b[1] = b[2] = 0;
-    for (int list = 0; list < 2; list++) {
-        const std::vector<int> &d = list ? ds : dc;
-        for (int v = 2; v <= 4; v++) {
-            std::vector<int> a(D.n, 0);
-            for (int t = 0; t < D.n; t++)
-                for (int i = 0; i <= v; i++) a[t] += std::abs(d[(size_t)t * kDig + i]);
-            for (int par = 0; par < 2; par++) {
-                const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
-                for (int o = 0; o < no; o++) {
-                    // angles (2 f + par) * point: advance by a fixed step from one input to the next
-                    const int step = half ? 2 * o % D.n : (2 * o + par) % D.n;
-                    int ang = half ? par * o % D.n : 0;
-                    long long sum = 0;
-                    for (int i = 0; i < ni; i++) {
-                        sum += a[ang];
-                        ang += step;
-                        if (ang >= D.n) ang -= D.n;
-                    }
-                    b[v - 2] = std::max(b[v - 2], 256 * sum);
+    struct Sums {
+        int v[3];
+    };
+    std::vector<Sums> a(D.n);
+    long long most[3] = {0, 0, 0};
+    for (const std::vector<int> *d : {&dc, &ds}) {
+        for (int t = 0; t < D.n; t++) {
+            const int *q = d->data() + (size_t)t * kDig;
+            const int two = std::abs(q[0]) + std::abs(q[1]) + std::abs(q[2]), three = two + std::abs(q[3]);
+            a[t] = {{two, three, three + std::abs(q[4])}};
+        }
+        for (int par = 0; par < 2; par++) {
+            const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
+            for (int o = 0; o < no; o++) {
+                // angles (2 f + par) * point: advance by a fixed step from one input to the next
+                const int step = half ? 2 * o % D.n : (2 * o + par) % D.n;
+                int ang = half ? par * o % D.n : 0, s0 = 0, s1 = 0, s2 = 0;
+                for (int i = 0; i < ni; i++) {
+                    s0 += a[ang].v[0];
+                    s1 += a[ang].v[1];
+                    s2 += a[ang].v[2];
+                    ang += step;
+                    if (ang >= D.n) ang -= D.n;
                 }
+                most[0] = std::max<long long>(most[0], s0);
+                most[1] = std::max<long long>(most[1], s1);
+                most[2] = std::max<long long>(most[2], s2);
             }
         }
     }
+    for (int v = 0; v < 3; v++) b[v] = 256 * most[v];
 }
 
 // The digits of one matrix set and what of it the sums can trust.
@@ -148,8 +154,10 @@ inline bool matrix_digits_for(const Dims &D, double factor, bool half, MatrixDig
         }
         m.expo = t < 4 ? ex + t : 0;
         m.post = t < 4 ? 1.0 : factor;
-        long long b[3];
-        level_bounds(D, half, m.c, m.s, b);
+        // no digits pass 2^24 in short lists
+        const long long any = 256 * 256 * (long long)D.K;
+        long long b[3] = {3 * any, 4 * any, 5 * any};
+        if (b[2] > 1 << 24) level_bounds(D, half, m.c, m.s, b);
         if (b[0] > 1 << 24) continue;
         bool ok = true;
         for (int v = 0; v < 2; v++) {

@@ -172,3 +172,20 @@ def test_server_estimate():
         assert api.solver_memory(s) <= srv._estimate(req)
         s.close()
         p.close()
+
+
+# A plan's first transform is queued like the others: its tables wait for nothing that is queued before them.
+def test_first_call_does_not_wait():
+    import torch
+    w, p = plan(64, 64, 90), plan(64, 64, 90)
+    for q in (w, p):
+        f = q.field()
+        q.synchronize()
+        e = torch.cuda.Event()
+        with torch.cuda.stream(torch.cuda.ExternalStream(q.stream)):
+            torch.cuda._sleep(400_000_000)  # 0.2 s
+            e.record()
+        api.fftp1d_real_to_complex_z(q, f)
+        done = e.query()  # of the second plan, whose kernels are loaded
+        q.synchronize()
+    assert not done
