@@ -1035,14 +1035,13 @@ __global__ void __launch_bounds__(256) k_untile(const double *tiles, double *out
 }
 
 // ------------------------------------------------------------------ tables
-// Digits [cos, sin][angle][7] of factor * cos and factor * sin at 2 pi t / n, as an argument of the kernel: a copy
-// would have to wait for the stream or for the host's memory.
-struct AngleDigits {
-    short d[2 * kMaxLen * kDig];
+// The first quadrant's cosines and sines of one set (MatrixDigits), as an argument of the kernel: a copy would have to
+// wait for the stream or for the host's memory.
+struct QuadrantArg {
+    long long v[2][kMaxLen / 4 + 1];
 };
-static_assert(sizeof(AngleDigits) < 32000, "kernel arguments");
-// -> the matrices of one set
-__global__ void k_fill_mat(__nv_bfloat16 *mat, const __grid_constant__ AngleDigits dig, int n, int K, Steps ks, int nq0, int nq1, int nchunk,
+// -> the matrices of the set
+__global__ void k_fill_mat(__nv_bfloat16 *mat, const __grid_constant__ QuadrantArg quad, int n, int K, Steps ks, int nq0, int nq1, int nchunk,
                            int nc, int half) {
     const long long total = (long long)nchunk * ks.all() * 16 * nc;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total; q += (long long)gridDim.x * blockDim.x) {
@@ -1056,11 +1055,12 @@ __global__ void k_fill_mat(__nv_bfloat16 *mat, const __grid_constant__ AngleDigi
         // the K side runs over points and the N side over frequencies, the other way about for half spectra
         const int pt = half ? j : k, fq = half ? k : j;
         const bool on = pt < K && fq < (par ? nq1 : nq0);
-        const int ang = on ? (int)((long long)(2 * fq + par) * pt % n) : 0;
+        const Folded f = fold_angle(n, on ? (int)((long long)(2 * fq + par) * pt % n) : 0);
+        const long long v = !on ? 0 : list ? f.ss * quad.v[1][f.t] : f.cs * quad.v[0][f.t];
         __nv_bfloat16 *dst = mat + (long long)t * (kDig * 16 * nc) + (kk / 8) * (nc * 8) + col * 8 + kk % 8;
+#pragma unroll
         for (int i = 0; i < kDig; i++)
-            dst[(long long)i * nc * 16] = __float2bfloat16(
-                on ? (float)dig.d[((long long)list * n + ang) * kDig + i] * __uint_as_float((unsigned)(127 - 9 * i) << 23) : 0.f);
+            dst[(long long)i * nc * 16] = __float2bfloat16((float)matrix_digit(v, i) * __uint_as_float((unsigned)(127 - 9 * i) << 23));
     }
 }
 
@@ -1124,11 +1124,9 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
     set.post = M.post;
     set.top[0] = M.top[0];
     set.top[1] = M.top[1];
-    AngleDigits h;
-    for (size_t q = 0; q < (size_t)n * kDig; q++) {
-        h.d[q] = (short)M.c[q];
-        h.d[(size_t)n * kDig + q] = (short)M.s[q];
-    }
+    QuadrantArg h;
+    std::copy(M.c.begin(), M.c.end(), h.v[0]);
+    std::copy(M.s.begin(), M.s.end(), h.v[1]);
     set.mat = table_memory(S, (size_t)D.nchunk * D.ks.all() * kDig * 32 * D.nc);
     if (!set.mat) {
         *status = kNoFast;

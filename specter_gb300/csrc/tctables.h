@@ -47,60 +47,68 @@ inline Dims dims(int n) {
     return d;
 }
 
-// cos and sin of 2 pi t / n for every t from one octant, in long double
-inline void circle(int n, std::vector<long double> &c, std::vector<long double> &s) {
+// cos and sin of 2 pi t / n for the first quadrant, t = 0 .. n / 4, in long double
+inline void quadrant(int n, std::vector<long double> &c, std::vector<long double> &s) {
     const long double pi = 3.14159265358979323846264338327950288L;
-    c.assign(n, 0.0L);
-    s.assign(n, 0.0L);
-    std::vector<std::pair<long double, long double>> cache(n + 1, {2.0L, 0.0L});  // by 8 t / n folded into the first octant
-    for (int t = 0; t < n; t++) {
-        // angle = 2 pi t / n = (pi / 4) (8 t / n): octant o and remainder u = 8 t - o n, in units of pi / (4 n)
-        const int o = 8 * t / n, u = 8 * t - o * n;
-        const int v = o & 1 ? n - u : u;
-        auto &it = cache[v];
-        if (it.first > 1.0L) {
-            const long double x = pi * (long double)v / (4.0L * (long double)n);
-            it = {cosl(x), sinl(x)};
-        }
-        long double a = it.first, b = it.second;
-        switch (o) {
-            case 0: break;
-            case 1: std::swap(a, b); break;
-            case 2: { const long double w = a; a = -b; b = w; break; }
-            case 3: a = -a; break;
-            case 4: a = -a; b = -b; break;
-            case 5: { const long double w = a; a = -b; b = -w; break; }
-            case 6: { const long double w = a; a = b; b = -w; break; }
-            default: b = -b; break;
-        }
-        c[t] = a;
-        s[t] = b;
+    c.resize(n / 4 + 1);
+    s.resize(n / 4 + 1);
+    for (int t = 0; t <= n / 4; t++) {
+        const bool first = 8 * t <= n;  // octant; the second from the angle's complement
+        const long double x = pi * (long double)(first ? 4 * t : n - 4 * t) / (2.0L * (long double)n);
+        c[t] = first ? cosl(x) : sinl(x);
+        s[t] = first ? sinl(x) : cosl(x);
     }
 }
 
-inline void matrix_digits(long double v, int d[kDig]) {
-    const long long V = llrintl(v * 4611686018427387904.0L);  // 2^62
-    unsigned long long bias = 0;
-    for (int i = 1; i < kDig; i++) bias += 256ull << (54 - 9 * i);
-    const unsigned long long w = (unsigned long long)V + bias;
-    d[0] = (int)((long long)w >> 54);
-    for (int i = 1; i < kDig; i++) d[i] = (int)((w >> (54 - 9 * i)) & 511) - 256;
+// the angle t of 0 .. n - 1 by one of the first quadrant (n even): cos = cs * cos, sin = ss * sin
+struct Folded {
+    int t, cs, ss;
+};
+SG_BOTH inline Folded fold_angle(int n, int t) {
+    Folded f = {t, 1, 1};
+    if (2 * f.t > n) f = {n - f.t, 1, -1};
+    if (4 * f.t > n) f = {n / 2 - f.t, -1, f.ss};
+    return f;
 }
+
+// digit i of a number in units of 2^-62: signed, in -256 .. 255 but for digit 0
+SG_BOTH inline int matrix_digit(long long v, int i) {
+    unsigned long long bias = 0;
+    for (int k = 1; k < kDig; k++) bias += 256ull << (54 - 9 * k);
+    const unsigned long long w = (unsigned long long)v + bias;
+    return i ? (int)((w >> (54 - 9 * i)) & 511) - 256 : (int)((long long)w >> 54);
+}
+
+// The matrices of one set: cosines and sines times a scale, in units of 2^-62 ...
+struct MatrixDigits {
+    std::vector<long long> c, s;  // of the first quadrant
+    int expo = 0;                 // ... times 2^expo
+    double post = 1.0;            // and times this after the products (1: none)
+    // A sum of level 3 or 4 whose result is below this is exact in FP32, whatever the order of its terms:
+    // had a partial sum passed 2^24, what is left of the bound could not have brought it back below.
+    float top[2] = {0.f, 0.f};
+    int digit(int n, bool sine, int t, int i) const {
+        const Folded f = fold_angle(n, t);
+        return matrix_digit(sine ? f.ss * s[f.t] : f.cs * c[f.t], i);
+    }
+};
 
 // Level v of an output is the sum over the list of the products of digit i of the data and digit v - i of the
 // matrix.  The largest absolute sum of the products, over the outputs, that any data digits (|d| <= 256) can make:
 // every partial sum in any order is below it.  For levels 2, 3 and 4 (those above are in all of them).
-inline void level_bounds(const Dims &D, bool half, const std::vector<int> &dc, const std::vector<int> &ds, long long b[3]) {
+inline void level_bounds(const Dims &D, bool half, const MatrixDigits &m, long long b[3]) {
     struct Sums {
         int v[3];
     };
     std::vector<Sums> a(D.n);
     long long most[3] = {0, 0, 0};
-    for (const std::vector<int> *d : {&dc, &ds}) {
+    for (int sine = 0; sine < 2; sine++) {
         for (int t = 0; t < D.n; t++) {
-            const int *q = d->data() + (size_t)t * kDig;
-            const int two = std::abs(q[0]) + std::abs(q[1]) + std::abs(q[2]), three = two + std::abs(q[3]);
-            a[t] = {{two, three, three + std::abs(q[4])}};
+            int sum = 0;
+            for (int i = 0; i < 5; i++) {
+                sum += std::abs(m.digit(D.n, sine, t, i));
+                if (i >= 2) a[t].v[i - 2] = sum;
+            }
         }
         for (int par = 0; par < 2; par++) {
             const int no = half ? D.K : D.nq[par], ni = half ? D.nq[par] : D.K;
@@ -124,40 +132,30 @@ inline void level_bounds(const Dims &D, bool half, const std::vector<int> &dc, c
     for (int v = 0; v < 3; v++) b[v] = 256 * most[v];
 }
 
-// The digits of one matrix set and what of it the sums can trust.
-struct MatrixDigits {
-    std::vector<int> c, s;  // [angle][kDig] of the cosines, of the sines
-    int expo = 0;           // times 2^expo
-    double post = 1.0;      // and times this after the products (1: none)
-    // A sum of level 3 or 4 whose result is below this is exact in FP32, whatever the order of its terms:
-    // had a partial sum passed 2^24, what is left of the bound could not have brought it back below.
-    float top[2] = {0.f, 0.f};
-};
-
 // factor = scale * 2^expo with scale in (1/2, 1]: the matrices hold cosines and sines times scale.  A smaller scale
 // where those digits miss the bounds, and the plain matrices with a multiplication after them where all do.
 // Bounds: level 2 (and so 0 and 1) exact for any data; levels 3 and 4 trusted up to 2^22 at least, the size from
 // which the epilogue looks at them (join_levels).
 inline bool matrix_digits_for(const Dims &D, double factor, bool half, MatrixDigits &m) {
     std::vector<long double> c, s;
-    circle(D.n, c, s);
-    m.c.resize((size_t)D.n * kDig);
-    m.s.resize((size_t)D.n * kDig);
+    quadrant(D.n, c, s);
+    m.c.resize(c.size());
+    m.s.resize(s.size());
     int ex = 0;
     double fr = std::frexp(factor, &ex);
     if (fr == 0.5) { fr = 1.0; ex -= 1; }
     for (int t = 0; t < 5; t++) {
         const long double sc = t < 4 ? (long double)fr / (long double)(1 << t) : 1.0L;
-        for (int k = 0; k < D.n; k++) {
-            matrix_digits(c[k] * sc, &m.c[(size_t)k * kDig]);
-            matrix_digits(s[k] * sc, &m.s[(size_t)k * kDig]);
+        for (size_t k = 0; k < c.size(); k++) {
+            m.c[k] = llrintl(c[k] * sc * 4611686018427387904.0L);  // 2^62
+            m.s[k] = llrintl(s[k] * sc * 4611686018427387904.0L);
         }
         m.expo = t < 4 ? ex + t : 0;
         m.post = t < 4 ? 1.0 : factor;
         // no digits pass 2^24 in short lists
         const long long any = 256 * 256 * (long long)D.K;
         long long b[3] = {3 * any, 4 * any, 5 * any};
-        if (b[2] > 1 << 24) level_bounds(D, half, m.c, m.s, b);
+        if (b[2] > 1 << 24) level_bounds(D, half, m, b);
         if (b[0] > 1 << 24) continue;
         bool ok = true;
         for (int v = 0; v < 2; v++) {

@@ -14,8 +14,11 @@ extern "C" int digits(int n, double factor, int half, int *c, int *s, int *expo,
     const sg::Dims D = sg::dims(n);
     sg::MatrixDigits m;
     if (!sg::matrix_digits_for(D, factor, half, m)) return 1;
-    std::copy(m.c.begin(), m.c.end(), c);
-    std::copy(m.s.begin(), m.s.end(), s);
+    for (int t = 0; t < n; t++)
+        for (int i = 0; i < sg::kDig; i++) {
+            c[t * sg::kDig + i] = m.digit(n, false, t, i);
+            s[t * sg::kDig + i] = m.digit(n, true, t, i);
+        }
     *expo = m.expo;
     *post = m.post;
     top[0] = m.top[0];
