@@ -660,7 +660,10 @@ int specter_plan_tile_caps(specter_plan *plan, const int caps[4]) {
     CHECK_PLAN(plan);
     if (!caps) { set_error("null argument"); return SPECTER_ERR_ARG; }
     for (int i = 0; i < 4; i++)
-        if (caps[i] > 0) plan->p->tile_cap[i] = caps[i];
+        if (caps[i] > 0) {
+            plan->p->tile_cap[i] = caps[i];
+            plan->p->cap_asked[i] = true;
+        }
     return SPECTER_OK;
 }
 
@@ -689,6 +692,7 @@ int specter_plan_set_option(specter_plan *plan, const char *name, int value) {
         if (!strcmp(name, caps[i])) {
             if (value < 1 || value > 16 || (value & (value - 1))) { set_error("tile caps are powers of two in [1, 16]"); return SPECTER_ERR_ARG; }
             P.tile_cap[i] = value;
+            P.cap_asked[i] = true;
             return SPECTER_OK;
         }
     set_error(std::string("unknown plan option ") + name);
@@ -731,6 +735,7 @@ int specter_solver_autotune(specter_solver *s, int caps[5]) {
         cudaEventElapsedTime(&ms, e0, e1);
         return ms;
     };
+    for (bool &asked : P.cap_asked) asked = true;  // each cap is timed as the one that a caller would set
     for (int kind = 0; kind < 4; kind++) {
         int best = P.tile_cap[kind];
         float best_ms = trial();

@@ -7,6 +7,7 @@
 
 #include "fast.h"
 #include "smem.h"
+#include "xnlrows.h"
 
 namespace sg {
 namespace {
@@ -130,10 +131,8 @@ int xnl(Plan &P, const XNLArgs &a, double bytes) {
     // the production x lengths (H = 256, 128) at 8 rows run a copy with the row count fixed,
     // which takes the pipelined form (two FFT buffers, row-major staging: x_nl_pipe_elems)
     constexpr bool kFixed = L1 == 16 && (L2 == 16 || L2 == 8);
-    // 16 rows that leave one block on an SM (H = 256) are slower than that form at 8 rows and two
-    // blocks (512^2 x 513, four components: 8.2 against 6.1 ms); where 16 rows leave room for two (H = 128)
-    // they are the faster ones
-    if (kFixed && rb == 16 && !P.batch && x_nl_elems<E>(P.tx4.d, P.nxh, P.H, 16) * sizeof(float2) > kFastBudget) rb = 8;
+    if (!P.batch)
+        rb = xnl_rows(rb, kFixed, x_nl_elems<E>(P.tx4.d, P.nxh, P.H, 16) * sizeof(float2) <= kFastBudget, P.cap_asked[Plan::kTileX]);
     const bool fixed = kFixed && rb == 8;
     if (P.batch) {  // record for a batched launch (batch.h): the plain body
         const size_t smb = x_nl_elems<E>(P.tx4.d, P.nxh, P.H, rb) * sizeof(float2);

@@ -343,7 +343,10 @@ static int run_stage(Plan &P, FusedState *fs, int o, const void *const vin[4], c
     if (fs->nlp) {
         // nl_fp32: the nonlinear term in FP32 from an FP32 copy of the stage input
         Plan &Q = *fs->nlp;
-        for (int k = 0; k < 3; k++) Q.tile_cap[k] = P.tile_cap[k];  // the autotuned z, y, x caps
+        for (int k = 0; k < 3; k++) {  // the autotuned z, y, x caps
+            Q.tile_cap[k] = P.tile_cap[k];
+            Q.cap_asked[k] = P.cap_asked[k];
+        }
         const size_t n = P.field_elems();
         // float-float state: the FP32 z-inverse of the nonlinear term reads it directly (the rounded
         // sum of each pair); an FP64 state is narrowed into the FP32 copies first

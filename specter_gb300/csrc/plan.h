@@ -115,6 +115,7 @@ struct Plan {
     // column kernels), set by the autotuner; a launcher uses min(cap, largest width that fits).
     enum { kTileZ = 0, kTileY = 1, kTileX = 2, kTileFused = 3 };
     int tile_cap[4] = {16, 16, 16, 16};
+    bool cap_asked[4] = {false, false, false, false};  // set by the caller or the autotuner
     // fused velocity stage as two kernels (per-component update, then the projection) or one
     int velocity_split = 1;
     // threads per block of the float-float column kernels (nl_fp32 form) on the generic
