@@ -64,15 +64,17 @@ __global__ void k_narrow(const double2 *src, float2 *dst, size_t n) {
 
 // float-float <-> FP64 fields of the nl_fp32 form (in place allowed: both are 16 bytes a complex
 // element), once per field per fused_step call.  On the FP64 pipe a 512^2 x 538 field took 1.07 and
-// 0.80 ms; on the bit patterns the copy is bound by memory.  The ranges taken so hold every value whose
-// pair is within the normal floats; zeros are apart, and what is left goes through FP64 arithmetic.
+// 0.80 ms; on the bit patterns the copy is bound by memory.  Zeros are apart, and values beyond the ranges taken so
+// go through FP64 arithmetic.
 
 // the pair of a double: its value rounded to 24 bits, and the rounded rest
 __device__ __forceinline__ ff ff_of(double v) {
     const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
     const int e = (int)((h >> 20) & 0x7ff);
     const unsigned sign = h & 0x80000000u;
-    if (e >= 897 && e <= 1086) {  // 2^-126 <= |v| < 2^64
+    // 2^-97 <= |v| < 2^64: below, the rounded rest may have bits under the smallest denormal float and would be
+    // rounded twice
+    if (e >= 926 && e <= 1086) {
         const unsigned f = __funnelshift_l(l, h, 3) & 0x7fffffu, rest = l & 0x1fffffffu;
         const unsigned up = (rest + 0x0fffffffu + (f & 1u)) >> 29;  // to nearest, ties to even
         const unsigned hi = (((unsigned)(e - 896) << 23) | f) + up;
