@@ -1075,7 +1075,7 @@ int specter_batch_create(specter_solver *const *solvers, int n, specter_batch **
         set_error("out of device memory (batch records)");
         return SPECTER_ERR_OOM;
     }
-    cudaMemcpy(b->recs, host.data(), host.size(), cudaMemcpyHostToDevice);
+    upload(b->recs, host.data(), host.size());
     cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     // the shared-memory limit is a per-kernel attribute: set each kernel's largest use once (a
     // kernel appears at several positions with different tile sizes)

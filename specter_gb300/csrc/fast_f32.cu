@@ -94,7 +94,7 @@ int build_fft4_table(FFT4Table &t, int n, int axis) {
         }
     }
     if (cudaMalloc(&t.mem, h.size() * sizeof(float2)) != cudaSuccess) { set_error("cudaMalloc failed"); return ERR_OOM; }
-    cudaMemcpy(t.mem, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    upload(t.mem, h.data(), h.size() * sizeof(float2));
     float2 *b = (float2 *)t.mem;
     t.d.n = n; t.d.L = L; t.d.L1 = L1; t.d.L2 = L2; t.d.blue = blue;
     t.d.tw4 = b;

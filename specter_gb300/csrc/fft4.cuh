@@ -67,6 +67,7 @@ static inline cudaError_t fft4_init_tables() {
     cudaError_t e = cudaMemcpyToSymbol(c_regtw_f, hf, sizeof hf);
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_regtw_d, hd, sizeof hd);
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_regtw_q, hq, sizeof hq);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // as upload (plan.h)
     return e;
 }
 

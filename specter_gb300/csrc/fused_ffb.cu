@@ -65,7 +65,7 @@ int build_ffb_table(FFBTable &t, int n, int j0, int win) {
         set_error("cudaMalloc failed (float-float z tables)");
         return ERR_OOM;
     }
-    if (cudaMemcpy(t.mem, h.data(), (size_t)T::kBytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload(t.mem, h.data(), (size_t)T::kBytes) != cudaSuccess) {
         cudaFree(t.mem);
         t.mem = nullptr;
         return check_launch("float-float z tables");
@@ -85,7 +85,7 @@ int build_ffb_table(FFBTable &t, int n, int j0, int win) {
                 set_error("cudaMalloc failed (float-float window tables)");
                 return ERR_OOM;
             }
-            if (cudaMemcpy(t.zmem, z.data(), z.size() * sizeof(ffc), cudaMemcpyHostToDevice) != cudaSuccess) {
+            if (upload(t.zmem, z.data(), z.size() * sizeof(ffc)) != cudaSuccess) {
                 free_ffb_table(t);
                 return check_launch("float-float window tables");
             }

@@ -107,7 +107,7 @@ int build_fft_table(FFTTable &t, int n, Prec prec) {
         for (int k = 0; k < n; k++) P((size_t)L + k, chirp[k]);
     }
     if (cudaMalloc(&t.mem, h.size()) != cudaSuccess) return ERR_OOM;
-    cudaMemcpy(t.mem, h.data(), h.size(), cudaMemcpyHostToDevice);
+    upload(t.mem, h.data(), h.size());
     char *b = (char *)t.mem;
     d.tw = b;
     if (d.blue) {
@@ -256,15 +256,15 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
     size_t okx = app(p->kx), oky = app(p->ky), okz = app(p->kz), oz_ = app(p->z), odir = app(p->dir);
     size_t ofx = app(p->fx), ofy = app(p->fy), ofz = app(p->fz);
     if (cudaMalloc(&p->dgeo, g.size() * sizeof(double)) != cudaSuccess) { set_error("cudaMalloc failed"); delete p; return ERR_OOM; }
-    cudaMemcpy(p->dgeo, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice);
+    upload(p->dgeo, g.data(), g.size() * sizeof(double));
     {
         std::vector<float> gf(g.begin(), g.end());
         if (cudaMalloc(&p->dgeof, gf.size() * sizeof(float)) != cudaSuccess) { set_error("cudaMalloc failed"); plan_destroy(p); return ERR_OOM; }
-        cudaMemcpy(p->dgeof, gf.data(), gf.size() * sizeof(float), cudaMemcpyHostToDevice);
+        upload(p->dgeof, gf.data(), gf.size() * sizeof(float));
         std::vector<ff> gq(g.size());
         for (size_t i = 0; i < g.size(); i++) gq[i] = ff_split(g[i]);
         if (cudaMalloc(&p->dgeoq, gq.size() * sizeof(ff)) != cudaSuccess) { set_error("cudaMalloc failed"); plan_destroy(p); return ERR_OOM; }
-        cudaMemcpy(p->dgeoq, gq.data(), gq.size() * sizeof(ff), cudaMemcpyHostToDevice);
+        upload(p->dgeoq, gq.data(), gq.size() * sizeof(ff));
     }
     // R2C / C2R post-processing twiddles exp(-2*pi*i*k/nx), k = 0..H
     {
@@ -275,7 +275,7 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
             if (p->prec == FP64) put<double>(h, k * es, v); else put<float>(h, k * es, v);
         }
         cudaMalloc(&p->dxtw, h.size());
-        cudaMemcpy(p->dxtw, h.data(), h.size(), cudaMemcpyHostToDevice);
+        upload(p->dxtw, h.data(), h.size());
     }
     if ((st = build_fft_table(p->tx, p->H, p->prec)) || (st = build_fft_table(p->ty, ny, p->prec)) ||
         (st = build_fft_table(p->tz, nz, p->prec))) {
@@ -313,7 +313,7 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
                 }
             }
         if (cudaMalloc(&p->dlapc, lc.size() * sizeof(double)) != cudaSuccess) { set_error("cudaMalloc failed"); plan_destroy(p); return ERR_OOM; }
-        cudaMemcpy(p->dlapc, lc.data(), lc.size() * sizeof(double), cudaMemcpyHostToDevice);
+        upload(p->dlapc, lc.data(), lc.size() * sizeof(double));
         G.lapc = p->dlapc;
     }
     p->nred = 4096;
@@ -326,7 +326,7 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
             w[2 * k + 1] = (double)v.imag();
         }
         cudaMalloc(&p->dwtw, w.size() * sizeof(double));
-        cudaMemcpy(p->dwtw, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice);
+        upload(p->dwtw, w.data(), w.size() * sizeof(double));
         G.wtw = p->dwtw;
         std::vector<ff> wq(2 * (size_t)nz);  // (re, im) pairs of float-float: an ffc per k
         for (int k = 0; k < nz; k++) {
@@ -335,7 +335,7 @@ int plan_create(Plan **out, const int n[3], const int c[3], const int o[3], cons
             wq[2 * k + 1] = ff_split(v.imag());
         }
         cudaMalloc(&p->dwtwq, wq.size() * sizeof(ff));
-        cudaMemcpy(p->dwtwq, wq.data(), wq.size() * sizeof(ff), cudaMemcpyHostToDevice);
+        upload(p->dwtwq, wq.data(), wq.size() * sizeof(ff));
         G.wtwq = p->dwtwq;
     }
     cudaMallocHost(&p->hred, sizeof(double) * (p->nred + 1));

@@ -25,6 +25,13 @@ enum Status {
 
 void set_error(const std::string &msg);
 
+// Tables from host memory, there when this returns.  cudaMemcpy may return before a copy from pageable memory has
+// landed (up to 64 KB), and the plans' streams do not wait for the default stream that it is on.
+inline cudaError_t upload(void *dst, const void *src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 struct FFTTable {
     FFTDesc d{};
     void *mem = nullptr;  // one device allocation holding tw / chirp / filters
