@@ -18,9 +18,11 @@ __device__ __forceinline__ void chain_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+constexpr unsigned kSMs = 152;
+
 // Only launches of one wave gain; larger ones measured the same or up to 3 % slower (128^2 x 154 to physical
 // space, 126 -> 129 us), so they are ordinary launches.
-constexpr unsigned long long kChainBlocks = 3 * 152;
+constexpr unsigned long long kChainBlocks = 3 * kSMs;
 
 template <typename... P, typename... A>
 void chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {

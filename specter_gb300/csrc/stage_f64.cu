@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(128) k_stage_herm(Geo g, double2 *th) {
 
 int elem_blocks(const Plan &P) {
     const long long n = (long long)P.nz * P.ny * P.nxh, b = (n + 255) / 256;
-    return (int)(b > 152 * 16 ? 152 * 16 : b);
+    return (int)(b > kSMs * 16 ? kSMs * 16 : b);
 }
 
 }  // namespace

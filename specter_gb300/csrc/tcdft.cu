@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) k_digits(DigArgs a) {
 }
 
 // Real rows.  PROD: the rows are sums of products of physical rows in tiles [k][128 lanes] (the
-// nonlinear term: sum over i of phys[i] * phys[J.deriv + i], times scale); else they come from a
+// nonlinear term: sum over i of phys[i] * phys[J.prod + i], times scale); else they come from a
 // field's rows.
 template <int LW, bool PROD>
 __global__ void __launch_bounds__(kDigThreads, 4) k_digits_real(DigArgs a, const double *phys, size_t fstride, double scale) {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kDigThreads, 4) k_digits_real(DigArgs a, const
     double *dst = (double *)smem;
     if (PROD) {
         const int l = threadIdx.x % LW;
-        const double *u = phys + (size_t)lt * s.n * kLanes + lane0 + l, *d = u + J.deriv * fstride;
+        const double *u = phys + (size_t)lt * s.n * kLanes + lane0 + l, *d = u + J.prod * fstride;
 #pragma unroll 2
         for (int k = threadIdx.x / LW; k < s.n; k += kDigThreads / LW) {
             const size_t o = (size_t)k * kLanes;
@@ -1132,7 +1132,7 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
         *status = kNoFast;
         return nullptr;
     }
-    k_fill_mat<<<304, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, h, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc,
+    k_fill_mat<<<2 * kSMs, 256, 0, P.stream>>>((__nv_bfloat16 *)set.mat, h, n, D.K, D.ks, D.nq[0], D.nq[1], D.nchunk, D.nc,
                                             half ? 1 : 0);
     if ((*status = check_launch("digit tables"))) return nullptr;
     return &(S->sets[key] = set);
@@ -1239,7 +1239,7 @@ int digit_lanes(int n) { return n <= 300 ? 32 : 16; }
 int digit_split(const Dims &D, int lw, size_t blocks) {
     const int rounds = (2 * D.ks.first * lw + kDigThreads - 1) / kDigThreads;
     int split = 1;
-    while (split < rounds && blocks * split < 304) split++;
+    while (split < rounds && blocks * split < 2 * kSMs) split++;
     return split;
 }
 
@@ -1259,8 +1259,8 @@ void launch_gemm(Plan &P, const Dims &D, GemmArgs &g, int nj) {
     const auto k = kAdd && add ? (two ? k_gemm<MODE, kAdd, 2, false> : mark ? k_gemm<MODE, kAdd, 1, true> : k_gemm<MODE, kAdd, 1, false>)
                                : (two ? k_gemm<MODE, false, 2, false> : mark ? k_gemm<MODE, false, 1, true> : k_gemm<MODE, false, 1, false>);
     allow_smem(k, smem);
-    if (g.units <= 152) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
-    else k<<<152, kGemmBlock, smem, P.stream>>>(g);
+    if (g.units <= kSMs) chain(k, g.units, kGemmBlock, smem, P.stream, g);  // one unit a block
+    else k<<<kSMs, kGemmBlock, smem, P.stream>>>(g);
 }
 
 template <typename K>
@@ -1394,7 +1394,7 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
             TcJob &J = jobs[c];
             J = TcJob{};
             J.out = (double2 *)out[c0 + c] + (size_t)t0 * kLanes * P.ldx;
-            J.deriv = 3 + 3 * c;
+            J.prod = 3 + 3 * c;
             tc_job_set(J, fwd);
         }
         s.ls = 2 * P.ldx;

@@ -22,6 +22,7 @@ struct TcJob {
     const double2 *add;   // added to the result when not null (same layout as out)
     const unsigned char *mat;  // matrix digits of the table set
     int deriv, expo;      // expo: power of two of the set's factor
+    int prod;             // sums of products of physical rows: the first of the three derivatives' fields
     double post;          // further factor applied to the result (1: none)
     float top[2];         // sums of levels 3 and 4 that are smaller are exact (MatrixDigits)
 };
