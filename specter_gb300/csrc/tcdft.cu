@@ -181,12 +181,12 @@ __device__ __forceinline__ size_t col_offset(const TcShape &s, unsigned c) {
 constexpr int kEpiQ = 5;
 constexpr int kEpiThreads = 128 * kEpiQ, kLoadWarp = kEpiThreads / 32, kMmaWarp = kLoadWarp + 1;
 constexpr int kGemmBlock = kEpiThreads + 64;
-constexpr int kGemmSmem = 223 * 1024;  // dynamic shared memory: what the static arrays leave of 227 KB
+constexpr int kGemmSmem = 221 * 1024;  // dynamic shared memory: what the static arrays leave of 227 KB
 constexpr int kGroups = (kMaxNc / 4 + kEpiQ - 1) / kEpiQ;  // groups of 4 outputs per epilogue warp
 
-// Outputs of a thread that its epilogue has left for mend_outputs: bit 16 * (sine list) + 4 * (group of the warp) +
-// (output of the group).
-__shared__ unsigned s_marks[kEpiThreads];
+// Outputs of a thread that its epilogue has left for mend_outputs, by parity: bit 16 * (sine list) + 4 * (group of
+// the warp) + (output of the group).
+__shared__ unsigned s_marks[2][kEpiThreads];
 
 // The levels of four outputs as integers, sum over v of l[v] * 2^kSh.  A level times 2^9v (level 5 times
 // 2^kSh, rounded) is an integer that an addition of 1.5 * 2^23 leaves in the low mantissa bits while it
@@ -226,7 +226,7 @@ struct Four {
     long long u[4];
 };
 template <bool MARK>
-__device__ __noinline__ Four join_levels_wide(unsigned tm, int nc, float top3, float top4, int at) {
+__device__ __noinline__ Four join_levels_wide(unsigned tm, int nc, float top3, float top4, int par, int at) {
     unsigned l[kLev][4];
 #pragma unroll
     for (int v = 0; v < kLev; v++) tmem_ld4(l[v], tm + v * nc);
@@ -236,7 +236,7 @@ __device__ __noinline__ Four join_levels_wide(unsigned tm, int nc, float top3, f
     for (int t = 0; t < 4; t++) {
         auto level = [&](int v, float w) { return (long long)__float2int_rn(__uint_as_float(l[v][t]) * w); };
         if (MARK && (fabsf(__uint_as_float(l[3][t])) * 134217728.f >= top3 || fabsf(__uint_as_float(l[4][t])) * 68719476736.f >= top4)) {
-            s_marks[threadIdx.x] |= 1u << (at + t);
+            s_marks[par][threadIdx.x] |= 1u << (at + t);
             l[3][t] = l[4][t] = 0;
         }
         r.u[t] = (level(0, 1.f) << kSh) + (level(1, 512.f) << (kSh - 9)) + (level(2, 262144.f) << (kSh - 18)) +
@@ -613,17 +613,17 @@ __device__ __forceinline__ Unit unit_of(const GemmArgs &a, unsigned u) {
 // from the digits, which are exact whatever their size.  Beside the epilogue, whose registers it would cost 4 % of
 // every launch from within.
 template <int MODE>
-__device__ __noinline__ void mend_outputs(const GemmArgs &a, unsigned u, int par, double *out) {
+__device__ __noinline__ void mend_outputs(const GemmArgs &a, unsigned u, double *out) {
     const Unit w = unit_of<MODE>(a, u);
     const TcJob &J = a.job[w.job];
     const TcShape &s = a.s;
     const int lane = threadIdx.x & 127, g0 = threadIdx.x >> 7, nc = a.nc;
     const int e = a.expo[((size_t)w.job * a.ntile + w.lt) * kLanes + lane], q = e - 1022 - 14 - kSh + J.expo;
-    unsigned marks = s_marks[threadIdx.x];
-    s_marks[threadIdx.x] = 0;
+    unsigned long long marks = s_marks[0][threadIdx.x] | (unsigned long long)s_marks[1][threadIdx.x] << 32;
+    s_marks[0][threadIdx.x] = s_marks[1][threadIdx.x] = 0;
     if (e >= kNaN) return;
     for (; marks; marks &= marks - 1) {
-        const int bit = __ffs(marks) - 1, sine = bit >> 4, list = 2 * par + sine;
+        const int bit = __ffsll(marks) - 1, par = bit >> 5, sine = bit >> 4 & 1, list = 2 * par + sine;
         const int col = (g0 + kEpiQ * (bit >> 2 & 3)) * 4 + (bit & 3), j = w.chunk * nc + col;
         if (col >= w.cols) continue;
         const unsigned char *data = a.ws + (((size_t)w.job * a.ntile + w.lt) * a.ks.all() + a.ks.before(list)) * kAStage + lane * 16;
@@ -658,19 +658,15 @@ __device__ __noinline__ void mend_outputs(const GemmArgs &a, unsigned u, int par
             if (f <= a.m) out[2 * f + sine] += v;
         } else {
             const bool two = j && 2 * j != a.m;
+            // x[k] = A + B and x[k + n/2] = A - B
+            const size_t h = (size_t)a.m * s.rs;
+            const double d0 = sine ? -v : v, d1 = par ? -v : v;  // of A[j] or B[j], and of A or B[n/2 - j]
             double *o0 = out + (size_t)j * s.rs, *o1 = out + (size_t)(a.m - j) * s.rs;
-            if (par == 0) {  // integers yet
-                *(long long *)o0 += sine ? -t : t;
-                if (two) *(long long *)o1 += t;
-            } else {
-                const size_t h = (size_t)a.m * s.rs;
-                const double b = sine ? -v : v;
-                o0[0] += b;
-                o0[h] -= b;
-                if (two) {
-                    o1[0] -= v;
-                    o1[h] += v;
-                }
+            o0[0] += d0;
+            o0[h] += par ? -d0 : d0;
+            if (two) {
+                o1[0] += d1;
+                o1[h] += par ? -d1 : d1;
             }
         }
     }
@@ -811,16 +807,16 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ 
 #pragma unroll
             for (int v = 0; v < kLev; v++) tmem_ld4(l[v], at + v * nc);
         };
-        auto gather = [&](const TcJob &J, int sine, int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
+        auto gather = [&](const TcJob &J, int par, int sine, int gi, const unsigned (&l)[kLev][4], long long (&u)[4]) {
             if (__any_sync(~0u, !join_levels(l, u))) {
                 const unsigned at = tset + (g0 + kEpiQ * gi) * 4;
-                const Four w = MARK ? join_levels_wide<true>(at, nc, J.top[0], J.top[1], 16 * sine + 4 * gi)
-                                    : join_levels_wide<false>(at, nc, 0.f, 0.f, 0);
+                const Four w = MARK ? join_levels_wide<true>(at, nc, J.top[0], J.top[1], par, 16 * sine + 4 * gi)
+                                    : join_levels_wide<false>(at, nc, 0.f, 0.f, 0, 0);
 #pragma unroll
                 for (int t = 0; t < 4; t++) u[t] = w.u[t];
             }
         };
-        if (MARK) s_marks[threadIdx.x] = 0;
+        if (MARK) s_marks[0][threadIdx.x] = s_marks[1][threadIdx.x] = 0;
         int lists = 0;
         auto take = [&] {  // the next list's sums are there
             const int set = lists % NACC;
@@ -875,7 +871,7 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ 
                         fetch(gi, l);
                         tmem_wait(l);
                         long long P[4];
-                        gather(J, 0, gi, l, P);
+                        gather(J, par, 0, gi, l, P);
 #pragma unroll
                         for (int t = 0; t < 4; t++) Ps[((g0 + kEpiQ * gi) * 4 + t) * kLanes] = P[t];
                     }
@@ -888,13 +884,10 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ 
                     if (gi < ngr) {
                         fetch(gi, l);
                         tmem_wait(l);
-                        gather(J, 1, gi, l, Q[gi]);
+                        gather(J, par, 1, gi, l, Q[gi]);
                     }
                 give();
-                if (!live) {
-                    if (MARK) s_marks[threadIdx.x] = 0;  // of what lies beyond the outputs
-                    continue;
-                }
+                if (!live) continue;
                 // a group's loads, conversions and stores one after another: loads do not move across stores
 #pragma unroll
                 for (int gi = 0; gi < kGroups; gi++)
@@ -1001,7 +994,10 @@ __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ 
                             }
                         }
                 }
-                if (MARK && s_marks[threadIdx.x]) mend_outputs<MODE>(a, u, par, out);
+            }
+            if (MARK && (s_marks[0][threadIdx.x] | s_marks[1][threadIdx.x])) {
+                if (live) mend_outputs<MODE>(a, u, out);
+                else s_marks[0][threadIdx.x] = s_marks[1][threadIdx.x] = 0;  // of what lies beyond the outputs
             }
         }
     }
