@@ -678,7 +678,8 @@ __device__ __noinline__ void mend_outputs(const GemmArgs &a, unsigned u, double 
 // lists are as short as that read: half spectra to rows of 96 x 96 x 122, 91 -> 80 us, of 64 x 64 x 90, 45 -> 40 us.
 // (As a run-time choice it costs longer lengths 5 to 14 %.)
 // MARK: some job has sums that FP32 may not hold (TcJob::top), so outputs may be left to mend_outputs.  At lengths
-// below about 300 hardly any has, and the launches that do without take 2 % less.
+// below about 300 hardly any has, and their launches do without the registers for it (with marks in every kernel a
+// step at 256^2 x 257 took 25.3 instead of 24.7 ms).
 template <int MODE, bool ADD, int NACC, bool MARK>
 __global__ void __launch_bounds__(kGemmBlock, 1) k_gemm(const __grid_constant__ GemmArgs a) {
     extern __shared__ __align__(1024) unsigned char smem[];
