@@ -210,10 +210,10 @@ int fused_create(Plan &P, const StageParams &sp, FusedState **out) {
         ok = ok && cudaMalloc(&fs->X1[i], P.field_bytes()) == cudaSuccess;
         if (sp.ord >= 3) ok = ok && cudaMalloc(&fs->X2[i], P.field_bytes()) == cudaSuccess;
     }
+    for (int i = 0; i < 2; i++) ok = ok && cudaMalloc(&fs->E[i], P.field_bytes()) == cudaSuccess;
     fs->plain = plain_f64(P, sp) && tc_reserve(P) == OK;
     const bool columns = !fs->plain;  // buffers of the column kernels
     if (sp.solver == 1 && columns) ok = ok && cudaMalloc(&fs->side, 2 * (size_t)P.ny * P.nzp * P.elt()) == cudaSuccess;  // BOUSS only
-    for (int i = 0; i < 2; i++) ok = ok && cudaMalloc(&fs->E[i], P.field_bytes()) == cudaSuccess;
     for (int i = 0; i < 3 && columns; i++) ok = ok && cudaMalloc(&fs->W[i], P.field_bytes()) == cudaSuccess;
     if (ok && sp.nl_fp32) {
         if (P.prec != FP64) {

@@ -1142,6 +1142,7 @@ const TcSet *tc_set(Plan &P, int n, double factor, int *status, bool half) {
 // The limit, MiB, against an RK2 step of convection, ms: 512^2 x 513 2048: 235, 1024: 240, 512: 249, 128: 312; 256^2 x 257
 // 25.1, 25.7, 27.9, 35.4; 128^2 x 129 (701 MB at most) 4.08, 4.08, 4.09, 4.86.
 constexpr size_t kRoomMiB = 2048;
+constexpr size_t kSpareMiB = 64;  // beyond this, at most an eighth of the free memory
 
 // bytes and lanes of digits for launches of up to `jobs` transforms (1 or more), in `most` bytes if 16 tiles fit them
 static void room_for(const Plan &P, int jobs, size_t most, size_t *bytes, size_t *lanes) {
@@ -1166,9 +1167,14 @@ static int room(Plan &P, int jobs) {
     if (P.digit_room_mb < 0) return kNoFast;
     if (S->ws_jobs >= jobs) return OK;
     if (capturing(P)) return S->ws ? OK : kNoFast;
-    size_t last = 0;
-    for (size_t most = (size_t)(P.digit_room_mb ? P.digit_room_mb : kRoomMiB) << 20;; most /= 2) {
-        size_t bytes, lanes;
+    size_t last = 0, most = (size_t)(P.digit_room_mb ? P.digit_room_mb : kRoomMiB) << 20, bytes, lanes;
+    room_for(P, jobs, most, &bytes, &lanes);
+    if (bytes > kSpareMiB << 20) {  // the fields that a solver allocates after it need the rest
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) == cudaSuccess) most = std::min(most, std::max(free / 8, kSpareMiB << 20));
+        else cudaGetLastError();
+    }
+    for (;; most /= 2) {
         room_for(P, jobs, most, &bytes, &lanes);
         if (bytes == last || (bytes <= S->ws_bytes && lanes <= S->expo_count)) break;  // no smaller, or no gain
         last = bytes;

@@ -136,6 +136,34 @@ def test_memory_of_single_transforms():
     assert free - api.device_memory()[0] < 8 * 16 * 72 * 128 * 154
 
 
+# An FP64 solver in the memory that it took before its transforms had buffers (about 40 fields, 0.9 GB).
+def test_little_memory():
+    import torch
+    shape = (128, 128, 154)
+
+    def run():
+        p = plan(*shape)
+        s = api.Solver(p, api.BOUSS, ord=2, dt=1e-4, nu=1e-3, kappa=1e-3)
+        rng = np.random.default_rng(1)
+        for f in s.state[:-1]:
+            f.upload(1e-3 * (rng.standard_normal(p.sshape) + 1j * rng.standard_normal(p.sshape)))
+        s.step(2)
+        out = [f.download() for f in s.state]
+        s.close()
+        p.close()
+        return out
+
+    want = run()
+    torch.cuda.empty_cache()
+    held = torch.empty(api.device_memory()[0] - 1300 * 2**20, dtype=torch.uint8, device="cuda")
+    try:
+        got = run()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
 # The first transform of a plan inside a stream capture, where nothing can be allocated, and one after it.
 @pytest.mark.parametrize("before", [False, True])
 def test_first_call_captured(before):
