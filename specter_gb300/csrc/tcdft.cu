@@ -1421,7 +1421,8 @@ int tc_x_nonlinear(Plan &P, const XNLArgs &x, double bytes) {
 }
 
 // FP64 passes over the digit-product transforms (tcdft.cu).  They serve every even length of 32 to
-// 550: at all of them they are faster than the FP64 Stockham engine, which the FP64 pipe bounds.
+// 550: nearly everywhere they are faster than the FP64 Stockham engine, which the FP64 pipe bounds (z passes
+// 1.0 to 8 times, on grids of 4 x 2 to 64 x 32 columns; y passes at lengths 32 and 36 with a few columns 0.9 times).
 // kNoFast: a form that they do not take (another length, a scale on part of the rows).
 static int tc_add(Plan &P, TcJob *jobs, int *nj, int n, double factor, const void *in, void *out, const void *add,
                   int deriv) {
@@ -1474,7 +1475,10 @@ int tc_z_forward(Plan &P, const ZFwdArgs &a, int nf, double bytes) {
 // coalesced (written row by row, 256^2 x 282 took 439 us instead of 251 and 61 for the copy).  A few short
 // rows stay with the Stockham engine, one launch instead of two or three (whole transforms to physical
 // space, Stockham against digits, us: 32 x 32 x 58 33 and 38, 64 x 64 x 90 60 and 51, 32 x 128 x 154 107 and 78,
-// 64 x 192 x 282 338 and 195).
+// 64 x 192 x 282 338 and 195).  Longer rows are digit products whatever their number, for half the error: up to 2432
+// rows, one wave of the Stockham kernel's blocks, that costs up to a third of a c2r pass and a tenth of an r2c pass at
+// lengths of 96 to 256 (rows of 128, 1080 of them, to physical space 34.5 and 45.1 us, from it 34.9 and 38.3; 3000
+// and more 1.03 and 1.15 times faster).
 constexpr unsigned kFewRows = 16 * kLanes;
 int tc_x(Plan &P, const XArgs &a, int nf, bool r2c, double bytes) {
     if (!tc_length_ok(P.nx) || (P.nx < 96 && (unsigned)a.nrows * P.ny < kFewRows)) return kNoFast;
